@@ -15,6 +15,7 @@
 
 #include "mdb_engine.h"
 #include "mdb_kernels.cuh"
+#include "mdb_steps.cuh"
 #include "mdb_util.h"
 
 namespace mdb {
@@ -47,14 +48,17 @@ void* drift_fn(int dm, bool ln) {
 }
 
 void* steps_fn(int dm, bool ln) {
+#define MDB_S(D, F) \
+  return ln ? (void*)k_run_steps<D, F, true> : (void*)k_run_steps<D, F, false>
   switch (dm) {
-    case DM_NVE: return ln ? (void*)k_md_steps<DM_NVE, FM_NVE, true>
-                           : (void*)k_md_steps<DM_NVE, FM_NVE, false>;
-    case DM_NH: return ln ? (void*)k_md_steps<DM_NH, FM_NH, true>
-                          : (void*)k_md_steps<DM_NH, FM_NH, false>;
-    default: return ln ? (void*)k_md_steps<DM_NPH, FM_NPH, true>
-                       : (void*)k_md_steps<DM_NPH, FM_NPH, false>;
+    case DM_NVE: MDB_S(DM_NVE, FM_NVE);
+    case DM_NH: MDB_S(DM_NH, FM_NH);
+    case DM_NPH: MDB_S(DM_NPH, FM_NPH);
+    case DM_PISTON: MDB_S(DM_PISTON, FM_PISTON);
+    // FIRE systems keep one lane per slot
+    default: return (void*)k_run_steps<DM_FIRE, FM_FIRE, false>;
   }
+#undef MDB_S
 }
 
 namespace {
@@ -428,124 +432,77 @@ int Engine::build() {
   return autotune_ ? tune() : MDB_OK;
 }
 
-// The multi-step kernel needs every block of the (single) system resident at
-// once (two per SM). AUTO and MULTI take it whenever that holds: up to that
-// size the per-phase launches and their tails dominate a step (measured
-// faster from 900 to 65,536 particles).
+// The resident steps kernel (mdb_steps.cuh) needs every block of the (single)
+// system on the device at once, at one slot per thread. AUTO and MULTI take it
+// whenever that holds, for calls of any length: up to that size launches,
+// reduction tails and barriers dominate a step.
 int Engine::choose_multi_step() {
   multi_step_ = false;
   multi_cap_ = 0;
   schedule_.multi_step = 0;
   schedule_.multi_step_blocks = 0;
   if (nsys() != 1 || !use_graphs_ || step_kernel_ == MDB_STEPS_PER_PHASE) return MDB_OK;
+  if (hsp_[0].items != 1) return MDB_OK;
   int nsm = 0;
   MDB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device_));
   int coop = 0;
   MDB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_));
   if (!coop) return MDB_OK;
+  // Shared list columns: 16-bit offsets, up to 40 KB a block (80 entries per
+  // thread); longer or 32-bit lists are read from global memory.
+  const int per = (max_nbr_ + hsp_[0].lanes - 1) / hsp_[0].lanes;
+  const int rows = (per + kListGroup - 1) / kListGroup * kListGroup;
+  steps_.list_rows = (dev_.nl16 && rows > 0 && rows <= 80) ? rows : 0;
+  steps_smem_ = sizeof(int16_t) * kThreads * (size_t)steps_.list_rows;
+  const bool fire = hsp_[0].kind == K_FIRE;
   int per_sm = 1 << 30;
-  for (int dm : {DM_NVE, DM_NH, DM_NPH}) {
+  for (int dm : {DM_NVE, DM_NH, DM_NPH, DM_PISTON, DM_FIRE}) {
+    if (fire != (dm == DM_FIRE)) continue;
     int b = 0;
-    MDB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, steps_fn(dm, lanes_), kThreads, 0));
+    MDB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, steps_fn(dm, lanes_), kThreads,
+                                                           steps_smem_));
     per_sm = std::min(per_sm, b);
   }
   multi_cap_ = per_sm * nsm;
-  multi_step_ = nblocks_ >= 1 && nblocks_ <= multi_cap_;
+  if (nblocks_ >= 1 && nblocks_ <= multi_cap_) {
+    auto alloc = [&](void** p, size_t bytes) -> int {
+      MDB_CUDA(cudaMalloc(p, bytes));
+      allocs_.push_back(*p);
+      bytes_ += (int64_t)bytes;
+      MDB_CUDA(cudaMemsetAsync(*p, 0, bytes, stream_));
+      return MDB_OK;
+    };
+    // one zeroed allocation: positions, block sums, maxima, counts, sequence
+    const size_t pos = sizeof(float4) * (size_t)ntot_;
+    const size_t part = sizeof(double) * 2 * kNP * (size_t)nblocks_;
+    const size_t mx = sizeof(unsigned long long) * 16;
+    const size_t cnt = sizeof(int32_t) * (size_t)(ncells_ + nblocks_ + 2);
+    char* base = nullptr;
+    int rc = alloc((void**)&base, pos + part + mx + cnt);
+    if (rc) return rc;
+    steps_.pff1 = (float4*)base;
+    steps_.part = (double*)(base + pos);
+    steps_.max = (unsigned long long*)(base + pos + part);
+    steps_.seq = (uint32_t*)(base + pos + part + mx);
+    steps_.count = (int32_t*)(steps_.seq + 2);
+    steps_.tile = steps_.count + ncells_;
+    multi_step_ = true;
+  }
   schedule_.multi_step = multi_step_ ? 1 : 0;
   schedule_.multi_step_blocks = multi_cap_;
   return MDB_OK;
 }
 
-// while (more) { k_md_steps ; if (rebuild) { rebuild ; force ; count } }
-int Engine::get_steps_graph(int dm, int fm, cudaGraphExec_t* exec) {
-  auto key = std::make_tuple(3, dm, fm, 1, 0);
-  auto it = graphs_.find(key);
-  if (it != graphs_.end()) {
-    *exec = it->second.second;
-    return MDB_OK;
-  }
-  cudaGraph_t g;
-  MDB_CUDA(cudaGraphCreate(&g, 0));
-  int rc = MDB_OK;
-  auto ck = [&](cudaError_t e, const char* what) {
-    if (rc == MDB_OK && e != cudaSuccess) rc = cuda_error(e, what);
-    return rc == MDB_OK;
-  };
-  cudaGraphConditionalHandle h_more = 0, h_rb = 0;
-  ck(cudaGraphConditionalHandleCreate(&h_more, g, 1, cudaGraphCondAssignDefault), "handle");
-  ck(cudaGraphConditionalHandleCreate(&h_rb, g, 0, 0), "handle");
-  cudaGraph_t body = nullptr, rb_body = nullptr;
-  cudaGraphNode_t nwhile, nsteps, nif;
-  if (rc == MDB_OK) {
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h_more;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    if (ck(cudaGraphAddNode(&nwhile, g, nullptr, 0, &cp), "cudaGraphAddNode(while)"))
-      body = cp.conditional.phGraph_out[0];
-  }
+// n steps (FIRE: iterations) in one cooperative launch.
+int Engine::run_resident(int dm, int64_t n) {
   Dev d = dev_;
   d.use_cond = 0;
-  if (rc == MDB_OK) {
-    void* args[] = {&d, &h_more, &h_rb};
-    cudaKernelNodeParams kp = {};
-    kp.func = steps_fn(dm, lanes_);
-    kp.gridDim = dim3(nblocks_);
-    kp.blockDim = dim3(kThreads);
-    kp.kernelParams = args;
-    if (ck(cudaGraphAddKernelNode(&nsteps, body, nullptr, 0, &kp), "cudaGraphAddKernelNode")) {
-      cudaLaunchAttributeValue v = {};
-      v.cooperative = 1;
-      ck(cudaGraphKernelNodeSetAttribute(nsteps, cudaLaunchAttributeCooperative, &v),
-         "cudaGraphKernelNodeSetAttribute(cooperative)");
-    }
-  }
-  if (rc == MDB_OK) {
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h_rb;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    if (ck(cudaGraphAddNode(&nif, body, &nsteps, 1, &cp), "cudaGraphAddNode(if)"))
-      rb_body = cp.conditional.phGraph_out[0];
-  }
-  if (rc == MDB_OK) rc = add_rebuild_body(rb_body, d);
-  if (rc == MDB_OK) {
-    // the rebuild body ends in its one finish kernel: the force phase of the
-    // pending step and the count follow it
-    size_t nn = 0;
-    ck(cudaGraphGetNodes(rb_body, nullptr, &nn), "cudaGraphGetNodes");
-    std::vector<cudaGraphNode_t> nodes(nn);
-    if (rc == MDB_OK) ck(cudaGraphGetNodes(rb_body, nodes.data(), &nn), "cudaGraphGetNodes");
-    cudaGraphNode_t last = nullptr;
-    for (size_t k = 0; k < nn && rc == MDB_OK; ++k) {
-      size_t nd = 0;
-      ck(cudaGraphNodeGetDependentNodes(nodes[k], nullptr, &nd), "cudaGraphNodeGetDependentNodes");
-      if (nd == 0) last = nodes[k];
-    }
-    if (rc == MDB_OK && !last) rc = set_error(MDB_ERR_STATE, "rebuild body has no last node");
-    cudaGraphNode_t nf, nc;
-    if (rc == MDB_OK)
-      rc = add_kernel_node(rb_body, &last, 1, force_fn(fm, true, lanes_), nblocks_, kThreads, dev_, &nf);
-    if (rc == MDB_OK) {
-      void* args[] = {&d, &h_more};
-      cudaKernelNodeParams kp = {};
-      kp.func = (void*)k_md_steps_count;
-      kp.gridDim = dim3(1);
-      kp.blockDim = dim3(32);
-      kp.kernelParams = args;
-      ck(cudaGraphAddKernelNode(&nc, rb_body, &nf, 1, &kp), "cudaGraphAddKernelNode");
-    }
-  }
-  cudaGraphExec_t ex = nullptr;
-  if (rc == MDB_OK) ck(cudaGraphInstantiate(&ex, g, 0), "cudaGraphInstantiate(steps)");
-  if (rc != MDB_OK) {
-    cudaGraphDestroy(g);
-    return rc;
-  }
-  graphs_[key] = std::make_pair(g, ex);
-  *exec = ex;
+  StepsMem m = steps_;
+  void* args[] = {&d, &m, &n};
+  MDB_CUDA(cudaLaunchCooperativeKernel(steps_fn(dm, lanes_), dim3(nblocks_), dim3(kThreads), args,
+                                       steps_smem_, stream_));
+  launches_ += 1;
+  count_launches(1);
   return MDB_OK;
 }
 
@@ -722,21 +679,7 @@ int Engine::get_graph(int kind, int dm, int fm, bool py, int chunk, cudaGraphExe
 int Engine::run_md(int dm, int fm, bool py, int64_t nsteps) {
   if (!built_) return set_error(MDB_ERR_STATE, "engine not built");
   MDB_CUDA(cudaSetDevice(device_));
-  // (calls of fewer steps take the per-phase graphs: below kMultiStepMinSteps
-  // the multi-step launch's fixed cost outweighs what it saves per step)
-  if (multi_step_ && py && nsteps >= kMultiStepMinSteps &&
-      (dm == DM_NVE || dm == DM_NH || dm == DM_NPH)) {
-    cudaGraphExec_t ex;
-    const int grc = get_steps_graph(dm, fm, &ex);
-    if (grc != MDB_OK) return grc;
-    k_md_steps_set<<<1, 32, 0, stream_>>>(dev_, nsteps);
-    MDB_CUDA(cudaGetLastError());
-    MDB_CUDA(cudaGraphLaunch(ex, stream_));
-    // the count kernel and one multi-step launch (more after each rebuild)
-    launches_ += 2;
-    count_launches(2);
-    return MDB_OK;
-  }
+  if (multi_step_ && py == (dm != DM_PISTON)) return run_resident(dm, nsteps);
   int64_t left = nsteps;
   if (use_graphs_) {
     static const int kChunks[] = {64, 8, 1};
@@ -799,6 +742,7 @@ int Engine::run_md_timed(int dm, int fm, bool py, int64_t nsteps, double* ms) {
 int Engine::run_fire(int64_t iters) {
   if (!built_) return set_error(MDB_ERR_STATE, "engine not built");
   MDB_CUDA(cudaSetDevice(device_));
+  if (multi_step_) return run_resident(DM_FIRE, iters);
   int64_t left = iters;
   if (use_graphs_) {
     static const int kChunks[] = {100, 10, 1};

@@ -122,10 +122,10 @@ class Engine {
   void drop_graphs();
   // The cached protocol graph (built at the first protocol run).
   int proto_graph(cudaGraphExec_t* exec);
-  // Whether MD steps run in the multi-step kernel (single system, all
-  // blocks resident), and its cached graph per drift/force mode.
+  // Whether steps run in the resident steps kernel (single system, all blocks
+  // resident), and n of them in one launch of it.
   int choose_multi_step();
-  int get_steps_graph(int dm, int fm, cudaGraphExec_t* exec);
+  int run_resident(int dm, int64_t n);
   void free_proto();
   cudaError_t wait_host() {
     ++host_waits_;
@@ -152,7 +152,9 @@ class Engine {
   bool multi_step_ = false;
   bool lanes_ = false;  // some system has several lanes per slot (SysParams::lanes)
   int lanes_opt_ = MDB_LANES_ONE;  // mdb_options_t.lanes (AUTO counts as ONE here)
-  int multi_cap_ = 0;  // blocks of the multi-step kernel the device holds at once
+  int multi_cap_ = 0;  // blocks of the resident steps kernel the device holds at once
+  StepsMem steps_{};
+  size_t steps_smem_ = 0;
   mdb_schedule_t schedule_{};
   int stream_priority_ = 0;  // levels above normal for stream_
   int64_t aos_cap_ = 0;

@@ -40,9 +40,6 @@ constexpr int kListPrefetchRows = 28;
 // phase. FIRE systems keep one lane per slot.
 constexpr int kLanes = 4;
 constexpr int kLanesMaxN = 16384;
-// MD calls of at least this many steps use the multi-step kernel where it is
-// enabled (one step: 46 us in it against 36 us per phase at N = 4096).
-constexpr int kMultiStepMinSteps = 4;
 
 // Force-phase variants.
 enum FMode : int32_t {
@@ -129,10 +126,7 @@ struct BatchGlobal {
   uint32_t sys_counter;
   int32_t nsys;
   int32_t all_done;
-  int64_t steps_left;  // multi-step kernel: steps of the running call not yet done
-  uint32_t bar_count;  // multi-step kernel: grid barrier arrivals
-  uint32_t bar_gen;    //   and generation
-  int32_t bar_err;     //   a barrier wait ran out of polls
+  int32_t bar_err;     // resident steps kernel: an exchange ran out of polls
   int32_t forced;      // the pending rebuild was forced (not asked for by a drift)
 };
 
@@ -202,6 +196,17 @@ struct Dev {
   int32_t use_cond;
   int32_t rb_grid;    // grid of the grid-stride rebuild kernels
   int32_t pf_rows;    // force phase: list rows of the next chunk prefetched per warp
+};
+
+// Device memory of the resident steps kernel.
+struct StepsMem {
+  float4* pff1;     // second buffer of float-float positions
+  int32_t* count;   // particles per cell; all zero outside a rebuild
+  int32_t* tile;    // particles per block's range of cells; all zero outside a rebuild
+  double* part;     // [2][kNP][nblocks] block sums of the exchanges
+  unsigned long long* max;  // [4][4] maxima of the exchanges
+  uint32_t* seq;    // [0] exchanges run so far, [1] arrivals (nblocks per exchange)
+  int32_t list_rows;  // rows of the shared list (0: lists are read from global memory)
 };
 
 }  // namespace mdb

@@ -321,19 +321,24 @@ struct DriftTail {
   double g_dof, T0, Q, rc_max, skin, Lx_b, Ly_b;
   int ncx, ncy, allpairs, prior;
 };
-__device__ __forceinline__ DriftTail drift_tail_inputs(const Dev& D, const SysParams& P,
-                                                       const SysState* S) {
+__device__ __forceinline__ DriftTail drift_tail_scalars(const SysParams& P, const SysState& S) {
   DriftTail t;
   t.g_dof = P.g_dof;
   t.T0 = P.T0;
   t.Q = P.Q;
   t.rc_max = P.rc_max;
   t.skin = P.skin;
-  t.Lx_b = S->Lx_b;
-  t.Ly_b = S->Ly_b;
-  t.ncx = S->ncx;
-  t.ncy = S->ncy;
-  t.allpairs = S->allpairs;
+  t.Lx_b = S.Lx_b;
+  t.Ly_b = S.Ly_b;
+  t.ncx = S.ncx;
+  t.ncy = S.ncy;
+  t.allpairs = S.allpairs;
+  t.prior = 0;
+  return t;
+}
+__device__ __forceinline__ DriftTail drift_tail_inputs(const Dev& D, const SysParams& P,
+                                                       const SysState* S) {
+  DriftTail t = drift_tail_scalars(P, *S);
   // a rebuild requested before this launch (a forced rebuild); for a lone
   // system nothing else changes the flag until this block sets it
   t.prior = (D.nsys == 1) ? *((volatile int*)&D.bg->any_rebuild) : 0;
@@ -422,8 +427,8 @@ __device__ __forceinline__ void pair_one(const float4 q, const PairCtx& c, float
 // a time before the dependent position gathers to keep loads in flight.
 // Position loads of the pair loop. NC: through the read-only data path, for
 // kernels that do not write positions. Otherwise a plain (weak, L1-cached)
-// load: the multi-step kernel writes the positions between its phases, and
-// the acquire of its grid barrier makes those writes visible to it.
+// load: the resident steps kernel writes the positions between its phases, and
+// the acquire of its exchange makes those writes visible to it.
 template <bool NC>
 __device__ __forceinline__ float4 ld_pos(const float4* p) {
   if (NC) return __ldg(p);
@@ -431,6 +436,24 @@ __device__ __forceinline__ float4 ld_pos(const float4* p) {
   asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                : "l"(p));
+  return v;
+}
+
+// Loads of lists, counts and cell ranges: read-only path in kernels that do
+// not write them, plain loads in the resident steps kernel, which rebuilds the
+// lists between its steps.
+template <bool NC>
+__device__ __forceinline__ int ld_idx(const int32_t* p) {
+  if (NC) return __ldg(p);
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+template <bool NC>
+__device__ __forceinline__ int ld_idx(const int16_t* p) {
+  if (NC) return (int)__ldg(p);
+  int v;
+  asm volatile("ld.global.s16 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 
@@ -454,7 +477,7 @@ __device__ __forceinline__ void pair_list(const float4* __restrict__ pff,
     int j[PF];
 #pragma unroll
     for (int q = 0; q < PF; ++q) {
-      int t = (int)__ldg(p + (int64_t)(k + q) * step);
+      int t = ld_idx<NC>(p + (int64_t)(k + q) * step);
       if (MIC) {
         t += li;
         t += (t < 0) ? n : 0;
@@ -467,7 +490,7 @@ __device__ __forceinline__ void pair_list(const float4* __restrict__ pff,
       pair_one<PY, ENERGY, VIRIAL, MIC, FLOOR>(ld_pos<NC>(base + j[q]), c, fs, fc, ws, wc, u, an);
   }
   for (; k < nn; ++k) {
-    int t = (int)__ldg(p + (int64_t)k * step);
+    int t = ld_idx<NC>(p + (int64_t)k * step);
     if (MIC) {
       t += li;
       t += (t < 0) ? n : 0;
@@ -493,21 +516,35 @@ __device__ __forceinline__ void split_box(double L, float& h, float& l, float& i
   inv = 1.0f / h;
 }
 
-// Slot i's position and the box in a pair context; PY = false leaves the y
-// image shift at 0 (walled y axis).
+// The box of a pair context; PY = false leaves the y image shift at 0 (walled
+// y axis).
+struct PairBox {
+  float2 nLh, nLl, invL;
+};
+template <bool PY>
+__device__ __forceinline__ PairBox pair_box(double Lx, double Ly) {
+  PairBox b;
+  float h, l, inv;
+  split_box(Lx, h, l, inv);
+  b.nLh.x = -h;
+  b.nLl.x = -l;
+  b.invL.x = inv;
+  split_box(Ly, h, l, inv);
+  b.nLh.y = -h;
+  b.nLl.y = -l;
+  b.invL.y = PY ? inv : 0.0f;
+  return b;
+}
+
+// Slot i's position and the box in a pair context.
 template <bool PY>
 __device__ __forceinline__ void set_pair_box(PairCtx& c, const float4 qi, double Lx, double Ly) {
   c.ih = make_float2(qi.x, qi.y);
   c.il = make_float2(qi.z, qi.w);
-  float h, l, inv;
-  split_box(Lx, h, l, inv);
-  c.nLh.x = -h;
-  c.nLl.x = -l;
-  c.invL.x = inv;
-  split_box(Ly, h, l, inv);
-  c.nLh.y = -h;
-  c.nLl.y = -l;
-  c.invL.y = PY ? inv : 0.0f;
+  const PairBox b = pair_box<PY>(Lx, Ly);
+  c.nLh = b.nLh;
+  c.nLl = b.nLl;
+  c.invL = b.invL;
 }
 
 // Pair parameters of slot i's class: "same" for partners of its own class,
@@ -523,22 +560,9 @@ __device__ __forceinline__ void set_profile_class(PairCtx& c, const SysParams& P
   c.e24ab = P.feps24[2];
 }
 
-// Sum of pair forces on slot i over its 3x3 cell stencil (or every slot of the
-// system for grids narrower than 3 cells). Returns F in FP64. tci receives the
-// type class of slot i, decoded from its float-float position (encode_ff), so
-// the type array is not read.
-//
-// LANES > 1: lane `lane` of the LANES lanes that share slot i sums its share
-// of the candidates (the caller adds the lanes' results in a fixed order).
-template <bool PY, bool ENERGY, bool VIRIAL, bool FLOOR = false, bool NC = true, int LANES = 1>
-__device__ __forceinline__ void particle_force(const Dev& D, const SysParams& P, const SysState& S,
-                                               int64_t i, double Lx, double Ly, double& fx,
-                                               double& fy, double& w, double& u, double& an,
-                                               int& tci, int lane = 0) {
-  PairCtx c;
-  const float4 qi = ld_pos<NC>(D.pff + i);
-  set_pair_box<PY>(c, qi, Lx, Ly);
-  tci = (int)ff_class(qi);
+// Pair parameters of class tci for the force loops.
+template <bool FLOOR>
+__device__ __forceinline__ void set_pair_class(PairCtx& c, const SysParams& P, int tci) {
   c.ts = (tci == 2) ? 99u : (uint32_t)tci;
   c.tsz = (tci == 1) ? 1u : 0u;
   const int sc = (tci == 2) ? 2 : tci;
@@ -558,12 +582,30 @@ __device__ __forceinline__ void particle_force(const Dev& D, const SysParams& P,
     c.r2fs = 1e-5f * P.fsig2[sc];
     c.r2fab = 1e-5f * P.fsig2[2];
   }
+}
+
+// Sum of pair forces on slot i over its 3x3 cell stencil (or every slot of the
+// system for grids narrower than 3 cells). Returns F in FP64. tci receives the
+// type class of slot i, decoded from its float-float position (encode_ff), so
+// the type array is not read.
+//
+// LANES > 1: lane `lane` of the LANES lanes that share slot i sums its share
+// of the candidates (the caller adds the lanes' results in a fixed order).
+template <bool PY, bool ENERGY, bool VIRIAL, bool FLOOR = false, bool NC = true, int LANES = 1>
+__device__ __forceinline__ void particle_force(const Dev& D, const float4* __restrict__ pff,
+                                               const SysParams& P, const SysState& S, int64_t i, double Lx, double Ly, double& fx,
+                                               double& fy, double& w, double& u, double& an,
+                                               int& tci, int lane = 0) {
+  PairCtx c;
+  const float4 qi = ld_pos<NC>(pff + i);
+  set_pair_box<PY>(c, qi, Lx, Ly);
+  tci = (int)ff_class(qi);
+  set_pair_class<FLOOR>(c, P, tci);
   float2 fs = make_float2(0.f, 0.f), fc = make_float2(0.f, 0.f);
   float ws = 0.f, wc = 0.f;
   u = 0.0;
   an = 0.0;
-  const float4* __restrict__ pff = D.pff;
-  const int nc = __ldg(D.ncount + i);
+  const int nc = ld_idx<NC>(D.ncount + i);
   if (nc >= 0) {
     const int li = (int)(i - P.p0);
     const int nn = nc & (kListInterior - 1);
@@ -587,7 +629,7 @@ __device__ __forceinline__ void particle_force(const Dev& D, const SysParams& P,
                                           u, an, lane);
   } else {
     const int ncx = S.ncx, ncy = S.ncy;
-    const int cell = D.cell_of[i];
+    const int cell = ld_idx<NC>(D.cell_of + i);
     const int cx = cell % ncx, cy = cell / ncx;
     const int* __restrict__ cs = D.cstart;
 #pragma unroll 1
@@ -601,17 +643,17 @@ __device__ __forceinline__ void particle_force(const Dev& D, const SysParams& P,
       }
       const int64_t row = P.c0 + (int64_t)yy * ncx;
       if (cx > 0 && cx < ncx - 1) {
-        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, __ldg(cs + row + cx - 1),
-                                              __ldg(cs + row + cx + 2), c, fs, fc, ws, wc, u, an, lane);
+        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, ld_idx<NC>(cs + row + cx - 1),
+                                              ld_idx<NC>(cs + row + cx + 2), c, fs, fc, ws, wc, u, an, lane);
       } else if (cx == 0) {
-        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, __ldg(cs + row), __ldg(cs + row + 2), c, fs, fc,
+        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, ld_idx<NC>(cs + row), ld_idx<NC>(cs + row + 2), c, fs, fc,
                                               ws, wc, u, an, lane);
-        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, __ldg(cs + row + ncx - 1),
-                                              __ldg(cs + row + ncx), c, fs, fc, ws, wc, u, an, lane);
+        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, ld_idx<NC>(cs + row + ncx - 1),
+                                              ld_idx<NC>(cs + row + ncx), c, fs, fc, ws, wc, u, an, lane);
       } else {
-        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, __ldg(cs + row + ncx - 2),
-                                              __ldg(cs + row + ncx), c, fs, fc, ws, wc, u, an, lane);
-        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, __ldg(cs + row), __ldg(cs + row + 1), c, fs, fc,
+        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, ld_idx<NC>(cs + row + ncx - 2),
+                                              ld_idx<NC>(cs + row + ncx), c, fs, fc, ws, wc, u, an, lane);
+        pair_range<PY, ENERGY, VIRIAL, FLOOR, NC, LANES>(pff, ld_idx<NC>(cs + row), ld_idx<NC>(cs + row + 1), c, fs, fc,
                                               ws, wc, u, an, lane);
       }
     }
@@ -663,7 +705,7 @@ __device__ __forceinline__ void pair_one_hp(const float4 q, const PairCtxD& c, d
   }
 }
 
-template <bool PY, bool ENERGY, bool VIRIAL, bool MIC, typename IDX>
+template <bool PY, bool ENERGY, bool VIRIAL, bool MIC, bool NC, typename IDX>
 __device__ __forceinline__ void pair_list_hp(const float4* __restrict__ pff,
                                              const IDX* __restrict__ nlist, int64_t ntot,
                                              int64_t i, int li, int n, int nn, const PairCtxD& c,
@@ -671,32 +713,28 @@ __device__ __forceinline__ void pair_list_hp(const float4* __restrict__ pff,
                                              double& an) {
   const float4* __restrict__ base = MIC ? pff + (i - li) : pff + i;
   for (int k = 0; k < nn; ++k) {
-    int t = (int)__ldg(nlist + i + (int64_t)k * ntot);
+    int t = ld_idx<NC>(nlist + i + (int64_t)k * ntot);
     if (MIC) {
       t += li;
       t += (t < 0) ? n : 0;
       t -= (t >= n) ? n : 0;
     }
-    pair_one_hp<PY, ENERGY, VIRIAL, MIC>(__ldg(base + t), c, fx, fy, w, u, an);
+    pair_one_hp<PY, ENERGY, VIRIAL, MIC>(ld_pos<NC>(base + t), c, fx, fy, w, u, an);
   }
 }
 
-template <bool PY, bool ENERGY, bool VIRIAL>
+template <bool PY, bool ENERGY, bool VIRIAL, bool NC>
 __device__ __forceinline__ void pair_range_hp(const float4* __restrict__ pff, int j0, int j1,
                                               const PairCtxD& c, double& fx, double& fy,
                                               double& w, double& u, double& an) {
   for (int j = j0; j < j1; ++j)
-    pair_one_hp<PY, ENERGY, VIRIAL, true>(__ldg(pff + j), c, fx, fy, w, u, an);
+    pair_one_hp<PY, ENERGY, VIRIAL, true>(ld_pos<NC>(pff + j), c, fx, fy, w, u, an);
 }
 
-// FP64 counterpart of particle_force (same outputs; w already halved).
-template <bool PY, bool ENERGY, bool VIRIAL>
-__device__ __forceinline__ void particle_force_hp(const Dev& D, const SysParams& P,
-                                               const SysState& S, int64_t i, double Lx,
-                                               double Ly, double& fx, double& fy, double& w,
-                                               double& u, double& an) {
+// FP64 pair context of the slot at qi.
+__device__ __forceinline__ PairCtxD pair_ctx_hp(const SysParams& P, const float4 qi, double Lx,
+                                                double Ly) {
   PairCtxD c;
-  const float4 qi = __ldg(D.pff + i);
   c.xi = (double)qi.x + (double)qi.z;
   c.yi = (double)qi.y + (double)qi.w;
   c.Lx = Lx;
@@ -717,36 +755,47 @@ __device__ __forceinline__ void particle_force_hp(const Dev& D, const SysParams&
   c.e4ab = 4.0 * P.eps[2];
   c.Vcs = P.Vc[sc];
   c.Vcab = P.Vc[2];
+  return c;
+}
+
+// FP64 counterpart of particle_force (same outputs; w already halved).
+template <bool PY, bool ENERGY, bool VIRIAL, bool NC = true>
+__device__ __forceinline__ void particle_force_hp(const Dev& D,
+                                               const float4* __restrict__ pff, const SysParams& P,
+                                               const SysState& S, int64_t i, double Lx,
+                                               double Ly, double& fx, double& fy, double& w,
+                                               double& u, double& an) {
+  const float4 qi = ld_pos<NC>(pff + i);
+  const PairCtxD c = pair_ctx_hp(P, qi, Lx, Ly);
   fx = fy = w = u = an = 0.0;
-  const float4* __restrict__ pff = D.pff;
-  const int nc = __ldg(D.ncount + i);
+  const int nc = ld_idx<NC>(D.ncount + i);
   if (nc >= 0) {
     const int li = (int)(i - P.p0);
     const int nn = nc & (kListInterior - 1);
     const bool interior = (nc & kListInterior) != 0;
     if (D.nl16) {
       if (interior)
-        pair_list_hp<PY, ENERGY, VIRIAL, false>(pff, D.nlist16, D.ntot, i, li, P.n, nn, c, fx,
+        pair_list_hp<PY, ENERGY, VIRIAL, false, NC>(pff, D.nlist16, D.ntot, i, li, P.n, nn, c, fx,
                                                 fy, w, u, an);
       else
-        pair_list_hp<PY, ENERGY, VIRIAL, true>(pff, D.nlist16, D.ntot, i, li, P.n, nn, c, fx, fy,
+        pair_list_hp<PY, ENERGY, VIRIAL, true, NC>(pff, D.nlist16, D.ntot, i, li, P.n, nn, c, fx, fy,
                                                w, u, an);
     } else {
       if (interior)
-        pair_list_hp<PY, ENERGY, VIRIAL, false>(pff, D.nlist, D.ntot, i, li, P.n, nn, c, fx, fy,
+        pair_list_hp<PY, ENERGY, VIRIAL, false, NC>(pff, D.nlist, D.ntot, i, li, P.n, nn, c, fx, fy,
                                                 w, u, an);
       else
-        pair_list_hp<PY, ENERGY, VIRIAL, true>(pff, D.nlist, D.ntot, i, li, P.n, nn, c, fx, fy,
+        pair_list_hp<PY, ENERGY, VIRIAL, true, NC>(pff, D.nlist, D.ntot, i, li, P.n, nn, c, fx, fy,
                                                w, u, an);
     }
   } else if (S.allpairs) {
     for (int64_t j = P.p0; j < P.p0 + P.n; ++j) {
       if (j == i) continue;
-      pair_one_hp<PY, ENERGY, VIRIAL, true>(__ldg(pff + j), c, fx, fy, w, u, an);
+      pair_one_hp<PY, ENERGY, VIRIAL, true>(ld_pos<NC>(pff + j), c, fx, fy, w, u, an);
     }
   } else {
     const int ncx = S.ncx, ncy = S.ncy;
-    const int cell = D.cell_of[i];
+    const int cell = ld_idx<NC>(D.cell_of + i);
     const int cx = cell % ncx, cy = cell / ncx;
     const int* __restrict__ cs = D.cstart;
     for (int dr = -1; dr <= 1; ++dr) {
@@ -759,17 +808,17 @@ __device__ __forceinline__ void particle_force_hp(const Dev& D, const SysParams&
       }
       const int64_t row = P.c0 + (int64_t)yy * ncx;
       if (cx > 0 && cx < ncx - 1) {
-        pair_range_hp<PY, ENERGY, VIRIAL>(pff, __ldg(cs + row + cx - 1), __ldg(cs + row + cx + 2),
+        pair_range_hp<PY, ENERGY, VIRIAL, NC>(pff, ld_idx<NC>(cs + row + cx - 1), ld_idx<NC>(cs + row + cx + 2),
                                           c, fx, fy, w, u, an);
       } else if (cx == 0) {
-        pair_range_hp<PY, ENERGY, VIRIAL>(pff, __ldg(cs + row), __ldg(cs + row + 2), c, fx, fy, w,
+        pair_range_hp<PY, ENERGY, VIRIAL, NC>(pff, ld_idx<NC>(cs + row), ld_idx<NC>(cs + row + 2), c, fx, fy, w,
                                           u, an);
-        pair_range_hp<PY, ENERGY, VIRIAL>(pff, __ldg(cs + row + ncx - 1), __ldg(cs + row + ncx),
+        pair_range_hp<PY, ENERGY, VIRIAL, NC>(pff, ld_idx<NC>(cs + row + ncx - 1), ld_idx<NC>(cs + row + ncx),
                                           c, fx, fy, w, u, an);
       } else {
-        pair_range_hp<PY, ENERGY, VIRIAL>(pff, __ldg(cs + row + ncx - 2), __ldg(cs + row + ncx),
+        pair_range_hp<PY, ENERGY, VIRIAL, NC>(pff, ld_idx<NC>(cs + row + ncx - 2), ld_idx<NC>(cs + row + ncx),
                                           c, fx, fy, w, u, an);
-        pair_range_hp<PY, ENERGY, VIRIAL>(pff, __ldg(cs + row), __ldg(cs + row + 1), c, fx, fy, w,
+        pair_range_hp<PY, ENERGY, VIRIAL, NC>(pff, ld_idx<NC>(cs + row), ld_idx<NC>(cs + row + 1), c, fx, fy, w,
                                           u, an);
       }
     }
@@ -814,19 +863,19 @@ struct ForceFinish {
     mx[0] = mx[1] = mx[2] = 0.0;
     bad = 0;
   }
-  __device__ __forceinline__ void operator()(const Dev& D, const SysParams& P, double Ly,
-                                             double h, double xi2, double fdt, int64_t i,
-                                             double fx, double fy, double w, double u, double an,
-                                             int tci) {
+  // The slot's velocity v is kicked in place and its acceleration returned in
+  // a; y is its y position (read for the walled y axis only).
+  __device__ __forceinline__ void kick(const SysParams& P, double Ly, double h, double xi2,
+                                       double fdt, double y, double fx, double fy, double w,
+                                       double u, double an, int tci, double2& v, double2& a) {
     const double m = (tci == 0) ? P.massA : P.massB;  // type 0 <=> class 0
-    double2 v = D.vel[i];
     if (FM == FM_OBS) {
       red[0] += u;
       red[1] += w;
       red[2] += m * fma(v.x, v.x, v.y * v.y);
       if (!PY) {
         double up, en;
-        wall_terms(D.pos[i].y, Ly, P.k_piston, up, en);
+        wall_terms(y, Ly, P.k_piston, up, en);
         red[3] += up;
         red[4] += en;
       }
@@ -843,7 +892,7 @@ struct ForceFinish {
       }
       if (!PY && (FM == FM_INIT || FM == FM_PISTON)) {
         double up, en;
-        const double wf = wall_terms(D.pos[i].y, Ly, P.k_piston, up, en);
+        const double wf = wall_terms(y, Ly, P.k_piston, up, en);
         if (wf != 0.0) ay = ay + wf / m;
         red[0] += up;
         red[1] += en;
@@ -873,9 +922,21 @@ struct ForceFinish {
         }
         red[0] += fma(v.x, ax, v.y * ay);
       }
-      D.acc[i] = make_double2(ax, ay);
-      if (FM != FM_INIT) D.vel[i] = v;
+      a = make_double2(ax, ay);
       if (!isfinite(ax) || !isfinite(ay) || !isfinite(v.x) || !isfinite(v.y)) bad = 1;
+    }
+  }
+  __device__ __forceinline__ void operator()(const Dev& D, const SysParams& P, double Ly,
+                                             double h, double xi2, double fdt, int64_t i,
+                                             double fx, double fy, double w, double u, double an,
+                                             int tci) {
+    constexpr bool kWalls = !PY && (FM == FM_OBS || FM == FM_INIT || FM == FM_PISTON);
+    double2 v = D.vel[i], a;
+    const double y = kWalls ? D.pos[i].y : 0.0;
+    kick(P, Ly, h, xi2, fdt, y, fx, fy, w, u, an, tci, v, a);
+    if (FM != FM_OBS) {
+      D.acc[i] = a;
+      if (FM != FM_INIT) D.vel[i] = v;
     }
   }
 };
@@ -900,10 +961,96 @@ __device__ __noinline__ ForceFinish<FM, PY> force_items_hp(Dev D, const SysParam
     double fx, fy, w, u, an;
     const float4 qi = __ldg(D.pff + i);
     const int tci = (int)ff_class(qi);
-    particle_force_hp<PY, kEnergy, kVirial>(D, P, *Sp, i, Lx, Ly, fx, fy, w, u, an);
+    particle_force_hp<PY, kEnergy, kVirial>(D, D.pff, P, *Sp, i, Lx, Ly, fx, fy, w, u, an);
     fin(D, P, Ly, h, xi2, fdt, i, fx, fy, w, u, an, tci);
   }
   return fin;
+}
+
+// Scalar update of a system after its force phase (one thread): totals tot and
+// maxima tmx of the phase's reductions, tin the scalars from before it. Returns
+// whether a FIRE system converged.
+template <int FM, bool PY>
+__device__ __forceinline__ int force_tail(SysState* S, const ForceTail& tin, double Lx, double Ly,
+                                          double h, const double (&tot)[kNP],
+                                          const double (&tmx)[3]) {
+  int conv = 0;
+  if (FM == FM_NH) {
+    S->K = tot[0];
+  } else if (FM == FM_NPH) {
+    const double A = Lx * Ly;
+    const double p_new = (A > 0.0) ? (tot[0] + tot[2]) / (2.0 * A) : 0.0;
+    double pA = tin.pA + h * (p_new - tin.p_ext);
+    if (tin.clamped) {
+      if (Ly <= tin.fl && pA < 0.0) pA = 0.0;
+      if (Ly >= tin.ce && pA > 0.0) pA = 0.0;
+    }
+    S->pA = pA;
+    S->last_P = p_new;
+    S->P_cur = (A > 0.0) ? (tot[1] + tot[2]) / (2.0 * A) : 0.0;
+    S->Wv = tot[2];
+  } else if (FM == FM_PISTON) {
+    const double Fp = tot[0];
+    const double a_new = (Fp - tin.p_ext * Lx) / tin.W;
+    double vp = tin.vp + h * a_new;
+    if (tin.clamped) {
+      if (Ly <= tin.fl && vp < 0.0) vp = 0.0;
+      if (Ly >= tin.ce && vp > 0.0) vp = 0.0;
+    }
+    S->vp = vp;
+    S->Fp = Fp;
+    S->wallU = tot[1];
+    S->last_P = Fp / Lx;
+  } else if (FM == FM_INIT) {
+    if (!PY) {
+      S->Fp = tot[0];
+      S->wallU = tot[1];
+    }
+  } else if (FM == FM_OBS) {
+    S->U = tot[0];
+    S->Wv = tot[1];
+    S->kin = tot[2];
+    S->kin2 = tot[3];
+    S->wallU = tot[4];
+    S->Wani = 0.5 * tot[5];
+  } else if (FM == FM_FIRE) {
+    // FIRE control (src/md_energy_minimizer.cu:171-203)
+    const double maxf = (tmx[1] > 0.0) ? __longlong_as_double(0x7ff8000000000000ULL) : tmx[0];
+    S->f_power = tot[0];
+    S->f_maxf = maxf;
+    // from the next iteration on, FP64 pair terms for this system
+    if (!tin.f_fp64 && maxf < tin.f_hp_below) S->f_fp64 = 1;
+    if (maxf < tin.f_tol) {
+      conv = 1;
+      S->f_conv = 1;
+      S->f_conv_step = tin.f_step;
+    } else {
+      if (tot[0] > 0.0) {
+        const int streak = tin.f_streak + 1;
+        S->f_streak = streak;
+        if (streak > tin.f_Nmin) {
+          const double d2 = tin.f_dt * tin.f_inc;
+          S->f_dt = d2 < tin.f_dt_max ? d2 : tin.f_dt_max;
+          const double a2 = tin.f_alpha * 0.99;
+          S->f_alpha = a2 > 0.0 ? a2 : 0.0;
+        }
+        S->f_zero_v = 0;
+      } else {
+        S->f_dt = tin.f_dt * tin.f_dec;
+        S->f_streak = 0;
+        S->f_alpha = tin.f_alpha0;
+        S->f_zero_v = 1;
+      }
+      S->f_step = tin.f_step + 1;
+    }
+  }
+  if (FM != FM_INIT && FM != FM_OBS && FM != FM_FIRE) {
+    const int64_t steps = tin.steps + 1;
+    S->steps = steps;
+    // an MD segment of a batch ends after its target number of steps
+    if (tin.target_steps > 0 && steps >= tin.target_steps) S->done = 1;
+  }
+  return conv;
 }
 
 // ------------------------------------------------------------ force phase --
@@ -911,11 +1058,11 @@ __device__ __noinline__ ForceFinish<FM, PY> force_items_hp(Dev D, const SysParam
 // y image convention (false = the piston's walled y axis, which also applies
 // the soft walls in FM_INIT/FM_OBS).
 //
-// force_phase is the work of block b of the launch; k_force runs it as one
-// kernel, k_md_steps as a phase of its multi-step loop (NC = false: plain
-// position loads, see ld_pos).
-template <int FM, bool PY, bool NC, bool LN>
-__device__ __forceinline__ void force_phase(const Dev& D, const int b) {
+// LN: the launch holds systems with several lanes per slot (the kernel
+// without them keeps the one-lane code only).
+template <int FM, bool PY, bool LN>
+__global__ void __launch_bounds__(kThreads, 4) k_force(Dev D) {
+  const int b = blockIdx.x;
   const int s = D.sys_of_block[b];
   const SysParams& P = D.sp[s];
   SysState* S = D.st + s;
@@ -967,7 +1114,7 @@ __device__ __forceinline__ void force_phase(const Dev& D, const int b) {
     double fx = 0.0, fy = 0.0, w = 0.0, u = 0.0, an = 0.0;
     int tci = 0;
     if (!skip && i < end)
-      particle_force<PY, kEnergy, kVirial, kHpCapable, NC, kLanes>(D, P, *S, i, Lx, Ly, fx, fy, w,
+      particle_force<PY, kEnergy, kVirial, kHpCapable, true, kLanes>(D, D.pff, P, *S, i, Lx, Ly, fx, fy, w,
                                                                  u, an, tci, lane);
 #pragma unroll
     for (int o = 1; o < kLanes; o <<= 1) {
@@ -1018,7 +1165,7 @@ __device__ __forceinline__ void force_phase(const Dev& D, const int b) {
       double fx, fy, w, u, an;
       int tci;
       if (i < end) {
-        particle_force<PY, kEnergy, kVirial, kHpCapable, NC>(D, P, *S, i, Lx, Ly, fx, fy, w, u, an,
+        particle_force<PY, kEnergy, kVirial, kHpCapable, true>(D, D.pff, P, *S, i, Lx, Ly, fx, fy, w, u, an,
                                                          tci);
         fin(D, P, Ly, h, xi2, fdt, i, fx, fy, w, u, an, tci);
       }
@@ -1032,93 +1179,10 @@ __device__ __forceinline__ void force_phase(const Dev& D, const int b) {
   if (!reduce_system<kNS, kNM>(D, P, S, fin.red, fin.mx, tot, tmx)) return;
   if (threadIdx.x != 0) return;
   int conv = 0;
-  if (!skip) {
-    if (FM == FM_NH) {
-      S->K = tot[0];
-    } else if (FM == FM_NPH) {
-      const double A = Lx * Ly;
-      const double p_new = (A > 0.0) ? (tot[0] + tot[2]) / (2.0 * A) : 0.0;
-      double pA = tin.pA + h * (p_new - tin.p_ext);
-      if (tin.clamped) {
-        if (Ly <= tin.fl && pA < 0.0) pA = 0.0;
-        if (Ly >= tin.ce && pA > 0.0) pA = 0.0;
-      }
-      S->pA = pA;
-      S->last_P = p_new;
-      S->P_cur = (A > 0.0) ? (tot[1] + tot[2]) / (2.0 * A) : 0.0;
-      S->Wv = tot[2];
-    } else if (FM == FM_PISTON) {
-      const double Fp = tot[0];
-      const double a_new = (Fp - tin.p_ext * Lx) / tin.W;
-      double vp = tin.vp + h * a_new;
-      if (tin.clamped) {
-        if (Ly <= tin.fl && vp < 0.0) vp = 0.0;
-        if (Ly >= tin.ce && vp > 0.0) vp = 0.0;
-      }
-      S->vp = vp;
-      S->Fp = Fp;
-      S->wallU = tot[1];
-      S->last_P = Fp / Lx;
-    } else if (FM == FM_INIT) {
-      if (!PY) {
-        S->Fp = tot[0];
-        S->wallU = tot[1];
-      }
-    } else if (FM == FM_OBS) {
-      S->U = tot[0];
-      S->Wv = tot[1];
-      S->kin = tot[2];
-      S->kin2 = tot[3];
-      S->wallU = tot[4];
-      S->Wani = 0.5 * tot[5];
-    } else if (FM == FM_FIRE) {
-      // FIRE control (src/md_energy_minimizer.cu:171-203)
-      const double maxf = (tmx[1] > 0.0) ? __longlong_as_double(0x7ff8000000000000ULL) : tmx[0];
-      S->f_power = tot[0];
-      S->f_maxf = maxf;
-      // from the next iteration on, FP64 pair terms for this system
-      if (!tin.f_fp64 && maxf < tin.f_hp_below) S->f_fp64 = 1;
-      if (maxf < tin.f_tol) {
-        conv = 1;
-        S->f_conv = 1;
-        S->f_conv_step = tin.f_step;
-      } else {
-        if (tot[0] > 0.0) {
-          const int streak = tin.f_streak + 1;
-          S->f_streak = streak;
-          if (streak > tin.f_Nmin) {
-            const double d2 = tin.f_dt * tin.f_inc;
-            S->f_dt = d2 < tin.f_dt_max ? d2 : tin.f_dt_max;
-            const double a2 = tin.f_alpha * 0.99;
-            S->f_alpha = a2 > 0.0 ? a2 : 0.0;
-          }
-          S->f_zero_v = 0;
-        } else {
-          S->f_dt = tin.f_dt * tin.f_dec;
-          S->f_streak = 0;
-          S->f_alpha = tin.f_alpha0;
-          S->f_zero_v = 1;
-        }
-        S->f_step = tin.f_step + 1;
-      }
-    }
-    if (FM != FM_INIT && FM != FM_OBS && FM != FM_FIRE) {
-      const int64_t steps = tin.steps + 1;
-      S->steps = steps;
-      // an MD segment of a batch ends after its target number of steps
-      if (tin.target_steps > 0 && steps >= tin.target_steps) S->done = 1;
-    }
-  }
+  if (!skip) conv = force_tail<FM, PY>(S, tin, Lx, Ly, h, tot, tmx);
   // (a system that was converged at launch is skipped)
   if (FM == FM_FIRE) S->f_drift = (!skip && !conv) ? 1 : 0;
   S->counter = 0u;
-}
-
-// LN: the launch holds systems with several lanes per slot (the kernel
-// without them keeps the one-lane code only).
-template <int FM, bool PY, bool LN>
-__global__ void __launch_bounds__(kThreads, 4) k_force(Dev D) {
-  force_phase<FM, PY, true, LN>(D, blockIdx.x);
 }
 
 // ------------------------------------------------------------ drift phase --
@@ -1131,12 +1195,167 @@ struct DriftCtx {
   int zero_v, py;
 };
 
-// One particle's drift from its loaded state.
+// Scalars of one drift that its tail writes back to the system.
+struct DriftScalars {
+  double pA1, vp1, aspect;
+  int clamped, boxbad;
+};
+
+// The scalar part of a drift from the system's state (identical in every
+// thread that evaluates it).
+// (BOX = false: the box has not changed since dc was last filled, and its
+// reciprocals are kept.)
+template <int DMd, bool BOX = true>
+__device__ __forceinline__ void drift_prelude(const SysParams& P, const SysState& S, DriftCtx& dc,
+                                              DriftScalars& ds) {
+  const double dt = P.dt, h = 0.5 * dt;
+  const double Lx_old = S.Lx, Ly_old = S.Ly;
+  double Lx = Lx_old, Ly = Ly_old;
+  double xi1 = 0.0, lam = 1.0, vsc = 1.0, pA1 = 0.0, vp1 = 0.0, aspect = S.aspect;
+  int clamped = 0, boxbad = 0;
+  if (DMd == DM_NH) xi1 = nh_xi(P, S.xi, S.K);
+  if (DMd == DM_NPH) {
+    // step_single_NPH (src/md_env.cu:1795-1881)
+    const double A_old = Lx_old * Ly_old;
+    pA1 = S.pA + h * (S.P_cur - S.p_ext);
+    double A_new = A_old + dt * (pA1 / P.W);
+    if (!(A_old > 0.0) || !(A_new > 0.0) || !isfinite(A_new)) boxbad = 1;
+    if (!(aspect > 0.0) || !isfinite(aspect)) aspect = Lx_old / Ly_old;
+    double Ly_new = sqrt(A_new / aspect);
+    double Lx_new = aspect * Ly_new;
+    if (Ly_new < S.fl) {
+      Ly_new = S.fl;
+      Lx_new = aspect * Ly_new;
+      A_new = Lx_new * Ly_new;
+      clamped = 1;
+    } else if (Ly_new > S.ce) {
+      Ly_new = S.ce;
+      Lx_new = aspect * Ly_new;
+      A_new = Lx_new * Ly_new;
+      clamped = 1;
+    }
+    lam = sqrt(A_new / A_old);
+    vsc = 1.0 / lam;
+    if (Lx_new <= 0.0 || Ly_new <= 0.0) boxbad = 1;
+    Lx = Lx_new;
+    Ly = Ly_new;
+  }
+  if (DMd == DM_PISTON) {
+    // step_single_NPH_piston (src/md_env.cu:1939-1989)
+    if (Lx_old <= 0.0 || Ly_old <= 0.0) boxbad = 1;
+    const double a_old = (S.Fp - S.p_ext * Lx_old) / P.W;
+    vp1 = S.vp + h * a_old;
+    double Ly_new = Ly_old + dt * vp1;
+    if (Ly_new < S.fl) {
+      Ly_new = S.fl;
+      clamped = 1;
+      if (vp1 < 0.0) vp1 = 0.0;
+    } else if (Ly_new > S.ce) {
+      Ly_new = S.ce;
+      clamped = 1;
+      if (vp1 > 0.0) vp1 = 0.0;
+    }
+    Ly = Ly_new;
+  }
+  double fdt = 0.0, alpha = 0.0;
+  int zero_v = 0;
+  if (DMd == DM_FIRE) {
+    fdt = S.f_dt;
+    alpha = S.f_alpha;
+    zero_v = S.f_zero_v;
+  }
+  dc.xi1 = xi1;
+  dc.lam = lam;
+  dc.vsc = vsc;
+  dc.fdt = fdt;
+  dc.alpha = alpha;
+  dc.zero_v = zero_v;
+  if (BOX) {
+    dc.dt = dt;
+    dc.h = h;
+    dc.Lx = Lx;
+    dc.Ly = Ly;
+    dc.ilx = 1.0 / Lx;
+    dc.ily = 1.0 / Ly;
+    dc.ilx_old = 1.0 / Lx_old;
+    dc.ily_old = 1.0 / Ly_old;
+    dc.massA = P.massA;
+    dc.massB = P.massB;
+    dc.offx = P.offx;
+    dc.offy = P.offy;
+    dc.py = (S.periodic_y != 0) ? 1 : 0;
+  }
+  ds.pA1 = pA1;
+  ds.vp1 = vp1;
+  ds.aspect = aspect;
+  ds.clamped = clamped;
+  ds.boxbad = boxbad;
+}
+
+// What the rebuild criterion compares with: constants while the box and the
+// cell grid stay.
+struct RebuildLimits {
+  double slop, wx, wy, list, jump;
+};
 template <int DMd>
-__device__ __forceinline__ void drift_particle(const Dev& D, const DriftCtx& c, int64_t i,
-                                               double2 x, double2 v, const double2 a, int t,
-                                               const float2 sb, double& ksum, double& mdx,
-                                               double& mdy, double& mjump, int& bad) {
+__device__ __forceinline__ RebuildLimits rebuild_limits(double Lx, double Ly,
+                                                        const DriftTail& tin) {
+  RebuildLimits r;
+  r.slop = 1e-3 + 4e-7 * fmax(Lx, Ly);
+  r.wx = Lx / (double)tin.ncx;
+  r.wy = (DMd == DM_PISTON) ? (tin.Ly_b / (double)tin.ncy) : Ly / (double)tin.ncy;
+  const double fx = Lx / tin.Lx_b;
+  const double fy = (DMd == DM_PISTON) ? 1.0 : Ly / tin.Ly_b;
+  const double f = fmin(fx, fy);
+  r.list = f * tin.skin - fmax(0.0, 1.0 - f) * tin.rc_max;
+  r.jump = tin.allpairs ? 0.25 * fmin(Lx, Ly) : tin.skin;
+  return r;
+}
+
+// Scalar update of a system after its drift (one thread); returns whether the
+// cell lists must be rebuilt before the next force phase.
+template <int DMd>
+__device__ __forceinline__ int drift_tail(SysState* S, const DriftCtx& dc, const DriftScalars& ds,
+                                          const DriftTail& tin, const RebuildLimits& lim,
+                                          const double (&tot)[kNP], const double (&tmx)[3]) {
+  int need = 0;
+  if (DMd == DM_NH) {
+    S->xi = nh_xi(dc.dt, tin.g_dof, tin.T0, tin.Q, dc.xi1, tot[0]);
+  } else if (DMd == DM_NPH) {
+    S->pA = ds.pA1;
+    S->aspect = ds.aspect;
+    S->Lx = dc.Lx;
+    S->Ly = dc.Ly;
+    S->clamped = ds.clamped;
+  } else if (DMd == DM_PISTON) {
+    S->vp = ds.vp1;
+    S->Ly = dc.Ly;
+    S->clamped = ds.clamped;
+  }
+  // Rebuild criterion. Cell stencil: a pair inside the cutoff now was
+  // within one cell width (per axis) at the last rebuild while
+  // 2*max displacement + rc_max stays below the current cell width.
+  // Neighbour lists (radius rc_ij + skin at the last rebuild): with the
+  // box scaled by f since then, a pair outside the list is still outside
+  // rc while 2*max displacement < f*skin - max(0, 1-f)*rc_max.
+  const double dmax = sqrt(tmx[0] * tmx[0] + tmx[1] * tmx[1]);
+  if (!tin.allpairs) {
+    if (2.0 * tmx[0] + lim.slop + tin.rc_max >= lim.wx) need = 1;
+    if (2.0 * tmx[1] + lim.slop + tin.rc_max >= lim.wy) need = 1;
+    if (2.0 * dmax + lim.slop >= lim.list) need = 1;
+  }
+  if (!(tmx[2] <= lim.jump)) need = 1;  // large single-step moves, NaN
+  return need;
+}
+
+// One particle's drift: x and v move in place; the displacement maxima since
+// the last rebuild (fdx, fdy: as fractions of the box, for periodic axes) and
+// the kinetic sum are the caller's.
+template <int DMd>
+__device__ __forceinline__ void drift_move(const DriftCtx& c, double2& x, double2& v,
+                                           const double2 a, int t, const float2 sb, double& ksum,
+                                           double& mdx, double& mdy, double& mjump, float& fdx,
+                                           float& fdy, int& bad) {
   const double m = t == 0 ? c.massA : c.massB;
   const double2 x0 = x;
   if (DMd == DM_NVE || DMd == DM_PISTON) {
@@ -1180,17 +1399,16 @@ __device__ __forceinline__ void drift_particle(const Dev& D, const DriftCtx& c, 
   const double xu = x.x, yu = x.y;
   x.x = pbc_wrap(x.x, c.Lx);
   if (DMd != DM_PISTON) x.y = pbc_wrap(x.y, c.Ly);
-  D.pos[i] = x;
-  D.vel[i] = v;
-  D.pff[i] = encode_ff(x.x, x.y, t, c.offx, c.offy);
   // displacement since the last rebuild and the single-step jump
   float dsx = (float)(x.x * c.ilx) - sb.x;
   dsx -= rintf(dsx);
+  fdx = fmaxf(fdx, fabsf(dsx));
   const double dxr = (double)fabsf(dsx) * c.Lx;
   double dyr;
   if (c.py && DMd != DM_PISTON) {
     float dsy = (float)(x.y * c.ily) - sb.y;
     dsy -= rintf(dsy);
+    fdy = fmaxf(fdy, fabsf(dsy));
     dyr = (double)fabsf(dsy) * c.Ly;
   } else {
     dyr = fabs(x.y - (double)sb.y);
@@ -1207,10 +1425,21 @@ __device__ __forceinline__ void drift_particle(const Dev& D, const DriftCtx& c, 
   }
 }
 
-// drift_phase is the work of block b of the launch (k_drift: one kernel;
-// k_md_steps: a phase of its multi-step loop).
+template <int DMd>
+__device__ __forceinline__ void drift_particle(const Dev& D, const DriftCtx& c, int64_t i,
+                                               double2 x, double2 v, const double2 a, int t,
+                                               const float2 sb, double& ksum, double& mdx,
+                                               double& mdy, double& mjump, int& bad) {
+  float fdx = 0.f, fdy = 0.f;
+  drift_move<DMd>(c, x, v, a, t, sb, ksum, mdx, mdy, mjump, fdx, fdy, bad);
+  D.pos[i] = x;
+  D.vel[i] = v;
+  D.pff[i] = encode_ff(x.x, x.y, t, c.offx, c.offy);
+}
+
 template <int DMd, bool LN>
-__device__ __forceinline__ void drift_phase(const Dev& D, const int b) {
+__global__ void __launch_bounds__(kThreads, 4) k_drift(Dev D) {
+  const int b = blockIdx.x;
   // (a lone system needs no table lookup: one dependent load less per block)
   const int s = D.nsys == 1 ? 0 : D.sys_of_block[b];
   const SysParams& P = D.sp[s];
@@ -1230,98 +1459,21 @@ __device__ __forceinline__ void drift_phase(const Dev& D, const int b) {
   }
   const bool skip = (S->done != 0) || (S->err != 0) || (DMd == DM_FIRE && S->f_drift == 0);
   constexpr int kNS = (DMd == DM_NH) ? 1 : 0, kNM = 3;
-  const double dt = P.dt, h = 0.5 * dt;
-  const double Lx_old = S->Lx, Ly_old = S->Ly;
-  double Lx = Lx_old, Ly = Ly_old;
-  const bool py = S->periodic_y != 0;
-  // ---- scalar prelude (identical in every block) ----
-  double xi1 = 0.0, lam = 1.0, vsc = 1.0, pA1 = 0.0, vp1 = 0.0, aspect = S->aspect;
-  int clamped = 0, boxbad = 0;
-  if (DMd == DM_NH) xi1 = nh_xi(P, S->xi, S->K);
-  if (DMd == DM_NPH) {
-    // step_single_NPH (src/md_env.cu:1795-1881)
-    const double A_old = Lx_old * Ly_old;
-    pA1 = S->pA + h * (S->P_cur - S->p_ext);
-    double A_new = A_old + dt * (pA1 / P.W);
-    if (!(A_old > 0.0) || !(A_new > 0.0) || !isfinite(A_new)) boxbad = 1;
-    if (!(aspect > 0.0) || !isfinite(aspect)) aspect = Lx_old / Ly_old;
-    double Ly_new = sqrt(A_new / aspect);
-    double Lx_new = aspect * Ly_new;
-    if (Ly_new < S->fl) {
-      Ly_new = S->fl;
-      Lx_new = aspect * Ly_new;
-      A_new = Lx_new * Ly_new;
-      clamped = 1;
-    } else if (Ly_new > S->ce) {
-      Ly_new = S->ce;
-      Lx_new = aspect * Ly_new;
-      A_new = Lx_new * Ly_new;
-      clamped = 1;
-    }
-    lam = sqrt(A_new / A_old);
-    vsc = 1.0 / lam;
-    if (Lx_new <= 0.0 || Ly_new <= 0.0) boxbad = 1;
-    Lx = Lx_new;
-    Ly = Ly_new;
-  }
-  if (DMd == DM_PISTON) {
-    // step_single_NPH_piston (src/md_env.cu:1939-1989)
-    if (Lx_old <= 0.0 || Ly_old <= 0.0) boxbad = 1;
-    const double a_old = (S->Fp - S->p_ext * Lx_old) / P.W;
-    vp1 = S->vp + h * a_old;
-    double Ly_new = Ly_old + dt * vp1;
-    if (Ly_new < S->fl) {
-      Ly_new = S->fl;
-      clamped = 1;
-      if (vp1 < 0.0) vp1 = 0.0;
-    } else if (Ly_new > S->ce) {
-      Ly_new = S->ce;
-      clamped = 1;
-      if (vp1 > 0.0) vp1 = 0.0;
-    }
-    Ly = Ly_new;
-  }
-  double fdt = 0.0, alpha = 0.0;
-  int zero_v = 0;
-  if (DMd == DM_FIRE) {
-    fdt = S->f_dt;
-    alpha = S->f_alpha;
-    zero_v = S->f_zero_v;
-  }
+  DriftCtx dc;
+  DriftScalars ds;
+  drift_prelude<DMd>(P, *S, dc, ds);
   double red[kNP];
 #pragma unroll
   for (int k = 0; k < kNP; ++k) red[k] = 0.0;
   double mx[3] = {0.0, 0.0, 0.0};
   int bad = 0;
-  const double ilx = 1.0 / Lx, ily = 1.0 / Ly;
-  const double ilx_old = 1.0 / Lx_old, ily_old = 1.0 / Ly_old;
   const int items = P.items;
   // a block covers spb slots per pass (kThreads / lanes; the other threads
   // only join the reduction)
   const int spb = LN ? kThreads / P.lanes : kThreads;
   const int64_t base = P.p0 + (int64_t)(b - P.b0) * spb * items + threadIdx.x;
   const int64_t end = (!LN || (int)threadIdx.x < spb) ? P.p0 + P.n : 0;
-  DriftCtx dc;
-  dc.dt = dt;
-  dc.h = h;
-  dc.xi1 = xi1;
-  dc.lam = lam;
-  dc.vsc = vsc;
-  dc.fdt = fdt;
-  dc.alpha = alpha;
-  dc.Lx = Lx;
-  dc.Ly = Ly;
-  dc.ilx = ilx;
-  dc.ily = ily;
-  dc.ilx_old = ilx_old;
-  dc.ily_old = ily_old;
-  dc.massA = P.massA;
-  dc.massB = P.massB;
-  dc.offx = P.offx;
-  dc.offy = P.offy;
-  dc.zero_v = zero_v;
-  dc.py = py ? 1 : 0;
-  if (!skip && !boxbad) {
+  if (!skip && !ds.boxbad) {
 #pragma unroll 1
     for (int it = 0; it < items; ++it) {
       const int64_t i = base + (int64_t)it * spb;
@@ -1339,43 +1491,10 @@ __device__ __forceinline__ void drift_phase(const Dev& D, const int b) {
   if (threadIdx.x != 0) return;
   int need = 0;
   if (!skip) {
-    if (boxbad) {
+    if (ds.boxbad) {
       S->err = 5;  // MDB_ERR_BOX
     } else {
-      if (DMd == DM_NH) {
-        S->xi = nh_xi(dt, tin.g_dof, tin.T0, tin.Q, xi1, tot[0]);
-      } else if (DMd == DM_NPH) {
-        S->pA = pA1;
-        S->aspect = aspect;
-        S->Lx = Lx;
-        S->Ly = Ly;
-        S->clamped = clamped;
-      } else if (DMd == DM_PISTON) {
-        S->vp = vp1;
-        S->Ly = Ly;
-        S->clamped = clamped;
-      }
-      // Rebuild criterion. Cell stencil: a pair inside the cutoff now was
-      // within one cell width (per axis) at the last rebuild while
-      // 2*max displacement + rc_max stays below the current cell width.
-      // Neighbour lists (radius rc_ij + skin at the last rebuild): with the
-      // box scaled by f since then, a pair outside the list is still outside
-      // rc while 2*max displacement < f*skin - max(0, 1-f)*rc_max.
-      const double slop = 1e-3 + 4e-7 * fmax(Lx, Ly);
-      const double wx = Lx / (double)tin.ncx;
-      const double wy = (DMd == DM_PISTON) ? (tin.Ly_b / (double)tin.ncy) : Ly / (double)tin.ncy;
-      const double fx = Lx / tin.Lx_b;
-      const double fy = (DMd == DM_PISTON) ? 1.0 : Ly / tin.Ly_b;
-      const double f = fmin(fx, fy);
-      const double dmax = sqrt(tmx[0] * tmx[0] + tmx[1] * tmx[1]);
-      if (!tin.allpairs) {
-        if (2.0 * tmx[0] + slop + tin.rc_max >= wx) need = 1;
-        if (2.0 * tmx[1] + slop + tin.rc_max >= wy) need = 1;
-        if (2.0 * dmax + slop >= f * tin.skin - fmax(0.0, 1.0 - f) * tin.rc_max) need = 1;
-        if (!(tmx[2] <= tin.skin)) need = 1;  // large single-step moves, NaN
-      } else {
-        need = (!(tmx[2] <= 0.25 * fmin(Lx, Ly))) ? 1 : 0;
-      }
+      need = drift_tail<DMd>(S, dc, ds, tin, rebuild_limits<DMd>(dc.Lx, dc.Ly, tin), tot, tmx);
       if (need) {
         S->need_rebuild = 1;
         atomicOr(&D.bg->any_rebuild, 1);
@@ -1384,123 +1503,6 @@ __device__ __forceinline__ void drift_phase(const Dev& D, const int b) {
   }
   S->counter = 0u;
   system_done_and_signal(D, tin.prior | need);
-}
-
-template <int DMd, bool LN>
-__global__ void __launch_bounds__(kThreads, 4) k_drift(Dev D) {
-  drift_phase<DMd, LN>(D, blockIdx.x);
-}
-
-// ------------------------------------------------------ multi-step kernel --
-// A single system whose blocks are all resident at once (a cooperative
-// launch) runs its steps in one kernel: drift phase, grid barrier, force
-// phase, grid barrier, per step. The phases are the kernels' own block
-// functions with the same blocks, so every sum has the same operands in the
-// same order as with one launch per phase: the results are bit for bit those
-// of the per-phase kernels. The kernel returns after the drift of a step that
-// needs a rebuild; the graph around it rebuilds, runs that step's force phase
-// and launches it again for the remaining steps.
-
-// Polls of a grid-barrier wait before it gives up (at least 32 ns each).
-constexpr unsigned kBarrierSpins = 1u << 22;
-
-// Grid-wide barrier. Thread 0 of each block arrives on a counter; the last
-// arrival resets it and advances the generation (release), the others poll
-// the generation (acquire). A wait that runs out of polls records bar_err
-// and returns; the kernel stops at its next check. That error is final for
-// the handle: the kernel sets the system's err flag, after which every phase
-// skips the system and every call reports it. Each call clears the arrival
-// counter before its first launch (k_md_steps_set), so that a later call on
-// such a handle passes its barriers and stops at once instead of waiting out
-// the polls on arrivals that an abandoned barrier left behind.
-__device__ __forceinline__ void grid_barrier(BatchGlobal* bg, unsigned nblocks) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned gen, prev;
-    __threadfence();  // the block's writes (ordered before by the CTA barrier)
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(gen) : "l"(&bg->bar_gen) : "memory");
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
-                 : "=r"(prev)
-                 : "l"(&bg->bar_count)
-                 : "memory");
-    if (prev == nblocks - 1) {
-      asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(&bg->bar_count), "r"(0u) : "memory");
-      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&bg->bar_gen), "r"(gen + 1u)
-                   : "memory");
-    } else {
-      unsigned cur = gen, polls = 0;
-      do {
-        __nanosleep(32);
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];"
-                     : "=r"(cur)
-                     : "l"(&bg->bar_gen)
-                     : "memory");
-      } while (cur == gen && ++polls < kBarrierSpins);
-      if (cur == gen) atomicExch(&bg->bar_err, 1);
-    }
-    __threadfence();
-  }
-  __syncthreads();
-}
-
-__device__ __forceinline__ int ld_volatile(const int32_t* p) { return *(const volatile int32_t*)p; }
-
-// Runs up to bg->steps_left steps of the single system (grid = its blocks).
-// On return bg->steps_left holds the steps not finished (the step whose
-// drift asked for a rebuild counts as not finished); h_rebuild is set when
-// such a step is pending and h_more while steps remain.
-// (Two blocks per SM: the drift and force phases in one kernel need more
-// than the 64 registers of four, which spilled 270 B; the small systems it
-// serves do not need the occupancy.)
-template <int DMd, int FM, bool LN>
-__global__ void __launch_bounds__(kThreads, 2)
-    k_md_steps(Dev D, cudaGraphConditionalHandle h_more, cudaGraphConditionalHandle h_rebuild) {
-  BatchGlobal* bg = D.bg;
-  const unsigned nb = gridDim.x;
-  const int64_t todo = *(const volatile int64_t*)&bg->steps_left;
-  int64_t done = 0;
-  int rebuild = 0, err = 0;
-  while (done < todo) {
-    drift_phase<DMd, LN>(D, blockIdx.x);
-    grid_barrier(bg, nb);
-    if (ld_volatile(&bg->bar_err)) {
-      err = 1;
-      break;
-    }
-    if (ld_volatile(&bg->any_rebuild)) {
-      rebuild = 1;
-      break;
-    }
-    force_phase<FM, true, false, LN>(D, blockIdx.x);
-    grid_barrier(bg, nb);
-    if (ld_volatile(&bg->bar_err)) {
-      err = 1;
-      break;
-    }
-    ++done;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const int64_t left = todo - done;
-    bg->steps_left = left;
-    if (err) D.st->err = 6;  // MDB_ERR_CUDA: a barrier wait gave up
-    cudaGraphSetConditional(h_rebuild, (rebuild && !err) ? 1u : 0u);
-    cudaGraphSetConditional(h_more, (left > 0 && !err) ? 1u : 0u);
-  }
-}
-
-// After the rebuild and the force phase of the pending step.
-__global__ void k_md_steps_count(Dev D, cudaGraphConditionalHandle h_more) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int64_t left = D.bg->steps_left - 1;
-  D.bg->steps_left = left;
-  cudaGraphSetConditional(h_more, left > 0 ? 1u : 0u);
-}
-
-__global__ void k_md_steps_set(Dev D, int64_t n) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    D.bg->steps_left = n;
-    D.bg->bar_count = 0u;  // no multi-step block runs now (stream order)
-  }
 }
 
 // K = sum 1/2 m |v|^2 (cal_local_K_kernel src/md_cuda_common.cu:554-589) into
