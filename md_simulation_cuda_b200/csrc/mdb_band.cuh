@@ -1,0 +1,677 @@
+// Force phase and list build over staged bands: for systems too large for the
+// resident steps kernel and for batches.
+//
+// A chunk is 256 consecutive slots of a system. Slots are sorted by cell, cells
+// by rows, so what a chunk's particles can meet are a few contiguous slot
+// ranges: the chunk's own stretch of its cell row and the same stretch of the
+// rows above and below, one cell wider on each side (four rows in two pieces
+// each where the chunk runs over the end of a row; whole rows where those are
+// short). This band, ~850 positions of 16 bytes, is what the block copies into
+// shared memory with one bulk copy per range (cp.async.bulk, completion on an
+// mbarrier), the next chunk's band while it works on this one.
+//
+// Why: the force phase was bound by waiting, not by issue (55% of the cycles) or
+// bytes (15% of HBM): each list entry is an index load and then a gather through
+// L1 that missed to L2 in 28% of its sectors, and a slot's last entries were
+// taken one at a time. From a staged band a gather costs ~30 cycles, an entry
+// is a 16-bit index into the band (no wrap, no 64-bit address), four entries
+// arrive in one 8-byte load, and lists are padded to groups of four with the
+// slot itself (r^2 = 0, which the pair term skips), so that no lane runs a
+// remainder loop. The candidates, their order and the arithmetic are those of
+// k_force: the results are the same bits.
+#pragma once
+
+#include "mdb_kernels.cuh"
+
+namespace mdb {
+
+// ------------------------------------------------------- asynchronous copy --
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+// Waits for the phase of the given parity; false when it ran out of tries
+// (each of which the hardware suspends for a while).
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+  for (unsigned tries = 0; tries < (1u << 22); ++tries) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// Copies n positions (16 bytes each, so every address and size is a multiple
+// of 16) to shared memory; completion counts on bar.
+__device__ __forceinline__ void copy_positions(float4* dst, const float4* src, int n,
+                                               uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          smem_addr(dst)),
+      "l"(src), "r"((uint32_t)n * 16u), "r"(smem_addr(bar))
+      : "memory");
+}
+
+// ------------------------------------------------------------------- bands --
+
+// First and one-past-last cell of piece r of the band of a chunk whose slots lie
+// in the cells from (x0, y0) to (x1, y1) of an ncx x ncy grid; the number of
+// pieces through nr. Pieces are disjoint runs of cells in slot order, and every
+// run of stencil cells that a slot of the chunk visits lies inside one of them:
+//  * full: whole rows y0 - 1 .. y1 + 1 (every row when that covers the grid),
+//    as one run, split where it passes the periodic edge;
+//  * one row: the cells x0 - 1 .. x1 + 1 of three rows, and for an end cell of
+//    the row the cell across the edge;
+//  * two rows (y1 = y0 + 1): of four rows the cells 0 .. x1 + 1 and
+//    x0 - 1 .. ncx - 1.
+// Rows beyond a walled y axis are empty.
+struct BandShape {
+  int x0, y0, x1, y1, ncx, ncy;
+  bool py, full;
+};
+__device__ __forceinline__ int band_pieces(const BandShape& s) {
+  if (s.full) return 3;
+  return s.y1 == s.y0 ? 6 : 8;
+}
+__device__ __forceinline__ bool band_piece(const BandShape& s, int r, int* c0, int* c1) {
+  if (s.full) {
+    int lo = s.y0 - 1, hi = s.y1 + 1;
+    if (hi - lo + 1 >= s.ncy || !s.py) {
+      lo = max(lo, 0);
+      hi = min(hi, s.ncy - 1);
+      if (s.py) {
+        lo = 0;
+        hi = s.ncy - 1;
+      }
+      *c0 = lo * s.ncx;
+      *c1 = (hi + 1) * s.ncx;
+      return r == 0;
+    }
+    // rows below the edge, in the grid, above the edge
+    if (r == 0) {
+      *c0 = (lo + s.ncy) * s.ncx;
+      *c1 = s.ncy * s.ncx;
+      return lo < 0;
+    }
+    if (r == 1) {
+      *c0 = max(lo, 0) * s.ncx;
+      *c1 = (min(hi, s.ncy - 1) + 1) * s.ncx;
+      return true;
+    }
+    *c0 = 0;
+    *c1 = (hi - s.ncy + 1) * s.ncx;
+    return hi >= s.ncy;
+  }
+  int y, a, b;
+  bool some = true;
+  if (s.y1 == s.y0) {
+    y = s.y0 - 1 + r / 2;
+    const int lo = max(s.x0 - 1, 0), hi = min(s.x1 + 1, s.ncx - 1);
+    if ((r & 1) == 0) {
+      a = lo;
+      b = hi;
+    } else {
+      // the cell across the edge, unless the run holds it
+      a = b = (s.x0 == 0) ? s.ncx - 1 : 0;
+      some = (s.x0 == 0 || s.x1 == s.ncx - 1) && !(a >= lo && a <= hi);
+    }
+  } else {
+    y = s.y0 - 1 + r / 2;
+    const int left = min(s.x1 + 1, s.ncx - 1), right = max(s.x0 - 1, 0);
+    const bool joined = right <= left + 1;
+    if ((r & 1) == 0) {
+      a = 0;
+      b = joined ? s.ncx - 1 : left;
+    } else {
+      a = right;
+      b = s.ncx - 1;
+      some = !joined;
+    }
+  }
+  if (y < 0 || y >= s.ncy) {
+    if (!s.py) some = false;
+    y += (y < 0) ? s.ncy : -s.ncy;
+  }
+  *c0 = y * s.ncx + a;
+  *c1 = y * s.ncx + b + 1;
+  return some;
+}
+
+// Computed by warp 0 of a block for the chunk that starts at slot cs: the
+// band's ranges into *b (shared or global memory). total = 0: no band (it
+// would exceed kBandCap).
+__device__ __forceinline__ void make_band(const Dev& D, const SysParams& P, const SysState& S,
+                                          int64_t cs, Band* b) {
+  const int lane = threadIdx.x & 31;
+  const int64_t last = min(cs + kThreads, P.p0 + P.n) - 1;
+  BandShape s;
+  s.ncx = S.ncx;
+  s.ncy = S.ncy;
+  s.py = S.periodic_y != 0;
+  const int f = D.cell_of[cs], l = D.cell_of[last];
+  s.x0 = f % s.ncx;
+  s.y0 = f / s.ncx;
+  s.x1 = l % s.ncx;
+  s.y1 = l / s.ncx;
+  const int32_t* cst = D.cstart + P.c0;
+  // whole rows when they fit (one run), or when the chunk spans more than two
+  {
+    const int lo = max(s.y0 - 1, 0), hi = min(s.y1 + 1, s.ncy - 1);
+    int rows = cst[(hi + 1) * s.ncx] - cst[lo * s.ncx];
+    if (s.py && s.y0 == 0) rows += cst[s.ncy * s.ncx] - cst[(s.ncy - 1) * s.ncx];
+    if (s.py && s.y1 == s.ncy - 1) rows += cst[s.ncx] - cst[0];
+    s.full = s.y1 > s.y0 + 1 || rows <= kBandCap;
+    // (three rows or fewer on a side: pieces could meet across the edge)
+    if (s.ncy < 5) s.full = true;
+  }
+  const int np = band_pieces(s);
+  int start = 0, len = 0;
+  if (lane < np) {
+    int c0, c1;
+    if (band_piece(s, lane, &c0, &c1)) {
+      start = cst[c0];
+      len = cst[c1] - start;
+    }
+  }
+  int end = len;
+#pragma unroll
+  for (int o = 1; o < kBandRanges; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, end, kBandRanges - 1);
+  const bool fits = total <= kBandCap;
+  if (lane < kBandRanges) {
+    b->start[lane] = start;
+    b->len[lane] = fits ? len : 0;
+    b->off[lane] = end - len;
+  }
+  if (lane == 0) b->total = fits ? total : 0;
+}
+
+// Place in the band of slot j (which some range holds).
+__device__ __forceinline__ int band_place(const Band& b, int j) {
+  int at = 0;
+#pragma unroll
+  for (int r = 0; r < kBandRanges; ++r) {
+    const int d = j - b.start[r];
+    if (d >= 0 && d < b.len[r]) at = b.off[r] + d;
+  }
+  return at;
+}
+
+// ---------------------------------------------------------- rebuild: lists --
+
+// The list of the slot at place `self` of a staged band (cell cx, cy): whole
+// groups go to out, the last one stays in g0, g1. Returns the count.
+template <bool MIC>
+__device__ __forceinline__ int build_band_list(const Dev& D, const SysParams& P, const SysState& S,
+                                               const Band& band, const float4* pos, int self,
+                                               int cx, int cy, bool py, uint2* out, uint32_t& g0,
+                                               uint32_t& g1) {
+  const int ncx = S.ncx, ncy = S.ncy;
+  PairCtx c;
+  const float4 qi = pos[self];
+  if (py)
+    set_pair_box<true>(c, qi, S.Lx, S.Ly);
+  else
+    set_pair_box<false>(c, qi, S.Lx, S.Ly);
+  const uint32_t tci = ff_class(qi);
+  const uint32_t ts = (tci == 2u) ? 99u : tci;
+  const float rl2s = P.frl2[tci == 2u ? 2 : tci], rl2ab = P.frl2[2];
+  const int maxn = D.max_nbr;
+  const int32_t* cst = D.cstart + P.c0;
+  int cnt = 0;
+  // one run of stencil cells: slots [a, e), contiguous in the band
+  auto scan = [&](int a, int e) {
+    const int at = band_place(band, a);
+    const int len = e - a;
+    for (int m = 0; m < len; m += 4) {
+      float4 qq[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) qq[u] = pos[at + (m + u < len ? m + u : 0)];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float2 dd;
+        const float r2 = pair_r2<MIC>(qq[u], c, dd);
+        const float rl2 = (ff_class(qq[u]) == ts) ? rl2s : rl2ab;
+        const int place = at + m + u;
+        if (r2 < rl2 && place != self && m + u < len) {
+          const uint32_t v = (uint32_t)place << (16 * (cnt & 1));
+          if ((cnt & 2) == 0) g0 |= v; else g1 |= v;
+          if ((cnt & 3) == 3) {
+            if (cnt < maxn) out[(int64_t)(cnt >> 2) * D.ntot] = make_uint2(g0, g1);
+            g0 = g1 = 0;
+          }
+          ++cnt;
+        }
+      }
+    }
+  };
+  for (int dr = -1; dr <= 1; ++dr) {
+    int yy = cy + dr;
+    if (py) {
+      if (yy < 0) yy += ncy;
+      if (yy >= ncy) yy -= ncy;
+    } else if (yy < 0 || yy >= ncy) {
+      continue;
+    }
+    const int32_t* row = cst + (int64_t)yy * ncx;
+    // (interior slots have the one run)
+    const bool mid = !MIC || (cx > 0 && cx < ncx - 1);
+    scan(row[mid ? cx - 1 : (cx == 0 ? 0 : ncx - 2)], row[mid ? cx + 2 : (cx == 0 ? 2 : ncx)]);
+    if (!mid) scan(row[cx == 0 ? ncx - 1 : 0], row[cx == 0 ? ncx : 1]);
+  }
+  return cnt;
+}
+
+// Bands of every chunk of the systems that rebuild, and their slots' lists:
+// entry e of slot k is the place of its partner in the chunk's band, 16 bits at
+// lists[((e / 4) * ntot + k) * 4 + e % 4], whole groups of four padded with the
+// slot's own place. One block per chunk in turn; the candidates are read from
+// the staged band. The entries, their order and the count are those of
+// build_list.
+__global__ void __launch_bounds__(kThreads) k_rb_band(Dev D) {
+  if (!rebuild_requested(D)) return;
+  extern __shared__ __align__(128) float4 sh_band[];
+  __shared__ Band band;
+  __shared__ __align__(8) uint64_t full;
+  const bool forced = *((volatile int*)&D.bg->forced) != 0;
+  if (threadIdx.x == 0) mbar_init(&full, 1);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncthreads();
+  uint32_t parity = 0;
+  for (int64_t q = blockIdx.x; q < D.nchunks; q += gridDim.x) {
+    const int s = D.sys_of_chunk[q];
+    if (!sys_rebuilds(D, s)) continue;  // (the whole block)
+    const SysParams& P = D.sp[s];
+    SysState* S = D.st + s;
+    const int64_t cs = P.p0 + (q - P.ch0) * kThreads;
+    const int64_t k = cs + threadIdx.x;
+    const bool act = k < P.p0 + P.n;
+    // a system that rebuilds again within kListMinReuse steps scans its cell
+    // stencil instead of a list it would hardly reuse
+    const bool recent = !forced && rebuild_clock(P, *S) - S->rb_last < kListMinReuse;
+    const bool lists = !S->allpairs && D.max_nbr > 0 && !recent;
+    if (threadIdx.x < 32) {
+      if (!S->allpairs) {
+        make_band(D, P, *S, cs, &band);
+      } else if (threadIdx.x < kBandRanges) {
+        band.start[threadIdx.x] = band.len[threadIdx.x] = band.off[threadIdx.x] = 0;
+        if (threadIdx.x == 0) band.total = 0;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < (int)(sizeof(Band) / 4))
+      ((int32_t*)(D.bands + q))[threadIdx.x] = ((const int32_t*)&band)[threadIdx.x];
+    if (band.total == 0 || !lists) {
+      if (act) D.ncount[k] = -1;
+      if (threadIdx.x == 0 && lists)  // the chunk's particles scan their stencils
+        atomicAdd(&S->nl_overflow, (int)min((int64_t)kThreads, P.p0 + P.n - cs));
+      __syncthreads();  // (the band is rewritten for the next chunk)
+      continue;
+    }
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0) mbar_expect(&full, (uint32_t)band.total * 16u);
+      __syncwarp();
+      if (threadIdx.x < kBandRanges && band.len[threadIdx.x] > 0)
+        copy_positions(sh_band + band.off[threadIdx.x], D.pff + band.start[threadIdx.x],
+                       band.len[threadIdx.x], &full);
+    }
+    const bool here = mbar_wait(&full, parity);
+    parity ^= 1u;
+    if (!here) {
+      if (act) D.ncount[k] = -1;
+      atomicExch(&D.bg->bar_err, 1);
+      S->err = 6;  // MDB_ERR_CUDA: the copy never arrived
+    } else if (act) {
+      const int cell = D.cell_of[k];
+      const int cx = cell % S->ncx, cy = cell / S->ncx;
+      const bool py = S->periodic_y != 0;
+      const bool interior =
+          cx >= 2 && cx <= S->ncx - 3 && (!py || (cy >= 2 && cy <= S->ncy - 3));
+      const int self = band_place(band, (int)k);
+      const int maxn = D.max_nbr;
+      uint32_t g0 = 0, g1 = 0;
+      uint2* out = D.lists + k;
+      const int cnt = interior ? build_band_list<false>(D, P, *S, band, sh_band, self, cx, cy, py,
+                                                        out, g0, g1)
+                               : build_band_list<true>(D, P, *S, band, sh_band, self, cx, cy, py,
+                                                       out, g0, g1);
+      if (cnt > maxn) {
+        D.ncount[k] = -1;  // too many neighbours: the force loop scans the stencil
+        atomicAdd(&S->nl_overflow, 1);
+      } else {
+        if ((cnt & 3) != 0) {
+          const uint32_t pad = (uint32_t)self | ((uint32_t)self << 16);
+          const int r = cnt & 3;
+          if (r == 1) g0 |= (uint32_t)self << 16;
+          if (r <= 2) g1 = pad;
+          if (r == 3) g1 |= (uint32_t)self << 16;
+          out[(int64_t)(cnt >> 2) * D.ntot] = make_uint2(g0, g1);
+        }
+        D.ncount[k] = cnt | (interior ? kListInterior : 0);
+      }
+    }
+    __syncthreads();  // every thread is done with the band
+  }
+}
+
+// ------------------------------------------------------------- force phase --
+
+// Pair sums over a slot's list in the staged band.
+template <bool PY, bool ENERGY, bool VIRIAL, bool MIC, bool FLOOR>
+__device__ __forceinline__ void band_list(const float4* __restrict__ band,
+                                          const uint2* __restrict__ list, int64_t ntot, int groups,
+                                          const PairCtx& c, float2& fs, float2& fc, float& ws,
+                                          float& wc, double& u, double& an) {
+  uint2 e = groups > 0 ? __ldg(list) : make_uint2(0u, 0u);
+  for (int g = 0; g < groups; ++g) {
+    const float4 q0 = band[e.x & 0xffffu], q1 = band[e.x >> 16];
+    const float4 q2 = band[e.y & 0xffffu], q3 = band[e.y >> 16];
+    list += ntot;
+    if (g + 1 < groups) e = __ldg(list);  // the next group's entries
+    pair_one<PY, ENERGY, VIRIAL, MIC, FLOOR>(q0, c, fs, fc, ws, wc, u, an);
+    pair_one<PY, ENERGY, VIRIAL, MIC, FLOOR>(q1, c, fs, fc, ws, wc, u, an);
+    pair_one<PY, ENERGY, VIRIAL, MIC, FLOOR>(q2, c, fs, fc, ws, wc, u, an);
+    pair_one<PY, ENERGY, VIRIAL, MIC, FLOOR>(q3, c, fs, fc, ws, wc, u, an);
+  }
+}
+
+// The same with FP64 pair terms.
+template <bool PY, bool ENERGY, bool VIRIAL, bool MIC>
+__device__ __forceinline__ void band_list_hp(const float4* band, const uint2* __restrict__ list,
+                                             int64_t ntot, int groups, const PairCtxD& c,
+                                             double& fx, double& fy, double& w, double& u,
+                                             double& an) {
+  for (int g = 0; g < groups; ++g, list += ntot) {
+    const uint2 e = __ldg(list);
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t at = ((k < 2 ? e.x : e.y) >> (16 * (k & 1))) & 0xffffu;
+      pair_one_hp<PY, ENERGY, VIRIAL, MIC>(band[at], c, fx, fy, w, u, an);
+    }
+  }
+}
+
+// Shared state of a block of k_force_band beside its two bands.
+struct BandShared {
+  Band bands[2];
+  uint64_t full[2], empty[2];
+  int lost;  // a wait ran out of tries
+};
+
+// Run r of the stencil of cell (cx, cy), in visiting order: two runs a row, the
+// second across the periodic x edge. Global slots [a, e); false: no such run.
+template <bool PY>
+__device__ __forceinline__ bool stencil_run(const int32_t* cst, int ncx, int ncy, int cx, int cy,
+                                            int r, int* a, int* e) {
+  int y = cy - 1 + (r >> 1);
+  if (PY) {
+    if (y < 0) y += ncy;
+    if (y >= ncy) y -= ncy;
+  } else if (y < 0 || y >= ncy) {
+    return false;
+  }
+  const int32_t* row = cst + (int64_t)y * ncx;
+  const bool mid = cx > 0 && cx < ncx - 1;
+  if ((r & 1) != 0) {
+    if (mid) return false;
+    *a = __ldg(row + (cx == 0 ? ncx - 1 : 0));
+    *e = __ldg(row + (cx == 0 ? ncx : 1));
+    return true;
+  }
+  *a = __ldg(row + (mid ? cx - 1 : (cx == 0 ? 0 : ncx - 2)));
+  *e = __ldg(row + (mid ? cx + 2 : (cx == 0 ? 2 : ncx)));
+  return true;
+}
+
+// The chunks of one block: pair sums and what follows them, into fin. HP: FP64
+// pair terms (a FIRE system past its switch point, and its observations).
+template <int FM, bool PY, bool HP>
+__device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, const SysState& S,
+                                           BandShared& sh, float4* sh_band, int q_first, int items,
+                                           ForceFinish<FM, PY>& fin) {
+  constexpr bool kEnergy = (FM == FM_OBS);
+  constexpr bool kVirial = (FM == FM_OBS || FM == FM_NPH);
+  constexpr bool kFloor = (FM == FM_FIRE || FM == FM_OBS || FM == FM_INIT);
+  const int nb = P.nb;
+  const int64_t end = P.p0 + P.n;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // Chunk of a pass: pass it takes chunk it * nb + rot, rot advancing by half
+  // the blocks per pass (a block's chunks spread over the system, each pass
+  // still covering one contiguous stretch).
+  int rot = q_first;
+  auto next_rot = [&](int r) {
+    r += nb / 2;
+    return r >= nb ? r - nb : r;
+  };
+  // Starts the copy of a chunk's band into buffer buf (warp 0).
+  auto stage = [&](int q, int buf) {
+    Band* bd = sh.bands + buf;
+    const Band* g = D.bands + P.ch0 + q;
+    int st = 0, ln = 0, of = 0;
+    if (lane < kBandRanges) {
+      st = g->start[lane];
+      ln = g->len[lane];
+      of = g->off[lane];
+      bd->start[lane] = st;
+      bd->len[lane] = ln;
+      bd->off[lane] = of;
+    }
+    const int total = g->total;
+    if (lane == 0) bd->total = total;
+    __syncwarp();
+    // (the arrival also releases the ranges to the warps that wait for the copy)
+    if (lane == 0) mbar_expect(sh.full + buf, (uint32_t)total * 16u);
+    __syncwarp();
+    if (lane < kBandRanges && ln > 0)
+      copy_positions(sh_band + buf * kBandCap + of, D.pff + st, ln, sh.full + buf);
+  };
+  if (warp == 0 && items > 0) stage(q_first, 0);
+  const double Lx = S.Lx, Ly = S.Ly;
+  const double h = 0.5 * P.dt;
+  const double xi2 = (FM == FM_NH) ? S.xi : 0.0;
+  const double fdt = (FM == FM_FIRE) ? S.f_dt : 0.0;
+#pragma unroll 1
+  for (int it = 0; it < items; ++it) {
+    const int buf = it & 1;
+    const int64_t cs = P.p0 + (int64_t)(it * nb + rot) * kThreads;
+    if (cs >= end) break;  // (every thread of the block agrees)
+    const int64_t i = cs + threadIdx.x;
+    const bool act = i < end;
+    const int nc = act ? __ldg(D.ncount + i) : -1;
+    rot = next_rot(rot);
+    {
+      const int q = (it + 1) * nb + rot;
+      const int64_t ncs = P.p0 + (int64_t)q * kThreads;
+      if (it + 1 < items && ncs < end) {
+        if (warp == 0) {
+          // the other buffer: free once every warp has left pass it - 1
+          if (it > 0 && !mbar_wait(sh.empty + (buf ^ 1), (uint32_t)((it - 1) >> 1) & 1u))
+            sh.lost = 1;
+          stage(q, buf ^ 1);
+        }
+        // L1 prefetch of the next chunk's list groups (32 slots of a group are
+        // two lines), counts and velocities
+        const int64_t wslot = ncs + (threadIdx.x & ~31);
+        if (wslot < end) {
+          if (lane * 2 < D.pf_rows && (lane >> 1) * 4 < D.max_nbr)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(D.lists + (int64_t)(lane >> 1) * D.ntot +
+                                                           wslot + (lane & 1) * 16));
+          if (ncs + threadIdx.x < end) {
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(D.ncount + ncs + threadIdx.x));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(D.vel + ncs + threadIdx.x));
+          }
+        }
+      }
+    }
+    if (!mbar_wait(sh.full + buf, (uint32_t)(it >> 1) & 1u)) sh.lost = 1;
+    const float4* band = sh_band + buf * kBandCap;
+    double fx = 0.0, fy = 0.0, w = 0.0, u = 0.0, an = 0.0;
+    int tci = 0;
+    if (act) {
+      const bool staged = sh.bands[buf].total > 0;
+      const float4 qi = staged ? band[band_place(sh.bands[buf], (int)i)] : __ldg(D.pff + i);
+      tci = (int)ff_class(qi);
+      PairCtx c;
+      PairCtxD cd;
+      float2 fs = make_float2(0.f, 0.f), fc = make_float2(0.f, 0.f);
+      float ws = 0.f, wc = 0.f;
+      if (HP) {
+        cd = pair_ctx_hp(P, qi, Lx, Ly);
+      } else {
+        c.ih = make_float2(qi.x, qi.y);
+        c.il = make_float2(qi.z, qi.w);
+        set_pair_class<kFloor>(c, P, tci);
+      }
+      const int groups = ((nc & (kListInterior - 1)) + 3) >> 2;
+      if (nc >= 0 && (nc & kListInterior) != 0) {
+        if (HP)
+          band_list_hp<PY, kEnergy, kVirial, false>(band, D.lists + i, D.ntot, groups, cd, fx, fy,
+                                                    w, u, an);
+        else
+          band_list<PY, kEnergy, kVirial, false, kFloor>(band, D.lists + i, D.ntot, groups, c, fs,
+                                                         fc, ws, wc, u, an);
+      } else {
+        if (!HP) set_pair_box<PY>(c, qi, Lx, Ly);
+        if (nc >= 0) {
+          if (HP)
+            band_list_hp<PY, kEnergy, kVirial, true>(band, D.lists + i, D.ntot, groups, cd, fx, fy,
+                                                     w, u, an);
+          else
+            band_list<PY, kEnergy, kVirial, true, kFloor>(band, D.lists + i, D.ntot, groups, c, fs,
+                                                          fc, ws, wc, u, an);
+        } else {
+          // no list: the stencil's runs from the band (or, without one, from
+          // global memory), or the whole system
+          const int cell = S.allpairs ? 0 : D.cell_of[i];
+          const int cx = cell % S.ncx, cy = cell / S.ncx;
+#pragma unroll 1
+          for (int r = 0; r < 6; ++r) {
+            int a, e;
+            if (S.allpairs) {
+              if (r > 0) break;
+              a = (int)P.p0;
+              e = (int)end;
+            } else if (!stencil_run<PY>(D.cstart + P.c0, S.ncx, S.ncy, cx, cy, r, &a, &e)) {
+              continue;
+            }
+            const float4* src = staged ? band + band_place(sh.bands[buf], a) : D.pff + a;
+            const int len = e - a;
+#pragma unroll 1
+            for (int m = 0; m < len; m += 4) {
+              float4 q[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) q[k] = m + k < len ? src[m + k] : qi;
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                if (HP)
+                  pair_one_hp<PY, kEnergy, kVirial, true>(q[k], cd, fx, fy, w, u, an);
+                else
+                  pair_one<PY, kEnergy, kVirial, true, kFloor>(q[k], c, fs, fc, ws, wc, u, an);
+              }
+            }
+          }
+        }
+      }
+      if (HP) {
+        w = 0.5 * w;
+      } else {
+        fx = (double)fs.x - (double)fc.x;
+        fy = (double)fs.y - (double)fc.y;
+        w = 0.5 * ((double)ws - (double)wc);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(sh.empty + buf);  // this warp has left the band
+    if (act) fin(D, P, Ly, h, xi2, fdt, i, fx, fy, w, u, an, tci);
+  }
+}
+
+// The FP64 form out of line: its registers do not count against the FP32 loop.
+template <int FM, bool PY>
+__device__ __noinline__ ForceFinish<FM, PY> band_items_hp(Dev D, const SysParams* P,
+                                                          const SysState* S, BandShared* sh,
+                                                          float4* sh_band, int q_first,
+                                                          int items) {
+  ForceFinish<FM, PY> fin;
+  fin.init();
+  band_items<FM, PY, true>(D, *P, *S, *sh, sh_band, q_first, items, fin);
+  return fin;
+}
+
+// The force phase of k_force over staged bands: the same blocks, chunks,
+// reductions and scalar tail.
+template <int FM, bool PY>
+__global__ void __launch_bounds__(kThreads, 4) k_force_band(Dev D) {
+  extern __shared__ __align__(128) float4 sh_band[];  // [2][kBandCap]
+  __shared__ BandShared sh;
+  const int b = blockIdx.x;
+  const int s = D.nsys == 1 ? 0 : D.sys_of_block[b];
+  const SysParams& P = D.sp[s];
+  SysState* S = D.st + s;
+  constexpr bool kHpCapable = (FM == FM_FIRE || FM == FM_OBS || FM == FM_INIT);
+  constexpr int kNS = ForceRed<FM>::NS, kNM = ForceRed<FM>::NM;
+  if (threadIdx.x == 0) {
+    mbar_init(sh.full + 0, 1);
+    mbar_init(sh.full + 1, 1);
+    mbar_init(sh.empty + 0, kThreads / 32);
+    mbar_init(sh.empty + 1, kThreads / 32);
+    sh.lost = 0;
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  // a finished batch system is still observed (FM_OBS) and re-evaluated (FM_INIT)
+  const bool skip = (FM != FM_OBS && FM != FM_INIT && S->done != 0) || (S->err != 0) ||
+                    (FM == FM_FIRE && (S->f_conv != 0 || S->f_step >= P.f_max_steps));
+  const double Lx = S->Lx, Ly = S->Ly;
+  const int items = skip ? 0 : P.items;
+  __syncthreads();
+  ForceFinish<FM, PY> fin;
+  if (kHpCapable && S->f_fp64 != 0) {
+    fin = band_items_hp<FM, PY>(D, &P, S, &sh, sh_band, b - P.b0, items);
+  } else {
+    fin.init();
+    band_items<FM, PY, false>(D, P, *S, sh, sh_band, b - P.b0, items, fin);
+  }
+  if (fin.bad) atomicOr(&S->nonfinite, 1);
+  ForceTail tin;
+  if (threadIdx.x == 0) tin = force_tail_inputs<FM>(P, S);
+  double tot[kNP];
+  double tmx[3];
+  if (!reduce_system<kNS, kNM>(D, P, S, fin.red, fin.mx, tot, tmx)) {
+    if (threadIdx.x == 0 && sh.lost) {
+      atomicExch(&D.bg->bar_err, 1);
+      S->err = 6;  // MDB_ERR_CUDA: a band never arrived
+    }
+    return;
+  }
+  if (threadIdx.x != 0) return;
+  int conv = 0;
+  if (!skip) conv = force_tail<FM, PY>(S, tin, Lx, Ly, 0.5 * P.dt, tot, tmx);
+  // (a system that was converged at launch is skipped)
+  if (FM == FM_FIRE) S->f_drift = (!skip && !conv) ? 1 : 0;
+  if (sh.lost) {
+    atomicExch(&D.bg->bar_err, 1);
+    S->err = 6;
+  }
+  S->counter = 0u;
+}
+
+}  // namespace mdb

@@ -14,12 +14,17 @@
 #include <string>
 
 #include "mdb_engine.h"
+#include "mdb_band.cuh"
 #include "mdb_kernels.cuh"
 #include "mdb_steps.cuh"
 #include "mdb_util.h"
 
 namespace mdb {
 
+namespace {
+
+// Kernel of a force phase (FM_*; py: periodic y); ln: the launch holds systems
+// with several lanes per slot.
 void* force_fn(int fm, bool py, bool ln) {
 #define MDB_F(M)                                                                 \
   return ln ? (py ? (void*)k_force<M, true, true> : (void*)k_force<M, false, true>) \
@@ -35,6 +40,33 @@ void* force_fn(int fm, bool py, bool ln) {
     default: MDB_F(FM_OBS);
   }
 #undef MDB_F
+}
+
+void* force_band_fn(int fm, bool py) {
+#define MDB_F(M) return py ? (void*)k_force_band<M, true> : (void*)k_force_band<M, false>
+  switch (fm) {
+    case FM_INIT: MDB_F(FM_INIT);
+    case FM_NVE: MDB_F(FM_NVE);
+    case FM_NH: MDB_F(FM_NH);
+    case FM_NPH: MDB_F(FM_NPH);
+    case FM_PISTON: MDB_F(FM_PISTON);
+    case FM_FIRE: MDB_F(FM_FIRE);
+    default: MDB_F(FM_OBS);
+  }
+#undef MDB_F
+}
+
+}  // namespace
+
+Engine::Kernel Engine::force_kernel(int fm, bool py) const {
+  if (banded_)
+    return {force_band_fn(fm, py), nblocks_, kThreads, sizeof(float4) * 2 * kBandCap};
+  return {force_fn(fm, py, lanes_), nblocks_, kThreads, 0};
+}
+
+Engine::Kernel Engine::list_kernel() const {
+  if (banded_) return {(void*)k_rb_band, nlist_grid_, kThreads, sizeof(float4) * kBandCap};
+  return {(void*)k_rb_nlist, nlist_grid_, kThreads, 0};
 }
 
 void* drift_fn(int dm, bool ln) {
@@ -163,7 +195,7 @@ int Engine::build() {
     skin_ = all_fire ? kSkinFire : kSkinMD;
   }
   int64_t p0 = 0, c0 = 0;
-  int b0 = 0;
+  int b0 = 0, ch0 = 0;
   int64_t maxn = 0;
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device_);
@@ -197,6 +229,7 @@ int Engine::build() {
     if (P.lanes > 1) lanes_ = true;
     P.nb = (n + spb * P.items - 1) / (spb * P.items);
     P.b0 = b0;
+    P.ch0 = ch0;
     P.kind = sp.kind;
     P.sig[0] = c.SIGMA_AA;
     P.sig[1] = c.SIGMA_BB;
@@ -277,6 +310,7 @@ int Engine::build() {
     S.rb_last = kNoRebuildYet;
     p0 += n;
     b0 += P.nb;
+    ch0 += (n + kThreads - 1) / kThreads;
     c0 += (int64_t)P.ccap_x * P.ccap_y;
   }
   ntot_ = p0;
@@ -336,7 +370,23 @@ int Engine::build() {
     const double rows = std::max(1.0, floor(hsp_[s].Ly0 / hsp_[s].r_cell));
     if (3.0 * hsp_[s].n / rows >= 30000.0) D.nl16 = 0;
   }
-  if (max_nbr_ > 0) {
+  D.nsys = ns;
+  D.nblocks = nblocks_;
+  D.ntot = ntot_;
+  D.ncells = ncells_;
+  rc = choose_multi_step();
+  if (rc) return rc;
+  // Systems that do not run in the resident steps kernel take the staged bands
+  // (one lane per slot).
+  banded_ = !multi_step_ && !lanes_;
+  int32_t* soc = nullptr;
+  if (banded_) {
+    D.nchunks = ch0;
+    MDB_ALLOC(soc, ch0);
+    D.sys_of_chunk = soc;
+    MDB_ALLOC(D.bands, ch0);
+    if (max_nbr_ > 0) MDB_ALLOC(D.lists, (int64_t)((max_nbr_ + 3) / 4) * ntot_);
+  } else if (max_nbr_ > 0) {
     if (D.nl16)
       MDB_ALLOC(D.nlist16, (int64_t)max_nbr_ * ntot_);
     else
@@ -357,10 +407,6 @@ int Engine::build() {
     if (rc2) return rc2;
   }
 #undef MDB_ALLOC
-  D.nsys = ns;
-  D.nblocks = nblocks_;
-  D.ntot = ntot_;
-  D.ncells = ncells_;
   D.use_cond = 0;
   const int64_t work = std::max(ntot_, ncells_);
   rb_grid_ = (int)std::min<int64_t>((work + kThreads - 1) / kThreads, (int64_t)nsm * 8);
@@ -374,8 +420,9 @@ int Engine::build() {
   // so that no SM is left with a partial second wave.
   {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_rb_nlist, kThreads,
-                                                      0) != cudaSuccess ||
+    const Kernel lk = list_kernel();
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lk.fn, kThreads, lk.smem) !=
+            cudaSuccess ||
         per_sm <= 0) {
       (void)cudaGetLastError();
       nlist_grid_ = rb_grid_;
@@ -387,8 +434,10 @@ int Engine::build() {
   }
 
   // block table, per-slot system ids, parameters, state
-  std::vector<int32_t> hsob(nblocks_), hsid(ntot_);
+  std::vector<int32_t> hsob(nblocks_), hsid(ntot_), hsoc(banded_ ? ch0 : 0);
   for (int s = 0; s < ns; ++s) {
+    if (banded_)
+      for (int k = 0; k < (hsp_[s].n + kThreads - 1) / kThreads; ++k) hsoc[hsp_[s].ch0 + k] = s;
     for (int b = 0; b < hsp_[s].nb; ++b) hsob[hsp_[s].b0 + b] = s;
     for (int k = 0; k < hsp_[s].n; ++k) hsid[hsp_[s].p0 + k] = s;
   }
@@ -396,6 +445,9 @@ int Engine::build() {
                            cudaMemcpyHostToDevice, stream_));
   MDB_CUDA(cudaMemcpyAsync(sid, hsid.data(), sizeof(int32_t) * hsid.size(),
                            cudaMemcpyHostToDevice, stream_));
+  if (banded_)
+    MDB_CUDA(cudaMemcpyAsync(soc, hsoc.data(), sizeof(int32_t) * hsoc.size(),
+                             cudaMemcpyHostToDevice, stream_));
   MDB_CUDA(cudaMemcpyAsync(dsp, hsp_.data(), sizeof(SysParams) * ns, cudaMemcpyHostToDevice,
                            stream_));
   MDB_CUDA(cudaMemcpyAsync(D.st, hst.data(), sizeof(SysState) * ns, cudaMemcpyHostToDevice,
@@ -427,8 +479,6 @@ int Engine::build() {
   schedule_.rebuild_grid = rb_grid_;
   schedule_.items = items_max;
   schedule_.skin = skin_;
-  rc = choose_multi_step();
-  if (rc) return rc;
   return autotune_ ? tune() : MDB_OK;
 }
 
@@ -506,10 +556,10 @@ int Engine::run_resident(int dm, int64_t n) {
   return MDB_OK;
 }
 
-int Engine::launch(void* fn, int grid, int block, const Dev& d) {
+int Engine::launch(void* fn, int grid, int block, const Dev& d, size_t smem) {
   Dev copy = d;
   void* args[] = {&copy};
-  MDB_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(block), args, 0, stream_));
+  MDB_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, stream_));
   launches_ += 1;
   count_launches(1);
   return MDB_OK;
@@ -527,7 +577,7 @@ int Engine::launch_rebuild_eager() {
   if ((rc = launch((void*)k_rb_cellsort, rb_grid_, kThreads, d))) return rc;
   if ((rc = launch((void*)k_rb_permute, rb_grid_, kThreads, d))) return rc;
   if ((rc = launch((void*)k_rb_copyback, rb_grid_, kThreads, d))) return rc;
-  if ((rc = launch((void*)k_rb_nlist, nlist_grid_, kThreads, d))) return rc;
+  if ((rc = launch(list_kernel(), d))) return rc;
   if ((rc = launch((void*)k_rb_finish, 1, kThreads, d))) return rc;
   return MDB_OK;
 }
@@ -553,7 +603,7 @@ int Engine::set_pext(double p) {
 
 int Engine::force(int fm, bool py) {
   MDB_CUDA(cudaSetDevice(device_));
-  return launch(force_fn(fm, py, lanes_), nblocks_, kThreads, dev_);
+  return launch(force_kernel(fm, py), dev_);
 }
 
 int Engine::reduce_K() {
@@ -562,14 +612,14 @@ int Engine::reduce_K() {
 }
 
 int Engine::add_kernel_node(cudaGraph_t g, const cudaGraphNode_t* deps, int ndeps, void* fn,
-                            int grid, int block, const Dev& d, cudaGraphNode_t* out) {
+                            int grid, int block, const Dev& d, cudaGraphNode_t* out, size_t smem) {
   Dev copy = d;
   void* args[] = {&copy};
   cudaKernelNodeParams kp = {};
   kp.func = fn;
   kp.gridDim = dim3(grid);
   kp.blockDim = dim3(block);
-  kp.sharedMemBytes = 0;
+  kp.sharedMemBytes = (unsigned)smem;
   kp.kernelParams = args;
   kp.extra = nullptr;
   MDB_CUDA(cudaGraphAddKernelNode(out, g, deps, (size_t)ndeps, &kp));
@@ -601,7 +651,7 @@ int Engine::add_rebuild_body(cudaGraph_t body, const Dev& d) {
   cudaGraphNode_t join[2];
   int rc = add_kernel_node(body, &prev, 1, (void*)k_rb_copyback, rb_grid_, kThreads, d, &join[0]);
   if (!rc)
-    rc = add_kernel_node(body, &prev, 1, (void*)k_rb_nlist, nlist_grid_, kThreads, d, &join[1]);
+    rc = add_kernel_node(body, &prev, 1, list_kernel(), d, &join[1]);
   cudaGraphNode_t fin;
   if (!rc) rc = add_kernel_node(body, join, 2, (void*)k_rb_finish, 1, kThreads, d, &fin);
   return rc;
@@ -651,11 +701,10 @@ int Engine::get_graph(int kind, int dm, int fm, bool py, int chunk, cudaGraphExe
       rc = add_kernel_node(g, prev ? &prev : nullptr, prev ? 1 : 0, drift_fn(dm, lanes_), nblocks_,
                            kThreads, dd, &nd);
       if (!rc) rc = add_cond_rebuild(g, nd, h, &nc);
-      if (!rc) rc = add_kernel_node(g, &nc, 1, force_fn(fm, py, lanes_), nblocks_, kThreads, dev_, &nf);
+      if (!rc) rc = add_kernel_node(g, &nc, 1, force_kernel(fm, py), dev_, &nf);
       prev = nf;
     } else {
-      rc = add_kernel_node(g, prev ? &prev : nullptr, prev ? 1 : 0, force_fn(FM_FIRE, true, lanes_),
-                           nblocks_, kThreads, dev_, &nf);
+      rc = add_kernel_node(g, prev ? &prev : nullptr, prev ? 1 : 0, force_kernel(FM_FIRE, true), dev_, &nf);
       if (!rc) rc = add_kernel_node(g, &nf, 1, drift_fn(DM_FIRE, lanes_), nblocks_, kThreads, dd, &nd);
       if (!rc) rc = add_cond_rebuild(g, nd, h, &nc);
       prev = nc;
@@ -703,7 +752,7 @@ int Engine::run_md(int dm, int fm, bool py, int64_t nsteps) {
     int rc;
     if ((rc = launch(drift_fn(dm, lanes_), nblocks_, kThreads, dev_))) return rc;
     if ((rc = launch_rebuild_eager())) return rc;
-    if ((rc = launch(force_fn(fm, py, lanes_), nblocks_, kThreads, dev_))) return rc;
+    if ((rc = launch(force_kernel(fm, py), dev_))) return rc;
   }
   return MDB_OK;
 }
@@ -721,7 +770,7 @@ int Engine::run_md_timed(int dm, int fm, bool py, int64_t nsteps, double* ms) {
     cudaEventRecord(ev[1], stream_);
     if (!rc) rc = launch_rebuild_eager();
     cudaEventRecord(ev[2], stream_);
-    if (!rc) rc = launch(force_fn(fm, py, lanes_), nblocks_, kThreads, dev_);
+    if (!rc) rc = launch(force_kernel(fm, py), dev_);
     cudaEventRecord(ev[3], stream_);
     cudaError_t e = cudaEventSynchronize(ev[3]);
     if (e != cudaSuccess) {
@@ -764,7 +813,7 @@ int Engine::run_fire(int64_t iters) {
   }
   for (; left > 0; --left) {
     int rc;
-    if ((rc = launch(force_fn(FM_FIRE, true, lanes_), nblocks_, kThreads, dev_))) return rc;
+    if ((rc = launch(force_kernel(FM_FIRE, true), dev_))) return rc;
     if ((rc = launch(drift_fn(DM_FIRE, lanes_), nblocks_, kThreads, dev_))) return rc;
     if ((rc = launch_rebuild_eager())) return rc;
   }
@@ -991,11 +1040,11 @@ int Engine::time_force(int fm, int reps, double* ms) {
   cudaEvent_t a, b;
   MDB_CUDA(cudaEventCreate(&a));
   MDB_CUDA(cudaEventCreate(&b));
-  int rc = launch(force_fn(fm, true, lanes_), nblocks_, kThreads, dev_);  // warm
+  int rc = launch(force_kernel(fm, true), dev_);  // warm
   double best = 1e30;
   for (int r = 0; !rc && r < reps; ++r) {
     cudaEventRecord(a, stream_);
-    rc = launch(force_fn(fm, true, lanes_), nblocks_, kThreads, dev_);
+    rc = launch(force_kernel(fm, true), dev_);
     cudaEventRecord(b, stream_);
     cudaEventSynchronize(b);
     float t = 0.f;

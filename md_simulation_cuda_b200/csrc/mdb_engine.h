@@ -105,10 +105,23 @@ class Engine {
 
  private:
   int ensure_device();
-  int launch(void* fn, int grid, int block, const Dev& d);
+  // A kernel, its launch shape and dynamic shared memory.
+  struct Kernel {
+    void* fn;
+    int grid, block;
+    size_t smem;
+  };
+  Kernel force_kernel(int fm, bool py) const;
+  Kernel list_kernel() const;
+  int launch(void* fn, int grid, int block, const Dev& d, size_t smem = 0);
+  int launch(const Kernel& k, const Dev& d) { return launch(k.fn, k.grid, k.block, d, k.smem); }
   int launch_rebuild_eager();
   int add_kernel_node(cudaGraph_t g, const cudaGraphNode_t* deps, int ndeps, void* fn, int grid,
-                      int block, const Dev& d, cudaGraphNode_t* out);
+                      int block, const Dev& d, cudaGraphNode_t* out, size_t smem = 0);
+  int add_kernel_node(cudaGraph_t g, const cudaGraphNode_t* deps, int ndeps, const Kernel& k,
+                      const Dev& d, cudaGraphNode_t* out) {
+    return add_kernel_node(g, deps, ndeps, k.fn, k.grid, k.block, d, out, k.smem);
+  }
   int add_rebuild_body(cudaGraph_t body, const Dev& d);
   int add_cond_rebuild(cudaGraph_t g, cudaGraphNode_t dep, cudaGraphConditionalHandle h,
                        cudaGraphNode_t* out);
@@ -145,11 +158,12 @@ class Engine {
   int nblocks_ = 0;
   int rb_grid_ = 0;
   int scan_grid_ = 0;
-  int nlist_grid_ = 0;  // k_rb_nlist: one wave of resident blocks
+  int nlist_grid_ = 0;  // list build: one wave of resident blocks
   int fire_prec_ = MDB_FIRE_AUTO;
   int autotune_ = 0;
   int step_kernel_ = MDB_STEPS_AUTO;
   bool multi_step_ = false;
+  bool banded_ = false;  // force phase and list build over staged bands (mdb_band.cuh)
   bool lanes_ = false;  // some system has several lanes per slot (SysParams::lanes)
   int lanes_opt_ = MDB_LANES_ONE;  // mdb_options_t.lanes (AUTO counts as ONE here)
   int multi_cap_ = 0;  // blocks of the resident steps kernel the device holds at once
@@ -172,9 +186,8 @@ class Engine {
   long long last_rebuilds_ = 0;
 };
 
-// Kernel of a force phase (FM_*; py: periodic y) and of a drift phase (DM_*);
-// ln: the launch holds systems with several lanes per slot.
-void* force_fn(int fm, bool py, bool ln);
+// Kernel of a drift phase (DM_*); ln: the launch holds systems with several
+// lanes per slot.
 void* drift_fn(int dm, bool ln);
 
 int reference_initial_frame(const mdb_config_t& cfg, std::vector<mdb_particle_t>& out);

@@ -68,6 +68,7 @@ struct SysParams {
   int32_t ccap_x, ccap_y;
   int32_t kind;
   int32_t lanes;  // lanes per slot in the force phase (1, or kLanes for small MD systems)
+  int32_t ch0;    // first chunk (kThreads consecutive slots) of the system
   float frl2[3];  // neighbour-list radius^2 per pair class: (rc_ij + skin)^2
   double sig[3], eps[3], Vc[3];  // AA, BB, AB
   double massA, massB, cutoff, rc_max, r_cell, skin;
@@ -157,6 +158,17 @@ struct NphProto {
   int32_t pad;
 };
 
+// The slot ranges a chunk's particles can meet, as staged in shared memory
+// (mdb_band.cuh): range r holds the slots [start, start + len) at places off,
+// off + 1, ... of the band.
+constexpr int kBandRanges = 8;
+constexpr int kBandCap = 1408;  // positions of a staged band: two bands and four
+                                // blocks an SM leave L1 some 50 KB
+struct Band {
+  int32_t start[kBandRanges], len[kBandRanges], off[kBandRanges];
+  int32_t total;  // 0: no band
+};
+
 // Kernel argument block (passed by value).
 struct Dev {
   const int32_t* sys_of_block;
@@ -180,6 +192,10 @@ struct Dev {
   int32_t* nlist;     // neighbour list, offset j - i of entry k of slot i at
   int16_t* nlist16;   //   nlist[k * ntot + i] (int32) or nlist16[...] (int16)
   int32_t* ncount;    // list length per slot (| kListInterior), -1: use the cell stencil
+  uint2* lists;       // banded engines: groups of four 16-bit band places, see k_rb_band
+  Band* bands;        // per chunk
+  const int32_t* sys_of_chunk;
+  int32_t nchunks;
   int32_t max_nbr;
   int32_t nl16;       // 1: 16-bit offsets (every stencil offset fits in int16)
   int32_t* ccount;
