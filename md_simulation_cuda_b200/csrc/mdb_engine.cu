@@ -65,10 +65,14 @@ Engine::Kernel Engine::force_kernel(int fm, bool py) const {
 }
 
 Engine::Kernel Engine::list_kernel() const {
-  if (banded_) return {(void*)k_rb_band, nlist_grid_, kThreads, sizeof(float4) * kBandCap};
+  if (banded_) return {(void*)k_rb_band, nlist_grid_, kThreads, sizeof(float4) * (kBandCap + kBandRoom)};
   return {(void*)k_rb_nlist, nlist_grid_, kThreads, 0};
 }
 
+namespace {
+
+// Kernel of a drift phase (DM_*); ln: the launch holds systems with several
+// lanes per slot.
 void* drift_fn(int dm, bool ln) {
   switch (dm) {
     case DM_NVE: return ln ? (void*)k_drift<DM_NVE, true> : (void*)k_drift<DM_NVE, false>;
@@ -77,6 +81,12 @@ void* drift_fn(int dm, bool ln) {
     case DM_PISTON: return ln ? (void*)k_drift<DM_PISTON, true> : (void*)k_drift<DM_PISTON, false>;
     default: return (void*)k_drift<DM_FIRE, false>;
   }
+}
+
+}  // namespace
+
+Engine::Kernel Engine::drift_kernel(int dm) const {
+  return {drift_fn(dm, lanes_), nblocks_, kThreads, 0};
 }
 
 void* steps_fn(int dm, bool ln) {
@@ -195,7 +205,7 @@ int Engine::build() {
     skin_ = all_fire ? kSkinFire : kSkinMD;
   }
   int64_t p0 = 0, c0 = 0;
-  int b0 = 0, ch0 = 0;
+  int b0 = 0, ch0 = 0, t0 = 0;
   int64_t maxn = 0;
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device_);
@@ -230,6 +240,7 @@ int Engine::build() {
     P.nb = (n + spb * P.items - 1) / (spb * P.items);
     P.b0 = b0;
     P.ch0 = ch0;
+    P.t0 = t0;
     P.kind = sp.kind;
     P.sig[0] = c.SIGMA_AA;
     P.sig[1] = c.SIGMA_BB;
@@ -312,6 +323,7 @@ int Engine::build() {
     b0 += P.nb;
     ch0 += (n + kThreads - 1) / kThreads;
     c0 += (int64_t)P.ccap_x * P.ccap_y;
+    t0 += (int)(((int64_t)P.ccap_x * P.ccap_y + kScanTile - 1) / kScanTile);
   }
   ntot_ = p0;
   nblocks_ = b0;
@@ -333,32 +345,24 @@ int Engine::build() {
   Dev& D = dev_;
   memset(&D, 0, sizeof(D));
   int32_t* sob;
-  int32_t* sid;
   SysParams* dsp;
   MDB_ALLOC(sob, nblocks_);
-  MDB_ALLOC(sid, ntot_);
   MDB_ALLOC(dsp, ns);
   D.sys_of_block = sob;
-  D.sysid = sid;
   D.sp = dsp;
   MDB_ALLOC(D.st, ns);
   MDB_ALLOC(D.bg, 1);
-  MDB_ALLOC(D.pos, ntot_);
-  MDB_ALLOC(D.vel, ntot_);
-  MDB_ALLOC(D.acc, ntot_);
-  MDB_ALLOC(D.type, ntot_);
-  MDB_ALLOC(D.theta, ntot_);
-  MDB_ALLOC(D.orig, ntot_);
-  MDB_ALLOC(D.pos2, ntot_);
-  MDB_ALLOC(D.vel2, ntot_);
-  MDB_ALLOC(D.acc2, ntot_);
-  MDB_ALLOC(D.type2, ntot_);
-  MDB_ALLOC(D.theta2, ntot_);
-  MDB_ALLOC(D.orig2, ntot_);
+  MDB_ALLOC(D.pos, 2 * ntot_);
+  MDB_ALLOC(D.vel, 2 * ntot_);
+  MDB_ALLOC(D.acc, 2 * ntot_);
+  MDB_ALLOC(D.type, 2 * ntot_);
+  MDB_ALLOC(D.theta, 2 * ntot_);
+  MDB_ALLOC(D.orig, 2 * ntot_);
   MDB_ALLOC(D.pff, ntot_);
   MDB_ALLOC(D.sb, ntot_);
   MDB_ALLOC(D.cell_of, ntot_);
   MDB_ALLOC(D.key, ntot_);
+  MDB_ALLOC(D.rank, ntot_);
   MDB_ALLOC(D.perm, ntot_);
   D.max_nbr = max_nbr_;
   MDB_ALLOC(D.ncount, ntot_);
@@ -379,11 +383,15 @@ int Engine::build() {
   // Systems that do not run in the resident steps kernel take the staged bands
   // (one lane per slot).
   banded_ = !multi_step_ && !lanes_;
-  int32_t* soc = nullptr;
+  int32_t *soc = nullptr, *sot = nullptr;
+  D.nchunks = ch0;
+  D.ntiles = t0;
+  MDB_ALLOC(soc, ch0);
+  MDB_ALLOC(sot, t0);
+  MDB_ALLOC(D.tcount, t0);
+  D.sys_of_chunk = soc;
+  D.sys_of_tile = sot;
   if (banded_) {
-    D.nchunks = ch0;
-    MDB_ALLOC(soc, ch0);
-    D.sys_of_chunk = soc;
     MDB_ALLOC(D.bands, ch0);
     if (max_nbr_ > 0) MDB_ALLOC(D.lists, (int64_t)((max_nbr_ + 3) / 4) * ntot_);
   } else if (max_nbr_ > 0) {
@@ -393,10 +401,7 @@ int Engine::build() {
       MDB_ALLOC(D.nlist, (int64_t)max_nbr_ * ntot_);
   }
   MDB_ALLOC(D.ccount, ncells_);
-  MDB_ALLOC(D.ccursor, ncells_);
   MDB_ALLOC(D.cstart, ncells_ + 1);
-  const int64_t ntiles = (ncells_ + kScanTile - 1) / kScanTile;
-  MDB_ALLOC(D.scan_part, ntiles + 1);
   MDB_ALLOC(D.part, (int64_t)nblocks_ * kNP);
   MDB_ALLOC(D.partm, (int64_t)nblocks_ * 4);
   aos_cap_ = maxn;
@@ -408,12 +413,8 @@ int Engine::build() {
   }
 #undef MDB_ALLOC
   D.use_cond = 0;
-  const int64_t work = std::max(ntot_, ncells_);
-  rb_grid_ = (int)std::min<int64_t>((work + kThreads - 1) / kThreads, (int64_t)nsm * 8);
-  rb_grid_ = std::max(rb_grid_, 1);
-  scan_grid_ = (int)std::min<int64_t>(ntiles, (int64_t)nsm * 4);
-  scan_grid_ = std::max(scan_grid_, 1);
-  D.rb_grid = rb_grid_;
+  rb_grid_ = std::max(1, std::min(ch0, nsm * 8));
+  scan_grid_ = std::max(1, std::min(t0, nsm * 4));
   D.pf_rows = kListPrefetchRows;
   // The list build is instruction-bound with per-slot costs that vary (list
   // lengths, minimum-image slots): one wave of resident blocks, grid-stride,
@@ -427,27 +428,26 @@ int Engine::build() {
       (void)cudaGetLastError();
       nlist_grid_ = rb_grid_;
     } else {
-      nlist_grid_ = (int)std::min<int64_t>((ntot_ + kThreads - 1) / kThreads,
-                                           (int64_t)nsm * per_sm);
+      nlist_grid_ = std::min(ch0, nsm * per_sm);
       nlist_grid_ = std::max(nlist_grid_, 1);
     }
   }
 
   // block table, per-slot system ids, parameters, state
-  std::vector<int32_t> hsob(nblocks_), hsid(ntot_), hsoc(banded_ ? ch0 : 0);
+  std::vector<int32_t> hsob(nblocks_), hsoc(ch0), hsot(t0);
   for (int s = 0; s < ns; ++s) {
-    if (banded_)
-      for (int k = 0; k < (hsp_[s].n + kThreads - 1) / kThreads; ++k) hsoc[hsp_[s].ch0 + k] = s;
+    const int chunks = (s + 1 < ns ? hsp_[s + 1].ch0 : ch0) - hsp_[s].ch0;
+    const int tiles = (s + 1 < ns ? hsp_[s + 1].t0 : t0) - hsp_[s].t0;
+    for (int k = 0; k < chunks; ++k) hsoc[hsp_[s].ch0 + k] = s;
+    for (int k = 0; k < tiles; ++k) hsot[hsp_[s].t0 + k] = s;
     for (int b = 0; b < hsp_[s].nb; ++b) hsob[hsp_[s].b0 + b] = s;
-    for (int k = 0; k < hsp_[s].n; ++k) hsid[hsp_[s].p0 + k] = s;
   }
   MDB_CUDA(cudaMemcpyAsync(sob, hsob.data(), sizeof(int32_t) * hsob.size(),
                            cudaMemcpyHostToDevice, stream_));
-  MDB_CUDA(cudaMemcpyAsync(sid, hsid.data(), sizeof(int32_t) * hsid.size(),
+  MDB_CUDA(cudaMemcpyAsync(soc, hsoc.data(), sizeof(int32_t) * hsoc.size(),
                            cudaMemcpyHostToDevice, stream_));
-  if (banded_)
-    MDB_CUDA(cudaMemcpyAsync(soc, hsoc.data(), sizeof(int32_t) * hsoc.size(),
-                             cudaMemcpyHostToDevice, stream_));
+  MDB_CUDA(cudaMemcpyAsync(sot, hsot.data(), sizeof(int32_t) * hsot.size(),
+                           cudaMemcpyHostToDevice, stream_));
   MDB_CUDA(cudaMemcpyAsync(dsp, hsp_.data(), sizeof(SysParams) * ns, cudaMemcpyHostToDevice,
                            stream_));
   MDB_CUDA(cudaMemcpyAsync(D.st, hst.data(), sizeof(SysState) * ns, cudaMemcpyHostToDevice,
@@ -457,6 +457,8 @@ int Engine::build() {
   MDB_CUDA(cudaMemcpyAsync(D.bg, &bg, sizeof(bg), cudaMemcpyHostToDevice, stream_));
   MDB_CUDA(cudaMemsetAsync(D.part, 0, sizeof(double) * (size_t)nblocks_ * kNP, stream_));
   MDB_CUDA(cudaMemsetAsync(D.partm, 0, sizeof(double) * (size_t)nblocks_ * 4, stream_));
+  MDB_CUDA(cudaMemsetAsync(D.ccount, 0, sizeof(int32_t) * (size_t)ncells_, stream_));
+  MDB_CUDA(cudaMemsetAsync(D.tcount, 0, sizeof(int32_t) * (size_t)t0, stream_));
   MDB_CUDA(cudaMemsetAsync(D.cell_of, 0, sizeof(int32_t) * (size_t)ntot_, stream_));
   MDB_CUDA(wait_host());
   built_ = true;
@@ -526,7 +528,7 @@ int Engine::choose_multi_step() {
     const size_t pos = sizeof(float4) * (size_t)ntot_;
     const size_t part = sizeof(double) * 2 * kNP * (size_t)nblocks_;
     const size_t mx = sizeof(unsigned long long) * 16;
-    const size_t cnt = sizeof(int32_t) * (size_t)(ncells_ + nblocks_ + 2);
+    const size_t cnt = sizeof(int32_t) * (size_t)(nblocks_ + 2);
     char* base = nullptr;
     int rc = alloc((void**)&base, pos + part + mx + cnt);
     if (rc) return rc;
@@ -534,8 +536,7 @@ int Engine::choose_multi_step() {
     steps_.part = (double*)(base + pos);
     steps_.max = (unsigned long long*)(base + pos + part);
     steps_.seq = (uint32_t*)(base + pos + part + mx);
-    steps_.count = (int32_t*)(steps_.seq + 2);
-    steps_.tile = steps_.count + ncells_;
+    steps_.tile = (int32_t*)(steps_.seq + 2);
     multi_step_ = true;
   }
   schedule_.multi_step = multi_step_ ? 1 : 0;
@@ -568,17 +569,11 @@ int Engine::launch(void* fn, int grid, int block, const Dev& d, size_t smem) {
 int Engine::launch_rebuild_eager() {
   const Dev& d = dev_;
   int rc;
-  if ((rc = launch((void*)k_rb_zero, rb_grid_, kThreads, d))) return rc;
   if ((rc = launch((void*)k_rb_bin, rb_grid_, kThreads, d))) return rc;
-  if ((rc = launch((void*)k_scan_tiles, scan_grid_, kScanBlock, d))) return rc;
-  if ((rc = launch((void*)k_scan_parts, 1, 1024, d))) return rc;
-  if ((rc = launch((void*)k_scan_add, rb_grid_, kThreads, d))) return rc;
+  if ((rc = launch((void*)k_rb_scan, scan_grid_, kScanBlock, d))) return rc;
   if ((rc = launch((void*)k_rb_scatter, rb_grid_, kThreads, d))) return rc;
-  if ((rc = launch((void*)k_rb_cellsort, rb_grid_, kThreads, d))) return rc;
   if ((rc = launch((void*)k_rb_permute, rb_grid_, kThreads, d))) return rc;
-  if ((rc = launch((void*)k_rb_copyback, rb_grid_, kThreads, d))) return rc;
   if ((rc = launch(list_kernel(), d))) return rc;
-  if ((rc = launch((void*)k_rb_finish, 1, kThreads, d))) return rc;
   return MDB_OK;
 }
 
@@ -627,34 +622,19 @@ int Engine::add_kernel_node(cudaGraph_t g, const cudaGraphNode_t* deps, int ndep
 }
 
 int Engine::add_rebuild_body(cudaGraph_t body, const Dev& d) {
-  struct K {
-    void* fn;
-    int grid, block;
-  } ks[] = {
-      {(void*)k_rb_zero, rb_grid_, kThreads},     {(void*)k_rb_bin, rb_grid_, kThreads},
-      {(void*)k_scan_tiles, scan_grid_, kScanBlock}, {(void*)k_scan_parts, 1, 1024},
-      {(void*)k_scan_add, rb_grid_, kThreads},    {(void*)k_rb_scatter, rb_grid_, kThreads},
-      {(void*)k_rb_cellsort, rb_grid_, kThreads}, {(void*)k_rb_permute, rb_grid_, kThreads},
-  };
+  const Kernel ks[] = {{(void*)k_rb_bin, rb_grid_, kThreads, 0},
+                       {(void*)k_rb_scan, scan_grid_, kScanBlock, 0},
+                       {(void*)k_rb_scatter, rb_grid_, kThreads, 0},
+                       {(void*)k_rb_permute, rb_grid_, kThreads, 0},
+                       list_kernel()};
   cudaGraphNode_t prev = nullptr;
-  for (const K& k : ks) {
+  for (const Kernel& k : ks) {
     cudaGraphNode_t node;
-    int rc = add_kernel_node(body, prev ? &prev : nullptr, prev ? 1 : 0, k.fn, k.grid, k.block, d,
-                             &node);
+    const int rc = add_kernel_node(body, prev ? &prev : nullptr, prev ? 1 : 0, k, d, &node);
     if (rc) return rc;
     prev = node;
   }
-  // After the permutation, the copy of the sorted FP64 state back into the
-  // primary arrays (memory-bound) and the list build (instruction-bound,
-  // reads only the float-float positions and cells) touch disjoint arrays:
-  // two branches that overlap, joined before the finish kernel.
-  cudaGraphNode_t join[2];
-  int rc = add_kernel_node(body, &prev, 1, (void*)k_rb_copyback, rb_grid_, kThreads, d, &join[0]);
-  if (!rc)
-    rc = add_kernel_node(body, &prev, 1, list_kernel(), d, &join[1]);
-  cudaGraphNode_t fin;
-  if (!rc) rc = add_kernel_node(body, join, 2, (void*)k_rb_finish, 1, kThreads, d, &fin);
-  return rc;
+  return MDB_OK;
 }
 
 int Engine::add_cond_rebuild(cudaGraph_t g, cudaGraphNode_t dep, cudaGraphConditionalHandle h,
@@ -698,14 +678,13 @@ int Engine::get_graph(int kind, int dm, int fm, bool py, int chunk, cudaGraphExe
     dd.use_cond = 1;
     cudaGraphNode_t nd, nc, nf;
     if (kind == 0) {
-      rc = add_kernel_node(g, prev ? &prev : nullptr, prev ? 1 : 0, drift_fn(dm, lanes_), nblocks_,
-                           kThreads, dd, &nd);
+      rc = add_kernel_node(g, prev ? &prev : nullptr, prev ? 1 : 0, drift_kernel(dm), dd, &nd);
       if (!rc) rc = add_cond_rebuild(g, nd, h, &nc);
       if (!rc) rc = add_kernel_node(g, &nc, 1, force_kernel(fm, py), dev_, &nf);
       prev = nf;
     } else {
       rc = add_kernel_node(g, prev ? &prev : nullptr, prev ? 1 : 0, force_kernel(FM_FIRE, true), dev_, &nf);
-      if (!rc) rc = add_kernel_node(g, &nf, 1, drift_fn(DM_FIRE, lanes_), nblocks_, kThreads, dd, &nd);
+      if (!rc) rc = add_kernel_node(g, &nf, 1, drift_kernel(DM_FIRE), dd, &nd);
       if (!rc) rc = add_cond_rebuild(g, nd, h, &nc);
       prev = nc;
     }
@@ -750,7 +729,7 @@ int Engine::run_md(int dm, int fm, bool py, int64_t nsteps) {
   }
   for (; left > 0; --left) {
     int rc;
-    if ((rc = launch(drift_fn(dm, lanes_), nblocks_, kThreads, dev_))) return rc;
+    if ((rc = launch(drift_kernel(dm), dev_))) return rc;
     if ((rc = launch_rebuild_eager())) return rc;
     if ((rc = launch(force_kernel(fm, py), dev_))) return rc;
   }
@@ -766,7 +745,7 @@ int Engine::run_md_timed(int dm, int fm, bool py, int64_t nsteps, double* ms) {
   int rc = MDB_OK;
   for (int64_t s = 0; s < nsteps && rc == MDB_OK; ++s) {
     cudaEventRecord(ev[0], stream_);
-    rc = launch(drift_fn(dm, lanes_), nblocks_, kThreads, dev_);
+    rc = launch(drift_kernel(dm), dev_);
     cudaEventRecord(ev[1], stream_);
     if (!rc) rc = launch_rebuild_eager();
     cudaEventRecord(ev[2], stream_);
@@ -814,7 +793,7 @@ int Engine::run_fire(int64_t iters) {
   for (; left > 0; --left) {
     int rc;
     if ((rc = launch(force_kernel(FM_FIRE, true), dev_))) return rc;
-    if ((rc = launch(drift_fn(DM_FIRE, lanes_), nblocks_, kThreads, dev_))) return rc;
+    if ((rc = launch(drift_kernel(DM_FIRE), dev_))) return rc;
     if ((rc = launch_rebuild_eager())) return rc;
   }
   return MDB_OK;
@@ -847,7 +826,7 @@ int Engine::get_frame(int s, mdb_particle_t* out) {
   MDB_CUDA(cudaSetDevice(device_));
   const SysParams& P = hsp_[s];
   const int g = (int)std::min<int64_t>((P.n + kThreads - 1) / kThreads, 4096);
-  k_export<<<g, kThreads, 0, stream_>>>(dev_, (DevParticle*)d_aos_, P.p0, P.n);
+  k_export<<<g, kThreads, 0, stream_>>>(dev_, (DevParticle*)d_aos_, P.p0, P.n, s);
   MDB_CUDA(cudaGetLastError());
   launches_ += 1;
   count_launches(1);
@@ -910,7 +889,7 @@ int Engine::export_async(int s, mdb_particle_t* host) {
   MDB_CUDA(cudaSetDevice(device_));
   const SysParams& P = hsp_[s];
   const int g = (int)std::min<int64_t>((P.n + kThreads - 1) / kThreads, 4096);
-  k_export<<<g, kThreads, 0, stream_>>>(dev_, (DevParticle*)d_aos_, P.p0, P.n);
+  k_export<<<g, kThreads, 0, stream_>>>(dev_, (DevParticle*)d_aos_, P.p0, P.n, s);
   MDB_CUDA(cudaGetLastError());
   launches_ += 1;
   count_launches(1);
@@ -925,7 +904,7 @@ int Engine::set_frame(int s, const mdb_particle_t* in) {
   MDB_CUDA(cudaMemcpyAsync(d_aos_, in, sizeof(mdb_particle_t) * (size_t)P.n,
                            cudaMemcpyHostToDevice, stream_));
   const int g = (int)std::min<int64_t>((P.n + kThreads - 1) / kThreads, 4096);
-  k_import<<<g, kThreads, 0, stream_>>>(dev_, (const DevParticle*)d_aos_, P.p0, P.n);
+  k_import<<<g, kThreads, 0, stream_>>>(dev_, (const DevParticle*)d_aos_, P.p0, P.n, s);
   MDB_CUDA(cudaGetLastError());
   launches_ += 1;
   count_launches(1);
@@ -935,7 +914,9 @@ int Engine::set_frame(int s, const mdb_particle_t* in) {
 int Engine::debug_cells(int s, int32_t* orig, int32_t* cell) {
   MDB_CUDA(cudaSetDevice(device_));
   const SysParams& P = hsp_[s];
-  MDB_CUDA(cudaMemcpyAsync(orig, dev_.orig + P.p0, sizeof(int32_t) * (size_t)P.n,
+  SysState S;
+  if (int rc = get_state(s, &S)) return rc;
+  MDB_CUDA(cudaMemcpyAsync(orig, dev_.orig + (S.buf ? ntot_ : 0) + P.p0, sizeof(int32_t) * (size_t)P.n,
                            cudaMemcpyDeviceToHost, stream_));
   MDB_CUDA(cudaMemcpyAsync(cell, dev_.cell_of + P.p0, sizeof(int32_t) * (size_t)P.n,
                            cudaMemcpyDeviceToHost, stream_));
@@ -1095,7 +1076,6 @@ int Engine::tune() {
     dev_.pf_rows = pf;
     nlist_grid_ = std::max(1, nlg);
     rb_grid_ = std::max(1, rbg);
-    dev_.rb_grid = rb_grid_;
     schedule_.from_cache = 1;
   } else {
     // force phase: list prefetch depth, timed on the workload's force kernel
@@ -1104,10 +1084,17 @@ int Engine::tune() {
     const int fm = all_fire ? FM_FIRE : FM_NH;
     std::vector<SysState> snap;
     if (int rc = get_states(snap)) return rc;
-    MDB_CUDA(cudaMemcpyAsync(dev_.vel2, dev_.vel, sizeof(double2) * (size_t)ntot_,
-                             cudaMemcpyDeviceToDevice, stream_));
-    MDB_CUDA(cudaMemcpyAsync(dev_.acc2, dev_.acc, sizeof(double2) * (size_t)ntot_,
-                             cudaMemcpyDeviceToDevice, stream_));
+    // (both halves of each array: SysState::buf names the one in use)
+    const size_t bytes = sizeof(double2) * 2 * (size_t)ntot_;
+    double2* keep = nullptr;
+    MDB_CUDA(cudaMalloc((void**)&keep, 2 * bytes));
+    struct Free {
+      void* p;
+      ~Free() { cudaFree(p); }
+    } free_keep{keep};
+    MDB_CUDA(cudaMemcpyAsync(keep, dev_.vel, bytes, cudaMemcpyDeviceToDevice, stream_));
+    MDB_CUDA(cudaMemcpyAsync(keep + 2 * ntot_, dev_.acc, bytes, cudaMemcpyDeviceToDevice,
+                             stream_));
     double best = 1e30;
     int best_pf = dev_.pf_rows;
     for (int cand : {28, 16, 8, 0}) {
@@ -1121,17 +1108,15 @@ int Engine::tune() {
       }
     }
     dev_.pf_rows = best_pf;
-    MDB_CUDA(cudaMemcpyAsync(dev_.vel, dev_.vel2, sizeof(double2) * (size_t)ntot_,
-                             cudaMemcpyDeviceToDevice, stream_));
-    MDB_CUDA(cudaMemcpyAsync(dev_.acc, dev_.acc2, sizeof(double2) * (size_t)ntot_,
-                             cudaMemcpyDeviceToDevice, stream_));
+    MDB_CUDA(cudaMemcpyAsync(dev_.vel, keep, bytes, cudaMemcpyDeviceToDevice, stream_));
+    MDB_CUDA(cudaMemcpyAsync(dev_.acc, keep + 2 * ntot_, bytes, cudaMemcpyDeviceToDevice,
+                             stream_));
     MDB_CUDA(cudaMemcpyAsync(dev_.st, snap.data(), sizeof(SysState) * snap.size(),
                              cudaMemcpyHostToDevice, stream_));
     MDB_CUDA(wait_host());
     // rebuild: list-build grid, then the grid of the other rebuild kernels
     const int one_wave = nlist_grid_;
-    const int64_t work = std::max(ntot_, ncells_);
-    const int cap = (int)std::max<int64_t>(1, (work + kThreads - 1) / kThreads);
+    const int cap = std::max(1, dev_.nchunks);
     best = 1e30;
     int best_nlg = one_wave;
     for (int cand : {one_wave, std::min(cap, 2 * one_wave), std::max(1, one_wave / 2)}) {
@@ -1149,7 +1134,6 @@ int Engine::tune() {
     int best_rbg = rb_grid_;
     for (int cand : {rb_grid_, std::min(cap, nsm * 16), std::min(cap, nsm * 4)}) {
       rb_grid_ = std::max(1, cand);
-      dev_.rb_grid = rb_grid_;
       double ms = 0.0;
       const int rc = time_rebuild(2, &ms);
       if (rc) return rc;
@@ -1159,7 +1143,6 @@ int Engine::tune() {
       }
     }
     rb_grid_ = best_rbg;
-    dev_.rb_grid = rb_grid_;
     cache_store(key, dev_.pf_rows, nlist_grid_, rb_grid_);
   }
   MDB_CUDA(wait_host());

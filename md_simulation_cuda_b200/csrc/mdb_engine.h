@@ -112,6 +112,7 @@ class Engine {
     size_t smem;
   };
   Kernel force_kernel(int fm, bool py) const;
+  Kernel drift_kernel(int dm) const;
   Kernel list_kernel() const;
   int launch(void* fn, int grid, int block, const Dev& d, size_t smem = 0);
   int launch(const Kernel& k, const Dev& d) { return launch(k.fn, k.grid, k.block, d, k.smem); }
@@ -185,10 +186,6 @@ class Engine {
   int64_t bytes_ = 0;
   long long last_rebuilds_ = 0;
 };
-
-// Kernel of a drift phase (DM_*); ln: the launch holds systems with several
-// lanes per slot.
-void* drift_fn(int dm, bool ln);
 
 int reference_initial_frame(const mdb_config_t& cfg, std::vector<mdb_particle_t>& out);
 

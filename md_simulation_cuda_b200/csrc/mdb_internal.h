@@ -69,6 +69,7 @@ struct SysParams {
   int32_t kind;
   int32_t lanes;  // lanes per slot in the force phase (1, or kLanes for small MD systems)
   int32_t ch0;    // first chunk (kThreads consecutive slots) of the system
+  int32_t t0;     // first tile (kScanTile consecutive cells) of the system
   float frl2[3];  // neighbour-list radius^2 per pair class: (rc_ij + skin)^2
   double sig[3], eps[3], Vc[3];  // AA, BB, AB
   double massA, massB, cutoff, rc_max, r_cell, skin;
@@ -94,7 +95,7 @@ struct SysState {
   double inv_wx, inv_wy, Lx_b, Ly_b;  // cell grid at the last rebuild
   int32_t ncx, ncy, allpairs, periodic_y;
   int32_t clamped, nph_init, piston_active, piston_init;
-  uint32_t dmax_x, dmax_y, jump;      // float bits (non-negative)
+  int32_t buf;                         // half of the particle arrays in use
   int32_t nl_overflow;                // particles whose list overflowed at the last rebuild
   int32_t need_rebuild;
   int32_t nonfinite;
@@ -128,6 +129,7 @@ struct BatchGlobal {
   int32_t nsys;
   int32_t all_done;
   int32_t bar_err;     // resident steps kernel: an exchange ran out of polls
+  uint32_t rb_count;   // blocks of the list kernel that have arrived
   int32_t forced;      // the pending rebuild was forced (not asked for by a drift)
 };
 
@@ -162,8 +164,9 @@ struct NphProto {
 // (mdb_band.cuh): range r holds the slots [start, start + len) at places off,
 // off + 1, ... of the band.
 constexpr int kBandRanges = 8;
-constexpr int kBandCap = 1408;  // positions of a staged band: two bands and four
-                                // blocks an SM leave L1 some 50 KB
+constexpr int kBandCap = 1408;   // positions of a staged band: two bands and four
+                                 // blocks an SM leave L1 some 50 KB
+constexpr int kBandRoom = 4;     // positions after it that may be read (never used)
 struct Band {
   int32_t start[kBandRanges], len[kBandRanges], off[kBandRanges];
   int32_t total;  // 0: no band
@@ -172,22 +175,20 @@ struct Band {
 // Kernel argument block (passed by value).
 struct Dev {
   const int32_t* sys_of_block;
-  const int32_t* sysid;  // per slot
   const SysParams* sp;
   SysState* st;
   BatchGlobal* bg;
+  // particle arrays: two halves of ntot slots, SysState::buf names the one that
+  // holds a system's current state (a rebuild sorts into the other)
   double2 *pos, *vel, *acc;
   int32_t* type;
   double* theta;
   int32_t* orig;
-  double2 *pos2, *vel2, *acc2;
-  int32_t* type2;
-  double* theta2;
-  int32_t* orig2;
   float4* pff;
   float2* sb;
   int32_t* cell_of;
-  int32_t* key;
+  int32_t* key;       // rebuild: cell of each source slot,
+  int32_t* rank;      //   its arrival rank in the cell
   int32_t* perm;
   int32_t* nlist;     // neighbour list, offset j - i of entry k of slot i at
   int16_t* nlist16;   //   nlist[k * ntot + i] (int32) or nlist16[...] (int16)
@@ -195,13 +196,13 @@ struct Dev {
   uint2* lists;       // banded engines: groups of four 16-bit band places, see k_rb_band
   Band* bands;        // per chunk
   const int32_t* sys_of_chunk;
-  int32_t nchunks;
+  const int32_t* sys_of_tile;
+  int32_t nchunks, ntiles;
   int32_t max_nbr;
   int32_t nl16;       // 1: 16-bit offsets (every stencil offset fits in int16)
-  int32_t* ccount;
-  int32_t* ccursor;
+  int32_t* ccount;    // particles per cell; zero outside a rebuild
+  int32_t* tcount;    // per tile; zero outside a rebuild
   int32_t* cstart;    // ncells + 1
-  int32_t* scan_part; // per scan tile
   double* part;       // nblocks * kNP   block partial sums
   double* partm;      // nblocks * 4     block partial maxima
   int32_t nsys;
@@ -210,14 +211,12 @@ struct Dev {
   int64_t ncells;
   cudaGraphConditionalHandle cond;
   int32_t use_cond;
-  int32_t rb_grid;    // grid of the grid-stride rebuild kernels
   int32_t pf_rows;    // force phase: list rows of the next chunk prefetched per warp
 };
 
 // Device memory of the resident steps kernel.
 struct StepsMem {
   float4* pff1;     // second buffer of float-float positions
-  int32_t* count;   // particles per cell; all zero outside a rebuild
   int32_t* tile;    // particles per block's range of cells; all zero outside a rebuild
   double* part;     // [2][kNP][nblocks] block sums of the exchanges
   unsigned long long* max;  // [4][4] maxima of the exchanges

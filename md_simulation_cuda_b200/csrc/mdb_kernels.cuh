@@ -14,6 +14,11 @@
 
 namespace mdb {
 
+// Which half of the particle arrays holds a system's current state.
+__device__ __forceinline__ int64_t half_of(const Dev& D, const SysState* S) {
+  return S->buf ? D.ntot : 0;
+}
+
 // ---------------------------------------------------------------- helpers --
 
 // pbc_wrap_hd (include/md_cuda_common.hpp:20-29): fmod(x, L), then + L when
@@ -343,6 +348,50 @@ __device__ __forceinline__ DriftTail drift_tail_inputs(const Dev& D, const SysPa
   // system nothing else changes the flag until this block sets it
   t.prior = (D.nsys == 1) ? *((volatile int*)&D.bg->any_rebuild) : 0;
   return t;
+}
+
+// ------------------------------------------------------- asynchronous copy --
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+// Waits for the phase of the given parity; false when it ran out of tries
+// (each of which the hardware suspends for a while).
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+  for (unsigned tries = 0; tries < (1u << 22); ++tries) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// Copies n elements of 16 bytes (so that every address and size is a multiple of
+// 16) to shared memory; completion counts on bar.
+template <typename T>
+__device__ __forceinline__ void copy_bulk(T* dst, const T* src, int n, uint64_t* bar) {
+  static_assert(sizeof(T) == 16, "16-byte elements");
+  asm volatile(
+      "cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          smem_addr(dst)),
+      "l"(src), "r"((uint32_t)n * 16u), "r"(smem_addr(bar))
+      : "memory");
 }
 
 // --------------------------------------------------------- pair interaction --
@@ -926,6 +975,7 @@ struct ForceFinish {
       if (!isfinite(ax) || !isfinite(ay) || !isfinite(v.x) || !isfinite(v.y)) bad = 1;
     }
   }
+  // i: the slot's index in the particle arrays (in the current half).
   __device__ __forceinline__ void operator()(const Dev& D, const SysParams& P, double Ly,
                                              double h, double xi2, double fdt, int64_t i,
                                              double fx, double fy, double w, double u, double an,
@@ -953,6 +1003,7 @@ __device__ __noinline__ ForceFinish<FM, PY> force_items_hp(Dev D, const SysParam
   constexpr bool kEnergy = (FM == FM_OBS);
   constexpr bool kVirial = (FM == FM_OBS || FM == FM_NPH);
   const SysParams& P = *Pp;
+  const int64_t half = half_of(D, Sp);
   ForceFinish<FM, PY> fin;
   fin.init();
   for (int it = 0; it < items; ++it) {
@@ -962,7 +1013,7 @@ __device__ __noinline__ ForceFinish<FM, PY> force_items_hp(Dev D, const SysParam
     const float4 qi = __ldg(D.pff + i);
     const int tci = (int)ff_class(qi);
     particle_force_hp<PY, kEnergy, kVirial>(D, D.pff, P, *Sp, i, Lx, Ly, fx, fy, w, u, an);
-    fin(D, P, Ly, h, xi2, fdt, i, fx, fy, w, u, an, tci);
+    fin(D, P, Ly, h, xi2, fdt, i + half, fx, fy, w, u, an, tci);
   }
   return fin;
 }
@@ -1066,12 +1117,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_force(Dev D) {
   const int s = D.sys_of_block[b];
   const SysParams& P = D.sp[s];
   SysState* S = D.st + s;
+  const int64_t half = half_of(D, S);
   if (!LN || P.lanes == 1) {
     // L1 prefetch of this thread's first slot and its first list rows
     const int64_t i0 = P.p0 + (int64_t)(b - P.b0) * kThreads + threadIdx.x;
     if (i0 < P.p0 + P.n) {
       asm volatile("prefetch.global.L1 [%0];" ::"l"(D.pff + i0));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.vel + i0));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.vel + half + i0));
       asm volatile("prefetch.global.L1 [%0];" ::"l"(D.ncount + i0));
       if (D.nl16 && D.max_nbr >= 8) {
 #pragma unroll
@@ -1126,7 +1178,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_force(Dev D) {
         an += __shfl_xor_sync(0xffffffffu, an, o);
       }
     }
-    if (!skip && i < end && lane == 0) fin(D, P, Ly, h, xi2, fdt, i, fx, fy, w, u, an, tci);
+    if (!skip && i < end && lane == 0) fin(D, P, Ly, h, xi2, fdt, i + half, fx, fy, w, u, an, tci);
   } else {
     fin.init();
     const int q_first = b - P.b0;
@@ -1157,7 +1209,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_force(Dev D) {
           }
           if (ncs + threadIdx.x < end) {
             asm volatile("prefetch.global.L1 [%0];" ::"l"(D.ncount + ncs + threadIdx.x));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(D.vel + ncs + threadIdx.x));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(D.vel + half + ncs + threadIdx.x));
             asm volatile("prefetch.global.L1 [%0];" ::"l"(D.pff + ncs + threadIdx.x));
           }
         }
@@ -1167,7 +1219,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_force(Dev D) {
       if (i < end) {
         particle_force<PY, kEnergy, kVirial, kHpCapable, true>(D, D.pff, P, *S, i, Lx, Ly, fx, fy, w, u, an,
                                                          tci);
-        fin(D, P, Ly, h, xi2, fdt, i, fx, fy, w, u, an, tci);
+        fin(D, P, Ly, h, xi2, fdt, i + half, fx, fy, w, u, an, tci);
       }
     }
   }
@@ -1194,6 +1246,22 @@ struct DriftCtx {
   double massA, massB, offx, offy;
   int zero_v, py;
 };
+
+// The cell grid of a rebuild at the system's current box (one thread, where the
+// rebuild is asked for).
+__device__ __forceinline__ void set_cell_grid(const SysParams& P, SysState* S) {
+  const double Lx = S->Lx, Ly = S->Ly;
+  const int ncx = grid_n(Lx, P.r_cell, P.ccap_x);
+  const int ncy = grid_n(Ly, P.r_cell, P.ccap_y);
+  S->ncx = ncx;
+  S->ncy = ncy;
+  S->allpairs = (ncx < 3 || (S->periodic_y && ncy < 3)) ? 1 : 0;
+  S->inv_wx = (double)ncx / Lx;
+  S->inv_wy = (double)ncy / Ly;
+  S->Lx_b = Lx;
+  S->Ly_b = Ly;
+  S->nl_overflow = 0;
+}
 
 // Scalars of one drift that its tail writes back to the system.
 struct DriftScalars {
@@ -1426,14 +1494,14 @@ __device__ __forceinline__ void drift_move(const DriftCtx& c, double2& x, double
 }
 
 template <int DMd>
-__device__ __forceinline__ void drift_particle(const Dev& D, const DriftCtx& c, int64_t i,
-                                               double2 x, double2 v, const double2 a, int t,
+__device__ __forceinline__ void drift_particle(const Dev& D, const DriftCtx& c, int64_t half,
+                                               int64_t i, double2 x, double2 v, const double2 a, int t,
                                                const float2 sb, double& ksum, double& mdx,
                                                double& mdy, double& mjump, int& bad) {
   float fdx = 0.f, fdy = 0.f;
   drift_move<DMd>(c, x, v, a, t, sb, ksum, mdx, mdy, mjump, fdx, fdy, bad);
-  D.pos[i] = x;
-  D.vel[i] = v;
+  D.pos[half + i] = x;
+  D.vel[half + i] = v;
   D.pff[i] = encode_ff(x.x, x.y, t, c.offx, c.offy);
 }
 
@@ -1444,16 +1512,17 @@ __global__ void __launch_bounds__(kThreads, 4) k_drift(Dev D) {
   const int s = D.nsys == 1 ? 0 : D.sys_of_block[b];
   const SysParams& P = D.sp[s];
   SysState* S = D.st + s;
+  const int64_t half = half_of(D, S);
   {
     // L1 prefetch of this thread's first particle: its DRAM latency overlaps
     // the scalar prologue below
     const int spb0 = LN ? kThreads / P.lanes : kThreads;
     const int64_t i0 = P.p0 + (int64_t)(b - P.b0) * spb0 * P.items + threadIdx.x;
     if ((int)threadIdx.x < spb0 && i0 < P.p0 + P.n) {
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.pos + i0));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.vel + i0));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.acc + i0));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.type + i0));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.pos + half + i0));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.vel + half + i0));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.acc + half + i0));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(D.type + half + i0));
       asm volatile("prefetch.global.L1 [%0];" ::"l"(D.sb + i0));
     }
   }
@@ -1478,8 +1547,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_drift(Dev D) {
     for (int it = 0; it < items; ++it) {
       const int64_t i = base + (int64_t)it * spb;
       if (i >= end) break;
-      drift_particle<DMd>(D, dc, i, D.pos[i], D.vel[i], D.acc[i], D.type[i], D.sb[i], red[0],
-                          mx[0], mx[1], mx[2], bad);
+      drift_particle<DMd>(D, dc, half, i, D.pos[half + i], D.vel[half + i], D.acc[half + i],
+                          D.type[half + i], D.sb[i], red[0], mx[0], mx[1], mx[2], bad);
     }
   }
   if (bad) atomicOr(&S->nonfinite, 1);
@@ -1496,6 +1565,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_drift(Dev D) {
     } else {
       need = drift_tail<DMd>(S, dc, ds, tin, rebuild_limits<DMd>(dc.Lx, dc.Ly, tin), tot, tmx);
       if (need) {
+        set_cell_grid(P, S);
         S->need_rebuild = 1;
         atomicOr(&D.bg->any_rebuild, 1);
       }
@@ -1513,6 +1583,7 @@ __global__ void __launch_bounds__(kThreads) k_reduce_K(Dev D) {
   const int s = D.nsys == 1 ? 0 : D.sys_of_block[b];
   const SysParams& P = D.sp[s];
   SysState* S = D.st + s;
+  const int64_t half = half_of(D, S);
   constexpr int kNS = 1, kNM = 0;
   double red[kNP];
 #pragma unroll
@@ -1523,8 +1594,8 @@ __global__ void __launch_bounds__(kThreads) k_reduce_K(Dev D) {
   for (int it = 0; it < P.items && (int)threadIdx.x < spb; ++it) {
     const int64_t i = base + (int64_t)it * spb;
     if (i >= P.p0 + P.n) break;
-    const double2 v = D.vel[i];
-    const double m = type_mass(P, D.type[i]);
+    const double2 v = D.vel[half + i];
+    const double m = type_mass(P, D.type[half + i]);
     red[0] += (0.5 * m) * fma(v.x, v.x, v.y * v.y);
   }
   double tot[kNP];
@@ -1536,92 +1607,139 @@ __global__ void __launch_bounds__(kThreads) k_reduce_K(Dev D) {
 }
 
 // ------------------------------------------------------ cell-list rebuild --
-// All rebuild kernels are grid-stride with a fixed grid and return at once
-// when no system asked for a rebuild (the eager path launches them every step;
-// the graph path puts them behind a conditional node).
+// Five kernels: bin, scan, scatter, permute, list. All return at once when no
+// system asked for a rebuild (the eager path launches them every step; the
+// graph path puts them behind a conditional node). In a batch a few systems
+// rebuild on almost every step, so what a pass costs then is its launch and
+// its look at the systems that do not: blocks take whole chunks (kThreads
+// slots of one system) or tiles (kScanTile cells of one system) and look at
+// the system's flag once.
+//
+// The sort is out of place: a system's particle arrays (pos, vel, acc, type,
+// theta, orig) have two halves of ntot slots, the permutation goes from the one
+// SysState::buf names into the other, and the last block of the list kernel
+// turns buf over. (Copying the sorted state back was 46 of 300 us per rebuild
+// of the 2,000,000-particle FIRE mix.) The cell and tile counters are zero
+// outside a rebuild: the scan clears the cells it has read, the last block the
+// tiles, so no pass zeroes them first.
 
 __device__ __forceinline__ bool rebuild_requested(const Dev& D) {
   return *((volatile int*)&D.bg->any_rebuild) != 0;
-}
-
-// System owning global cell c (cells of system s are [c0_s, c0_s + ccap_s)).
-__device__ __forceinline__ int cell_system(const Dev& D, int64_t c) {
-  int lo = 0, hi = D.nsys - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (D.sp[mid].c0 <= c) lo = mid; else hi = mid - 1;
-  }
-  return lo;
 }
 
 __device__ __forceinline__ bool sys_rebuilds(const Dev& D, int s) {
   return *((volatile int*)&D.st[s].need_rebuild) != 0;
 }
 
-// Zero the cell counters of every system that rebuilds and compute its grid
-// for the current box. Systems that do not rebuild keep their counts, so the
-// global scan reproduces their cell ranges unchanged.
-__global__ void k_rb_zero(Dev D) {
-  if (!rebuild_requested(D)) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (int64_t c = tid; c < D.ncells; c += stride) {
-    if (!sys_rebuilds(D, cell_system(D, c))) continue;
-    D.ccount[c] = 0;
-    D.ccursor[c] = 0;
+// The slots of one thread in the chunks q, q + gridDim, ... (K of them at once):
+// slot (-1: none, or its system does not rebuild) and system. The passes below
+// are chains of dependent loads and little else, so a thread follows K chains
+// side by side (1,048,576 slots: scatter 17 -> 8 us).
+template <int K>
+struct RebuildSlots {
+  int64_t i[K];
+  int s[K];
+  __device__ __forceinline__ RebuildSlots(const Dev& D, int q0) {
+    bool on[K];
+    int q[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      q[k] = q0 + k * (int)gridDim.x;
+      on[k] = q[k] < D.nchunks;
+      s[k] = (on[k] && D.nsys > 1) ? D.sys_of_chunk[q[k]] : 0;
+    }
+    if (D.nsys > 1) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) on[k] = on[k] && sys_rebuilds(D, s[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const SysParams& P = D.sp[s[k]];
+      i[k] = P.p0 + (int64_t)(q[k] - P.ch0) * kThreads + threadIdx.x;
+      if (!on[k] || i[k] >= P.p0 + P.n) i[k] = -1;
+    }
   }
-  for (int64_t s = tid; s < D.nsys; s += stride) {
-    if (!sys_rebuilds(D, (int)s)) continue;
-    const SysParams& P = D.sp[s];
-    SysState* S = D.st + s;
-    const double Lx = S->Lx, Ly = S->Ly;
-    const int ncx = grid_n(Lx, P.r_cell, P.ccap_x);
-    const int ncy = grid_n(Ly, P.r_cell, P.ccap_y);
-    S->ncx = ncx;
-    S->ncy = ncy;
-    S->allpairs = (ncx < 3 || (S->periodic_y && ncy < 3)) ? 1 : 0;
-    S->inv_wx = (double)ncx / Lx;
-    S->inv_wy = (double)ncy / Ly;
-    S->Lx_b = Lx;
-    S->Ly_b = Ly;
-    S->nl_overflow = 0;
+};
+
+// Cell of each slot, its arrival rank in the cell (arbitrary), and the particles
+// per cell and tile.
+__global__ void __launch_bounds__(kThreads) k_rb_bin(Dev D) {
+  if (!rebuild_requested(D)) return;
+  constexpr int K = 4;
+  const int lane = threadIdx.x & 31;
+  for (int q = blockIdx.x; q < D.nchunks; q += K * (int)gridDim.x) {
+    const RebuildSlots<K> R(D, q);
+    double2 p[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (R.i[k] >= 0) p[k] = D.pos[half_of(D, D.st + R.s[k]) + R.i[k]];
+    int cell[K], r[K], first[K];
+    unsigned mates[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const SysState* S = D.st + R.s[k];
+      const SysParams& P = D.sp[R.s[k]];
+      cell[k] = -1;
+      if (R.i[k] >= 0)
+        cell[k] = bin_axis(p[k].y * S->inv_wy, S->ncy) * S->ncx + bin_axis(p[k].x * S->inv_wx, S->ncx);
+      // one add for the slots of a warp in one cell
+      mates[k] = __match_any_sync(0xffffffffu, cell[k]);
+      first[k] = __ffs(mates[k]) - 1;
+      r[k] = 0;
+      if (cell[k] >= 0 && lane == first[k])
+        r[k] = atomicAdd(D.ccount + P.c0 + cell[k], __popc(mates[k]));
+      // one add for a warp inside one tile (nearly all are)
+      const int tile = cell[k] < 0 ? -1 : cell[k] / kScanTile;
+      const int t0 = __shfl_sync(0xffffffffu, tile, 0);
+      const unsigned same = __ballot_sync(0xffffffffu, tile == t0);
+      if (tile >= 0) {
+        if (tile != t0)
+          atomicAdd(D.tcount + P.t0 + tile, 1);
+        else if (lane == 0)
+          atomicAdd(D.tcount + P.t0 + tile, __popc(same));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int rank = __shfl_sync(0xffffffffu, r[k], first[k]) +
+                       __popc(mates[k] & ((1u << lane) - 1u));
+      if (R.i[k] >= 0) {
+        D.key[R.i[k]] = cell[k];
+        D.rank[R.i[k]] = rank;
+      }
+    }
   }
 }
 
-__global__ void k_rb_bin(Dev D) {
-  if (!rebuild_requested(D)) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D.ntot; i += stride) {
-    const int s = D.sysid[i];
-    if (!sys_rebuilds(D, s)) continue;
-    const SysState* S = D.st + s;
-    const double2 p = D.pos[i];
-    const int ncx = S->ncx, ncy = S->ncy;
-    const int cx = bin_axis(p.x * S->inv_wx, ncx);
-    const int cy = bin_axis(p.y * S->inv_wy, ncy);
-    const int key = (int)(D.sp[s].c0 + (int64_t)cy * ncx + cx);
-    D.key[i] = key;
-    atomicAdd(D.ccount + key, 1);
-  }
-}
-
-// Exclusive scan of ccount into cstart: per-tile scan, scan of tile sums,
-// add. cstart[ncells] receives the total.
-__global__ void __launch_bounds__(kScanBlock) k_scan_tiles(Dev D) {
+// First slot of each cell: the system's first slot, the particles of the tiles
+// before and of the cells before in the tile.
+__global__ void __launch_bounds__(kScanBlock) k_rb_scan(Dev D) {
   if (!rebuild_requested(D)) return;
   __shared__ int sh[kScanBlock / 32];
-  const int64_t ntiles = (D.ncells + kScanTile - 1) / kScanTile;
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t base = tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
+  __shared__ int sh_before[kScanBlock / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int t = blockIdx.x; t < D.ntiles; t += gridDim.x) {
+    const int s = D.sys_of_tile[t];
+    if (!sys_rebuilds(D, s)) continue;
+    const SysParams& P = D.sp[s];
+    const SysState* S = D.st + s;
+    const int ncell = S->ncx * S->ncy;
+    const int first = (t - P.t0) * kScanTile;
+    if (first >= ncell) continue;
+    int before = 0;
+    for (int k = P.t0 + (int)threadIdx.x; k < t; k += kScanBlock) before += D.tcount[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (lane == 0) sh_before[w] = before;
+    int* count = D.ccount + P.c0;
+    const int base = first + (int)threadIdx.x * kScanItems;
     int v[kScanItems];
     int sum = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-      v[k] = (base + k < D.ncells) ? D.ccount[base + k] : 0;
+      v[k] = base + k < ncell ? count[base + k] : 0;
       sum += v[k];
     }
-    // block exclusive scan of per-thread sums
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int x = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1630,139 +1748,140 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_tiles(Dev D) {
     }
     if (lane == 31) sh[w] = x;
     __syncthreads();
-    if (w == 0) {
-      int t = lane < kScanBlock / 32 ? sh[lane] : 0;
+    int run = (int)P.p0 + x - sum;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, t, o);
-        if (lane >= o) t += y;
-      }
-      if (lane < kScanBlock / 32) sh[lane] = t;
+    for (int k = 0; k < kScanBlock / 32; ++k) {
+      run += sh_before[k];
+      if (k < w) run += sh[k];
     }
-    __syncthreads();
-    int run = x - sum + (w > 0 ? sh[w - 1] : 0);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-      if (base + k < D.ncells) D.cstart[base + k] = run;
-      run += v[k];
+      if (base + k < ncell) {
+        D.cstart[P.c0 + base + k] = run;
+        count[base + k] = 0;
+        run += v[k];
+        // (one past the last cell: the next system's first slot)
+        if (base + k == ncell - 1) D.cstart[P.c0 + ncell] = run;
+      }
     }
-    if (threadIdx.x == kScanBlock - 1) D.scan_part[tile] = run;
     __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(1024) k_scan_parts(Dev D) {
+__global__ void __launch_bounds__(kThreads) k_rb_scatter(Dev D) {
   if (!rebuild_requested(D)) return;
-  __shared__ int sh[32];
-  __shared__ int carry;
-  const int64_t ntiles = (D.ncells + kScanTile - 1) / kScanTile;
-  if (threadIdx.x == 0) carry = 0;
+  constexpr int K = 4;
+  for (int q = blockIdx.x; q < D.nchunks; q += K * (int)gridDim.x) {
+    const RebuildSlots<K> R(D, q);
+    int key[K], rank[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (R.i[k] >= 0) {
+        key[k] = D.key[R.i[k]];
+        rank[k] = D.rank[R.i[k]];
+      }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (R.i[k] >= 0) rank[k] += D.cstart[D.sp[R.s[k]].c0 + key[k]];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (R.i[k] >= 0) D.perm[rank[k]] = (int)R.i[k];
+  }
+}
+
+// Each particle to its place: after the particles of lower source slots in its
+// cell (the stable sort by cell), with the float-float copy, the cell and the
+// rebuild position. A thread takes an entry of perm, so a warp's reads may
+// scatter (particles that moved far) while its writes stay inside a few cells.
+__global__ void __launch_bounds__(kThreads, 4) k_rb_permute(Dev D) {
+  if (!rebuild_requested(D)) return;
+  constexpr int K = 2;
+  // (inside an MD step the force phase that follows writes the accelerations)
+  const bool forced = *((volatile int*)&D.bg->forced) != 0;
+  for (int q = blockIdx.x; q < D.nchunks; q += K * (int)gridDim.x) {
+    const RebuildSlots<K> R(D, q);
+    int src[K], cell[K], ca[K], ce[K], before[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) src[k] = R.i[k] >= 0 ? D.perm[R.i[k]] : 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) cell[k] = R.i[k] >= 0 ? D.key[src[k]] : 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int32_t* cs = D.cstart + D.sp[R.s[k]].c0 + cell[k];
+      ca[k] = R.i[k] >= 0 ? cs[0] : 0;
+      ce[k] = R.i[k] >= 0 ? cs[1] : 0;
+      before[k] = 0;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      for (int e = ca[k]; e < ce[k]; e += 4) {
+        int other[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) other[u] = D.perm[min(e + u, ce[k] - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) before[k] += (e + u < ce[k] && other[u] < src[k]) ? 1 : 0;
+      }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (R.i[k] < 0) continue;
+      const SysParams& P = D.sp[R.s[k]];
+      const SysState* S = D.st + R.s[k];
+      const int64_t from = half_of(D, S) + src[k];
+      const int64_t at = ca[k] + before[k];
+      const int64_t to = D.ntot - half_of(D, S) + at;
+      const double2 p = D.pos[from];
+      const int t = D.type[from];
+      D.vel[to] = D.vel[from];
+      if (forced || P.kind == K_FIRE) D.acc[to] = D.acc[from];
+      D.theta[to] = D.theta[from];
+      D.orig[to] = D.orig[from];
+      D.pos[to] = p;
+      D.type[to] = t;
+      D.cell_of[at] = cell[k];
+      D.pff[at] = encode_ff(p.x, p.y, t, P.offx, P.offy);
+      const float sx = (float)(p.x * (1.0 / S->Lx));
+      const float sy = S->periodic_y ? (float)(p.y * (1.0 / S->Ly)) : (float)p.y;
+      D.sb[at] = make_float2(sx, sy);
+    }
+  }
+}
+
+// Steps (MD) or iterations (FIRE) the system has run: the clock of its
+// rebuild history.
+__device__ __forceinline__ int64_t rebuild_clock(const SysParams& P, const SysState& S) {
+  return P.kind == K_FIRE ? (int64_t)S.f_step : S.steps;
+}
+
+// End of a rebuild, by the block of the list kernel that arrives last: the
+// sorted halves become current, the tile counters and flags are cleared.
+__device__ __forceinline__ void rebuild_finish(const Dev& D, bool forced) {
+  __shared__ int sh_last;
   __syncthreads();
-  for (int64_t base = 0; base < ntiles; base += 1024) {
-    const int64_t k = base + threadIdx.x;
-    const int v = k < ntiles ? D.scan_part[k] : 0;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) sh[w] = x;
-    __syncthreads();
-    if (w == 0) {
-      int t = sh[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, t, o);
-        if (lane >= o) t += y;
-      }
-      sh[lane] = t;
-    }
-    __syncthreads();
-    const int excl = x - v + (w > 0 ? sh[w - 1] : 0) + carry;
-    __syncthreads();
-    if (k < ntiles) D.scan_part[k] = excl;
-    if (threadIdx.x == 1023) carry = excl + v;
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned prev;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
+                 : "=r"(prev)
+                 : "l"(&D.bg->rb_count)
+                 : "memory");
+    sh_last = prev == gridDim.x - 1 ? 1 : 0;
   }
-  if (threadIdx.x == 0) D.cstart[D.ncells] = carry;
-}
-
-__global__ void k_scan_add(Dev D) {
-  if (!rebuild_requested(D)) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < D.ncells; c += stride)
-    D.cstart[c] += D.scan_part[c / kScanTile];
-}
-
-__global__ void k_rb_scatter(Dev D) {
-  if (!rebuild_requested(D)) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D.ntot; i += stride) {
-    if (!sys_rebuilds(D, D.sysid[i])) continue;
-    const int key = D.key[i];
-    const int slot = D.cstart[key] + atomicAdd(D.ccursor + key, 1);
-    D.perm[slot] = (int)i;
+  __syncthreads();
+  if (!sh_last) return;
+  for (int t = threadIdx.x; t < D.ntiles; t += blockDim.x)
+    if (sys_rebuilds(D, D.sys_of_tile[t])) D.tcount[t] = 0;
+  __syncthreads();
+  for (int s = threadIdx.x; s < D.nsys; s += blockDim.x) {
+    SysState* S = D.st + s;
+    if (!S->need_rebuild) continue;
+    S->need_rebuild = 0;
+    S->buf ^= 1;
+    S->rebuilds += 1;
+    S->rb_last = forced ? kNoRebuildYet : rebuild_clock(D.sp[s], *S);
   }
-}
-
-// Within a cell the scatter order is arbitrary; sorting each cell's slots by
-// source slot makes the permutation the stable sort by cell.
-__global__ void k_rb_cellsort(Dev D) {
-  if (!rebuild_requested(D)) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < D.ncells; c += stride) {
-    if (!sys_rebuilds(D, cell_system(D, c))) continue;
-    const int a = D.cstart[c], e = D.cstart[c + 1];
-    for (int k = a + 1; k < e; ++k) {
-      const int v = D.perm[k];
-      int q = k - 1;
-      while (q >= a && D.perm[q] > v) {
-        D.perm[q + 1] = D.perm[q];
-        --q;
-      }
-      D.perm[q + 1] = v;
-    }
-  }
-}
-
-__global__ void k_rb_permute(Dev D) {
-  if (!rebuild_requested(D)) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < D.ntot; k += stride) {
-    const int s = D.sysid[k];
-    if (!sys_rebuilds(D, s)) continue;
-    const int src = D.perm[k];
-    const SysParams& P = D.sp[s];
-    const SysState* S = D.st + s;
-    const double2 p = D.pos[src];
-    const int t = D.type[src];
-    D.pos2[k] = p;
-    D.vel2[k] = D.vel[src];
-    D.acc2[k] = D.acc[src];
-    D.type2[k] = t;
-    D.theta2[k] = D.theta[src];
-    D.orig2[k] = D.orig[src];
-    D.cell_of[k] = (int)(D.key[src] - P.c0);
-    D.pff[k] = encode_ff(p.x, p.y, t, P.offx, P.offy);
-    const float sx = (float)(p.x * (1.0 / S->Lx));
-    const float sy = S->periodic_y ? (float)(p.y * (1.0 / S->Ly)) : (float)p.y;
-    D.sb[k] = make_float2(sx, sy);
-  }
-}
-
-__global__ void k_rb_copyback(Dev D) {
-  if (!rebuild_requested(D)) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < D.ntot; k += stride) {
-    if (!sys_rebuilds(D, D.sysid[k])) continue;
-    D.pos[k] = D.pos2[k];
-    D.vel[k] = D.vel2[k];
-    D.acc[k] = D.acc2[k];
-    D.type[k] = D.type2[k];
-    D.theta[k] = D.theta2[k];
-    D.orig[k] = D.orig2[k];
+  if (threadIdx.x == 0) {
+    D.bg->rb_count = 0u;
+    D.bg->any_rebuild = 0;
+    D.bg->forced = 0;
   }
 }
 
@@ -1859,21 +1978,16 @@ __device__ __forceinline__ int build_list(const Dev& D, const SysParams& P, cons
   return cnt;
 }
 
-// Steps (MD) or iterations (FIRE) the system has run: the clock of its
-// rebuild history.
-__device__ __forceinline__ int64_t rebuild_clock(const SysParams& P, const SysState& S) {
-  return P.kind == K_FIRE ? (int64_t)S.f_step : S.steps;
-}
-
-__global__ void k_rb_nlist(Dev D) {
+__global__ void __launch_bounds__(kThreads) k_rb_nlist(Dev D) {
   if (!rebuild_requested(D)) return;
   const bool forced = *((volatile int*)&D.bg->forced) != 0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < D.ntot; k += stride) {
-    const int s = D.sysid[k];
+  for (int q = blockIdx.x; q < D.nchunks; q += gridDim.x) {
+    const int s = D.sys_of_chunk[q];
     if (!sys_rebuilds(D, s)) continue;
     const SysParams& P = D.sp[s];
     SysState* S = D.st + s;
+    const int64_t k = P.p0 + (int64_t)(q - P.ch0) * kThreads + threadIdx.x;
+    if (k >= P.p0 + P.n) continue;
     // a system that rebuilds again within kListMinReuse steps scans its cell
     // stencil instead of a list it would hardly reuse
     const bool recent = !forced && rebuild_clock(P, *S) - S->rb_last < kListMinReuse;
@@ -1904,26 +2018,7 @@ __global__ void k_rb_nlist(Dev D) {
     }
     D.ncount[k] = cnt | ((interior && nowrap) ? kListInterior : 0);
   }
-}
-
-__global__ void k_rb_finish(Dev D) {
-  if (!rebuild_requested(D)) return;
-  const bool forced = *((volatile int*)&D.bg->forced) != 0;
-  for (int s = threadIdx.x; s < D.nsys; s += blockDim.x) {
-    SysState* S = D.st + s;
-    if (!S->need_rebuild) continue;
-    S->need_rebuild = 0;
-    S->dmax_x = 0u;
-    S->dmax_y = 0u;
-    S->jump = 0u;
-    S->rebuilds += 1;
-    S->rb_last = forced ? kNoRebuildYet : rebuild_clock(D.sp[s], *S);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    D.bg->any_rebuild = 0;
-    D.bg->forced = 0;
-  }
+  rebuild_finish(D, forced);
 }
 
 // ------------------------------------------------------------ profiles --
@@ -1958,14 +2053,15 @@ __global__ void __launch_bounds__(kThreads) k_profiles(Dev D, int s, int nb,
                                                        unsigned long long* ptens, int* counts) {
   const SysParams& P = D.sp[s];
   const SysState& S = D.st[s];
+  const int64_t half = half_of(D, &S);
   const double Lx = S.Lx, Ly = S.Ly;
   PairCtx c;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < P.n; k += stride) {
     const int64_t i = P.p0 + k;
-    const double2 p = D.pos[i];
-    const double2 v = D.vel[i];
-    const int ti = D.type[i];
+    const double2 p = D.pos[half + i];
+    const double2 v = D.vel[half + i];
+    const int ti = D.type[half + i];
     if (p.x >= 0.0 && p.x <= Lx) {
       int b = (int)(p.x / Lx * nb);
       b = b < 0 ? 0 : (b >= nb ? nb - 1 : b);
@@ -2049,7 +2145,9 @@ struct DevParticle {  // include/md_particle.hpp:31-38 (64 bytes)
   double theta;
 };
 
-__global__ void k_import(Dev D, const DevParticle* __restrict__ in, int64_t p0, int64_t n) {
+__global__ void k_import(Dev D, const DevParticle* __restrict__ in, int64_t p0, int64_t n,
+                         int s) {
+  p0 += half_of(D, D.st + s);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
     const DevParticle q = in[k];
@@ -2067,6 +2165,7 @@ __global__ void k_import(Dev D, const DevParticle* __restrict__ in, int64_t p0, 
 // src/md_energy_minimizer.cu:386-419) and zeroes v and a when asked.
 __global__ void k_fire_prepare(Dev D, int64_t p0, int64_t n, int s) {
   const SysState* S = D.st + s;
+  p0 += half_of(D, S);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
     const int64_t slot = p0 + k;
@@ -2079,7 +2178,8 @@ __global__ void k_fire_prepare(Dev D, int64_t p0, int64_t n, int s) {
   }
 }
 
-__global__ void k_export(Dev D, DevParticle* __restrict__ out, int64_t p0, int64_t n) {
+__global__ void k_export(Dev D, DevParticle* __restrict__ out, int64_t p0, int64_t n, int s) {
+  p0 += half_of(D, D.st + s);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
     const int64_t slot = p0 + k;
@@ -2123,6 +2223,7 @@ __global__ void k_force_rebuild(Dev D, int periodic_y) {
   for (int s = threadIdx.x; s < D.nsys; s += blockDim.x) {
     D.st[s].need_rebuild = 1;
     if (periodic_y >= 0) D.st[s].periodic_y = periodic_y;
+    set_cell_grid(D.sp[s], D.st + s);
   }
   if (threadIdx.x == 0) {
     D.bg->any_rebuild = 1;

@@ -339,7 +339,7 @@ int Engine::proto_graph(cudaGraphExec_t* exec) {
       dd.use_cond = 1;
       cudaGraphNode_t nd, nc, nf;
       rc = add_kernel_node(cg, prev ? &prev : nullptr, prev ? 1 : 0,
-                           drift_fn(nph ? DM_NPH : DM_NH, lanes_), nblocks_, kThreads, dd, &nd);
+                           drift_kernel(nph ? DM_NPH : DM_NH), dd, &nd);
       if (rc == MDB_OK) rc = add_cond_rebuild(cg, nd, hr, &nc);
       if (rc == MDB_OK)
         rc = add_kernel_node(cg, &nc, 1, force_kernel(nph ? FM_NPH : FM_NH, true), dev_, &nf);

@@ -408,6 +408,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
   const bool own = act && lane == 0;
   const bool shared_list = M.list_rows > 0;
   const int64_t rebuilds0 = S.rebuilds;
+  const int64_t half = half_of(D, &S);  // (the sort in here is in place)
   int16_t* col = sh_lists + tid;
 
   // the slot's state, in registers from here on
@@ -416,10 +417,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
   float4 qi = make_float4(0.f, 0.f, 0.f, 0.f);
   int t = 0, nc = 0, rows = 0;
   if (act) {
-    x = D.pos[i];
-    v = D.vel[i];
-    a = D.acc[i];
-    t = D.type[i];
+    x = D.pos[half + i];
+    v = D.vel[half + i];
+    a = D.acc[half + i];
+    t = D.type[half + i];
     sb = D.sb[i];
     qi = D.pff[i];
     nc = D.ncount[i];
@@ -459,8 +460,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
     // One pass is a step: drift, rebuild, force. A FIRE iteration is force,
     // drift, rebuild.
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      if ((half == 0) != FIRE) {
+    for (int phase = 0; phase < 2; ++phase) {
+      if ((phase == 0) != FIRE) {
         // ---- drift
         if (sh.ds.boxbad) {
           __syncthreads();
@@ -513,15 +514,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
         if (sh.need) {
           // ---- rebuild (the passes of k_rb_*, on the slots' own threads)
           if (tid == 0) {
-            const int ncx = grid_n(S.Lx, P.r_cell, P.ccap_x);
-            const int ncy = grid_n(S.Ly, P.r_cell, P.ccap_y);
-            S.ncx = ncx;
-            S.ncy = ncy;
-            S.allpairs = (ncx < 3 || (S.periodic_y && ncy < 3)) ? 1 : 0;
-            S.inv_wx = (double)ncx / S.Lx;
-            S.inv_wy = (double)ncy / S.Ly;
-            S.Lx_b = S.Lx;
-            S.Ly_b = S.Ly;
+            set_cell_grid(P, &S);
             if (blockIdx.x == 0) D.st->nl_overflow = 0;
           }
           __syncthreads();
@@ -532,14 +525,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
           double theta = 0.0;
           if (own) {
             key = bin_axis(x.y * S.inv_wy, S.ncy) * S.ncx + bin_axis(x.x * S.inv_wx, S.ncx);
-            rank = atomicAdd(M.count + key, 1);
+            rank = atomicAdd(D.ccount + P.c0 + key, 1);
             // one add per warp and tile: neighbouring slots share tiles, and
             // single adds queued for 40,000 cycles at 60,000 slots
             const int tile = key / per;
             const unsigned same = __match_any_sync(__activemask(), tile);
             if ((tid & 31) == __ffs(same) - 1) atomicAdd(M.tile + tile, __popc(same));
-            orig = D.orig[i];
-            theta = D.theta[i];
+            orig = D.orig[half + i];
+            theta = D.theta[half + i];
           }
           exchange<0, 0, 0>(M, sh, seq, in, out);
           if (sh.abort) break;
@@ -559,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
             const int c1 = min(ncell, c0 + per);
             for (int cb = c0; cb < c1; cb += kThreads) {
               const int cc = cb + tid;
-              const int cn = cc < c1 ? __ldcg(M.count + cc) : 0;
+              const int cn = cc < c1 ? __ldcg(D.ccount + P.c0 + cc) : 0;
               int xs = cn;
 #pragma unroll
               for (int o = 1; o < 32; o <<= 1) {
@@ -576,7 +569,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
               }
               if (cc < c1) {
                 D.cstart[P.c0 + cc] = (int)P.p0 + base + xs - cn;
-                M.count[cc] = 0;
+                D.ccount[P.c0 + cc] = 0;
               }
               carry += all;
               __syncthreads();
@@ -606,12 +599,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
               for (int e = 0; e < 8; ++e) before += other[e] < (int)i ? 1 : 0;
             }
             const int64_t dst = ca + before;
-            D.pos[dst] = x;
-            D.vel[dst] = v;
-            D.acc[dst] = a;
-            D.type[dst] = t;
-            D.theta[dst] = theta;
-            D.orig[dst] = orig;
+            D.pos[half + dst] = x;
+            D.vel[half + dst] = v;
+            D.acc[half + dst] = a;
+            D.type[half + dst] = t;
+            D.theta[half + dst] = theta;
+            D.orig[half + dst] = orig;
             D.cell_of[dst] = key;
             D.pff[dst] = qi;
             M.pff1[dst] = qi;
@@ -641,10 +634,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
             }
           }
           if (act) {
-            x = __ldcg(D.pos + i);
-            v = __ldcg(D.vel + i);
-            a = __ldcg(D.acc + i);
-            t = __ldcg(D.type + i);
+            x = __ldcg(D.pos + half + i);
+            v = __ldcg(D.vel + half + i);
+            a = __ldcg(D.acc + half + i);
+            t = __ldcg(D.type + half + i);
             sb = __ldcg(D.sb + i);
             qi = __ldcg(cur + i);
             if (lane == 0) D.ncount[i] = nc;
@@ -744,9 +737,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
   }
   if (bad) atomicOr(&D.st->nonfinite, 1);
   if (own) {
-    D.pos[i] = x;
-    D.vel[i] = v;
-    D.acc[i] = a;
+    D.pos[half + i] = x;
+    D.vel[half + i] = v;
+    D.acc[half + i] = a;
     D.pff[i] = qi;
   }
   if (act && shared_list && S.rebuilds != rebuilds0) {
