@@ -268,16 +268,11 @@ __device__ __forceinline__ int build_band_list(const Dev& D, const SysParams& P,
 // slot's own place. One block per chunk in turn; the candidates are read from
 // the staged band. The entries, their order and the count are those of
 // build_list.
-__global__ void __launch_bounds__(kThreads, 4) k_rb_band(Dev D) {
-  if (!rebuild_requested(D)) return;
-  extern __shared__ __align__(128) float4 sh_band[];
-  __shared__ Band band;
-  __shared__ __align__(8) uint64_t full;
-  const bool forced = *((volatile int*)&D.bg->forced) != 0;
-  if (threadIdx.x == 0) mbar_init(&full, 1);
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  __syncthreads();
-  uint32_t parity = 0;
+// (full: an mbarrier for one arrival, parity its current phase. False: a copy
+// never arrived.)
+__device__ __forceinline__ bool rb_band(const Dev& D, float4* sh_band, Band& band, uint64_t& full,
+                                        uint32_t& parity, bool forced) {
+  bool all = true;
   for (int q = blockIdx.x; q < D.nchunks; q += gridDim.x) {
     const int s = D.sys_of_chunk[q];
     if (!sys_rebuilds(D, s)) continue;  // (the whole block)
@@ -317,10 +312,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_rb_band(Dev D) {
     }
     const bool here = mbar_wait(&full, parity);
     parity ^= 1u;
+    all = all && here;
     if (!here) {
       if (act) D.ncount[k] = -1;
-      atomicExch(&D.bg->bar_err, 1);
-      S->err = 6;  // MDB_ERR_CUDA: the copy never arrived
     } else if (act) {
       const int cell = D.cell_of[k];
       const int cx = cell % S->ncx, cy = cell / S->ncx;
@@ -341,23 +335,49 @@ __global__ void __launch_bounds__(kThreads, 4) k_rb_band(Dev D) {
     }
     __syncthreads();  // every thread is done with the band
   }
+  return all;
+}
+
+__global__ void __launch_bounds__(kThreads, 4) k_rb_band(Dev D) {
+  if (!rebuild_requested(D)) return;
+  extern __shared__ __align__(128) float4 sh_band[];
+  __shared__ Band band;
+  __shared__ __align__(8) uint64_t full;
+  const bool forced = *((volatile int*)&D.bg->forced) != 0;
+  if (threadIdx.x == 0) mbar_init(&full, 1);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncthreads();
+  uint32_t parity = 0;
+  if (!rb_band(D, sh_band, band, full, parity, forced)) {
+    atomicExch(&D.bg->bar_err, 1);
+    for (int s = 0; s < D.nsys; ++s) D.st[s].err = 6;  // MDB_ERR_CUDA: a copy never arrived
+  }
   rebuild_finish(D, forced);
 }
 
 // ------------------------------------------------------------- force phase --
 
+// A group of list entries (NC: see ld_idx).
+template <bool NC>
+__device__ __forceinline__ uint2 ld_group(const uint2* p) {
+  if (NC) return __ldg(p);
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+
 // Pair sums over a slot's list in the staged band.
-template <bool PY, bool ENERGY, bool VIRIAL, bool MIC, bool FLOOR>
+template <bool PY, bool ENERGY, bool VIRIAL, bool MIC, bool FLOOR, bool NC>
 __device__ __forceinline__ void band_list(const float4* __restrict__ band,
                                           const uint2* __restrict__ list, int64_t ntot, int groups,
                                           const PairCtx& c, float2& fs, float2& fc, float& ws,
                                           float& wc, double& u, double& an) {
-  uint2 e = groups > 0 ? __ldg(list) : make_uint2(0u, 0u);
+  uint2 e = groups > 0 ? ld_group<NC>(list) : make_uint2(0u, 0u);
   for (int g = 0; g < groups; ++g) {
     const float4 q0 = band[e.x & 0xffffu], q1 = band[e.x >> 16];
     const float4 q2 = band[e.y & 0xffffu], q3 = band[e.y >> 16];
     list += ntot;
-    if (g + 1 < groups) e = __ldg(list);  // the next group's entries
+    if (g + 1 < groups) e = ld_group<NC>(list);  // the next group's entries
     pair_one<PY, ENERGY, VIRIAL, MIC, FLOOR>(q0, c, fs, fc, ws, wc, u, an);
     pair_one<PY, ENERGY, VIRIAL, MIC, FLOOR>(q1, c, fs, fc, ws, wc, u, an);
     pair_one<PY, ENERGY, VIRIAL, MIC, FLOOR>(q2, c, fs, fc, ws, wc, u, an);
@@ -366,13 +386,13 @@ __device__ __forceinline__ void band_list(const float4* __restrict__ band,
 }
 
 // The same with FP64 pair terms.
-template <bool PY, bool ENERGY, bool VIRIAL, bool MIC>
+template <bool PY, bool ENERGY, bool VIRIAL, bool MIC, bool NC>
 __device__ __forceinline__ void band_list_hp(const float4* band, const uint2* __restrict__ list,
                                              int64_t ntot, int groups, const PairCtxD& c,
                                              double& fx, double& fy, double& w, double& u,
                                              double& an) {
   for (int g = 0; g < groups; ++g, list += ntot) {
-    const uint2 e = __ldg(list);
+    const uint2 e = ld_group<NC>(list);
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
       const uint32_t at = ((k < 2 ? e.x : e.y) >> (16 * (k & 1))) & 0xffffu;
@@ -390,7 +410,7 @@ struct BandShared {
 
 // Run r of the stencil of cell (cx, cy), in visiting order: two runs a row, the
 // second across the periodic x edge. Global slots [a, e); false: no such run.
-template <bool PY>
+template <bool PY, bool NC>
 __device__ __forceinline__ bool stencil_run(const int32_t* cst, int ncx, int ncy, int cx, int cy,
                                             int r, int* a, int* e) {
   int y = cy - 1 + (r >> 1);
@@ -404,21 +424,23 @@ __device__ __forceinline__ bool stencil_run(const int32_t* cst, int ncx, int ncy
   const bool mid = cx > 0 && cx < ncx - 1;
   if ((r & 1) != 0) {
     if (mid) return false;
-    *a = __ldg(row + (cx == 0 ? ncx - 1 : 0));
-    *e = __ldg(row + (cx == 0 ? ncx : 1));
+    *a = ld_idx<NC>(row + (cx == 0 ? ncx - 1 : 0));
+    *e = ld_idx<NC>(row + (cx == 0 ? ncx : 1));
     return true;
   }
-  *a = __ldg(row + (mid ? cx - 1 : (cx == 0 ? 0 : ncx - 2)));
-  *e = __ldg(row + (mid ? cx + 2 : (cx == 0 ? 2 : ncx)));
+  *a = ld_idx<NC>(row + (mid ? cx - 1 : (cx == 0 ? 0 : ncx - 2)));
+  *e = ld_idx<NC>(row + (mid ? cx + 2 : (cx == 0 ? 2 : ncx)));
   return true;
 }
 
 // The chunks of one block: pair sums and what follows them, into fin. HP: FP64
-// pair terms (a FIRE system past its switch point, and its observations).
-template <int FM, bool PY, bool HP>
+// pair terms (a FIRE system past its switch point, and its observations). pass
+// counts the passes run on sh's barriers so far: it gives the buffer and the
+// barriers' parities.
+template <int FM, bool PY, bool HP, bool NC>
 __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, const SysState& S,
                                            BandShared& sh, float4* sh_band, int q_first, int items,
-                                           ForceFinish<FM, PY>& fin) {
+                                           uint32_t& pass, ForceFinish<FM, PY>& fin) {
   constexpr bool kEnergy = (FM == FM_OBS);
   constexpr bool kVirial = (FM == FM_OBS || FM == FM_NPH);
   constexpr bool kFloor = (FM == FM_FIRE || FM == FM_OBS || FM == FM_INIT);
@@ -456,28 +478,27 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
     if (lane < kBandRanges && ln > 0)
       copy_bulk(sh_band + buf * kBandCap + of, D.pff + st, ln, sh.full + buf);
   };
-  if (warp == 0 && items > 0) stage(q_first, 0);
+  if (warp == 0 && items > 0) stage(q_first, (int)(pass & 1u));
   const double Lx = S.Lx, Ly = S.Ly;
   const double h = 0.5 * P.dt;
   const double xi2 = (FM == FM_NH) ? S.xi : 0.0;
   const double fdt = (FM == FM_FIRE) ? S.f_dt : 0.0;
 #pragma unroll 1
-  for (int it = 0; it < items; ++it) {
-    const int buf = it & 1;
+  for (int it = 0; it < items; ++it, ++pass) {
+    const int buf = (int)(pass & 1u);
     const int64_t cs = P.p0 + (int64_t)(it * nb + rot) * kThreads;
     if (cs >= end) break;  // (every thread of the block agrees)
     const int64_t i = cs + threadIdx.x;
     const bool act = i < end;
-    const int nc = act ? __ldg(D.ncount + i) : -1;
+    const int nc = act ? ld_idx<NC>(D.ncount + i) : -1;
     rot = next_rot(rot);
     {
       const int q = (it + 1) * nb + rot;
       const int64_t ncs = P.p0 + (int64_t)q * kThreads;
       if (it + 1 < items && ncs < end) {
         if (warp == 0) {
-          // the other buffer: free once every warp has left pass it - 1
-          if (it > 0 && !mbar_wait(sh.empty + (buf ^ 1), (uint32_t)((it - 1) >> 1) & 1u))
-            sh.lost = 1;
+          // the other buffer: free once every warp has left the pass before
+          if (pass > 0 && !mbar_wait(sh.empty + (buf ^ 1), ((pass - 1) >> 1) & 1u)) sh.lost = 1;
           stage(q, buf ^ 1);
         }
         // L1 prefetch of the next chunk's list groups (32 slots of a group are
@@ -494,13 +515,13 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
         }
       }
     }
-    if (!mbar_wait(sh.full + buf, (uint32_t)(it >> 1) & 1u)) sh.lost = 1;
+    if (!mbar_wait(sh.full + buf, (pass >> 1) & 1u)) sh.lost = 1;
     const float4* band = sh_band + buf * kBandCap;
     double fx = 0.0, fy = 0.0, w = 0.0, u = 0.0, an = 0.0;
     int tci = 0;
     if (act) {
       const bool staged = sh.bands[buf].total > 0;
-      const float4 qi = staged ? band[band_place(sh.bands[buf], (int)i)] : __ldg(D.pff + i);
+      const float4 qi = staged ? band[band_place(sh.bands[buf], (int)i)] : ld_pos<NC>(D.pff + i);
       tci = (int)ff_class(qi);
       PairCtx c;
       PairCtxD cd;
@@ -516,24 +537,24 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
       const int groups = ((nc & (kListInterior - 1)) + 3) >> 2;
       if (nc >= 0 && (nc & kListInterior) != 0) {
         if (HP)
-          band_list_hp<PY, kEnergy, kVirial, false>(band, D.lists + i, D.ntot, groups, cd, fx, fy,
+          band_list_hp<PY, kEnergy, kVirial, false, NC>(band, D.lists + i, D.ntot, groups, cd, fx, fy,
                                                     w, u, an);
         else
-          band_list<PY, kEnergy, kVirial, false, kFloor>(band, D.lists + i, D.ntot, groups, c, fs,
+          band_list<PY, kEnergy, kVirial, false, kFloor, NC>(band, D.lists + i, D.ntot, groups, c, fs,
                                                          fc, ws, wc, u, an);
       } else {
         if (!HP) set_pair_box<PY>(c, qi, Lx, Ly);
         if (nc >= 0) {
           if (HP)
-            band_list_hp<PY, kEnergy, kVirial, true>(band, D.lists + i, D.ntot, groups, cd, fx, fy,
+            band_list_hp<PY, kEnergy, kVirial, true, NC>(band, D.lists + i, D.ntot, groups, cd, fx, fy,
                                                      w, u, an);
           else
-            band_list<PY, kEnergy, kVirial, true, kFloor>(band, D.lists + i, D.ntot, groups, c, fs,
+            band_list<PY, kEnergy, kVirial, true, kFloor, NC>(band, D.lists + i, D.ntot, groups, c, fs,
                                                           fc, ws, wc, u, an);
         } else {
           // no list: the stencil's runs from the band (or, without one, from
           // global memory), or the whole system
-          const int cell = S.allpairs ? 0 : D.cell_of[i];
+          const int cell = S.allpairs ? 0 : ld_idx<NC>(D.cell_of + i);
           const int cx = cell % S.ncx, cy = cell / S.ncx;
 #pragma unroll 1
           for (int r = 0; r < 6; ++r) {
@@ -542,7 +563,7 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
               if (r > 0) break;
               a = (int)P.p0;
               e = (int)end;
-            } else if (!stencil_run<PY>(D.cstart + P.c0, S.ncx, S.ncy, cx, cy, r, &a, &e)) {
+            } else if (!stencil_run<PY, NC>(D.cstart + P.c0, S.ncx, S.ncy, cx, cy, r, &a, &e)) {
               continue;
             }
             const float4* src = staged ? band + band_place(sh.bands[buf], a) : D.pff + a;
@@ -598,14 +619,16 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
 }
 
 // The FP64 form out of line: its registers do not count against the FP32 loop.
-template <int FM, bool PY>
+template <int FM, bool PY, bool NC>
 __device__ __noinline__ ForceFinish<FM, PY> band_items_hp(Dev D, const SysParams* P,
                                                           const SysState* S, BandShared* sh,
-                                                          float4* sh_band, int q_first,
-                                                          int items) {
+                                                          float4* sh_band, int q_first, int items,
+                                                          uint32_t* pass) {
   ForceFinish<FM, PY> fin;
   fin.init();
-  band_items<FM, PY, true>(D, *P, *S, *sh, sh_band, q_first, items, fin);
+  uint32_t at = *pass;
+  band_items<FM, PY, true, NC>(D, *P, *S, *sh, sh_band, q_first, items, at, fin);
+  *pass = at;
   return fin;
 }
 
@@ -636,11 +659,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_band(Dev D) {
   const int items = skip ? 0 : P.items;
   __syncthreads();
   ForceFinish<FM, PY> fin;
+  uint32_t pass = 0;
   if (kHpCapable && S->f_fp64 != 0) {
-    fin = band_items_hp<FM, PY>(D, &P, S, &sh, sh_band, b - P.b0, items);
+    fin = band_items_hp<FM, PY, true>(D, &P, S, &sh, sh_band, b - P.b0, items, &pass);
   } else {
     fin.init();
-    band_items<FM, PY, false>(D, P, *S, sh, sh_band, b - P.b0, items, fin);
+    band_items<FM, PY, false, true>(D, P, *S, sh, sh_band, b - P.b0, items, pass, fin);
   }
   if (fin.bad) atomicOr(&S->nonfinite, 1);
   ForceTail tin;

@@ -15,6 +15,7 @@
 
 #include "mdb_engine.h"
 #include "mdb_band.cuh"
+#include "mdb_band_steps.cuh"
 #include "mdb_kernels.cuh"
 #include "mdb_steps.cuh"
 #include "mdb_util.h"
@@ -101,6 +102,16 @@ void* steps_fn(int dm, bool ln) {
     default: return (void*)k_run_steps<DM_FIRE, FM_FIRE, false>;
   }
 #undef MDB_S
+}
+
+void* band_steps_fn(int dm) {
+  switch (dm) {
+    case DM_NVE: return (void*)k_run_band<DM_NVE, FM_NVE>;
+    case DM_NH: return (void*)k_run_band<DM_NH, FM_NH>;
+    case DM_NPH: return (void*)k_run_band<DM_NPH, FM_NPH>;
+    case DM_PISTON: return (void*)k_run_band<DM_PISTON, FM_PISTON>;
+    default: return (void*)k_run_band<DM_FIRE, FM_FIRE>;
+  }
 }
 
 namespace {
@@ -484,76 +495,96 @@ int Engine::build() {
   return autotune_ ? tune() : MDB_OK;
 }
 
-// The resident steps kernel (mdb_steps.cuh) needs every block of the (single)
-// system on the device at once, at one slot per thread. AUTO and MULTI take it
-// whenever that holds, for calls of any length: up to that size launches,
-// reduction tails and barriers dominate a step.
+// Steps of a single system in one launch need all of its blocks on the device
+// at once. At one slot per thread, two blocks an SM (up to 75,776 particles on
+// 148 SMs): the resident steps kernel (mdb_steps.cuh), state in registers. Above
+// that: the steps kernel over staged bands (mdb_band_steps.cuh), one wave of
+// four blocks an SM, which every size fits (its slots per thread grow). AUTO and
+// MULTI take them for calls of any length: launches, reduction tails and
+// barriers dominate a step of the small systems and are a quarter of it at
+// 262,144.
 int Engine::choose_multi_step() {
-  multi_step_ = false;
+  multi_step_ = band_steps_ = false;
   multi_cap_ = 0;
   schedule_.multi_step = 0;
   schedule_.multi_step_blocks = 0;
   if (nsys() != 1 || !use_graphs_ || step_kernel_ == MDB_STEPS_PER_PHASE) return MDB_OK;
-  if (hsp_[0].items != 1) return MDB_OK;
   int nsm = 0;
   MDB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device_));
   int coop = 0;
   MDB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_));
   if (!coop) return MDB_OK;
+  const bool fire = hsp_[0].kind == K_FIRE;
+  // blocks of a kernel family that fit at once (the least over its modes)
+  auto capacity = [&](bool bands, size_t smem, int* out) -> int {
+    int per_sm = 1 << 30;
+    for (int dm : {DM_NVE, DM_NH, DM_NPH, DM_PISTON, DM_FIRE}) {
+      if (fire != (dm == DM_FIRE)) continue;
+      int b = 0;
+      MDB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+          &b, bands ? band_steps_fn(dm) : steps_fn(dm, lanes_), kThreads, smem));
+      per_sm = std::min(per_sm, b);
+    }
+    *out = per_sm * nsm;
+    return MDB_OK;
+  };
   // Shared list columns: 16-bit offsets, up to 40 KB a block (80 entries per
   // thread); longer or 32-bit lists are read from global memory.
   const int per = (max_nbr_ + hsp_[0].lanes - 1) / hsp_[0].lanes;
   const int rows = (per + kListGroup - 1) / kListGroup * kListGroup;
   steps_.list_rows = (dev_.nl16 && rows > 0 && rows <= 80) ? rows : 0;
   steps_smem_ = sizeof(int16_t) * kThreads * (size_t)steps_.list_rows;
-  const bool fire = hsp_[0].kind == K_FIRE;
-  int per_sm = 1 << 30;
-  for (int dm : {DM_NVE, DM_NH, DM_NPH, DM_PISTON, DM_FIRE}) {
-    if (fire != (dm == DM_FIRE)) continue;
-    int b = 0;
-    MDB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, steps_fn(dm, lanes_), kThreads,
-                                                           steps_smem_));
-    per_sm = std::min(per_sm, b);
-  }
-  multi_cap_ = per_sm * nsm;
-  if (nblocks_ >= 1 && nblocks_ <= multi_cap_) {
-    auto alloc = [&](void** p, size_t bytes) -> int {
-      MDB_CUDA(cudaMalloc(p, bytes));
-      allocs_.push_back(*p);
-      bytes_ += (int64_t)bytes;
-      MDB_CUDA(cudaMemsetAsync(*p, 0, bytes, stream_));
-      return MDB_OK;
-    };
-    // one zeroed allocation: positions, block sums, maxima, counts, sequence
-    const size_t pos = sizeof(float4) * (size_t)ntot_;
-    const size_t part = sizeof(double) * 2 * kNP * (size_t)nblocks_;
-    const size_t mx = sizeof(unsigned long long) * 16;
-    const size_t cnt = sizeof(int32_t) * (size_t)(nblocks_ + 2);
-    char* base = nullptr;
-    int rc = alloc((void**)&base, pos + part + mx + cnt);
-    if (rc) return rc;
-    steps_.pff1 = (float4*)base;
-    steps_.part = (double*)(base + pos);
-    steps_.max = (unsigned long long*)(base + pos + part);
-    steps_.seq = (uint32_t*)(base + pos + part + mx);
-    steps_.tile = (int32_t*)(steps_.seq + 2);
-    multi_step_ = true;
-  }
+  int rc = capacity(false, steps_smem_, &multi_cap_);
+  if (rc) return rc;
+  multi_step_ = hsp_[0].items == 1 && nblocks_ <= multi_cap_;
   schedule_.multi_step = multi_step_ ? 1 : 0;
   schedule_.multi_step_blocks = multi_cap_;
+  if (!multi_step_ && !lanes_) {
+    steps_smem_ = sizeof(float4) * (2 * kBandCap + kBandRoom);
+    int cap = 0;
+    rc = capacity(true, steps_smem_, &cap);
+    if (rc) return rc;
+    band_steps_ = nblocks_ <= cap;
+  }
+  if (!multi_step_ && !band_steps_) return MDB_OK;
+  // one zeroed allocation: positions (second buffer), block sums, maxima,
+  // sequence, tile counts
+  const size_t pos = multi_step_ ? sizeof(float4) * (size_t)ntot_ : 0;
+  const size_t part = sizeof(double) * 2 * kNP * (size_t)nblocks_;
+  const size_t mx = sizeof(unsigned long long) * 16;
+  const size_t cnt = sizeof(int32_t) * (size_t)(nblocks_ + 2);
+  const size_t bytes = pos + part + mx + cnt;
+  char* base = nullptr;
+  MDB_CUDA(cudaMalloc((void**)&base, bytes));
+  allocs_.push_back(base);
+  bytes_ += (int64_t)bytes;
+  MDB_CUDA(cudaMemsetAsync(base, 0, bytes, stream_));
+  steps_.pff1 = (float4*)base;
+  steps_.part = (double*)(base + pos);
+  steps_.max = (unsigned long long*)(base + pos + part);
+  steps_.seq = (uint32_t*)(base + pos + part + mx);
+  steps_.tile = (int32_t*)(steps_.seq + 2);
   return MDB_OK;
 }
 
-// n steps (FIRE: iterations) in one cooperative launch.
+// n steps (FIRE: iterations) in cooperative launches. A launch holds the device
+// until it ends, so it is kept short enough for the kernels of other streams to
+// run in between.
 int Engine::run_resident(int dm, int64_t n) {
   Dev d = dev_;
   d.use_cond = 0;
   StepsMem m = steps_;
-  void* args[] = {&d, &m, &n};
-  MDB_CUDA(cudaLaunchCooperativeKernel(steps_fn(dm, lanes_), dim3(nblocks_), dim3(kThreads), args,
-                                       steps_smem_, stream_));
-  launches_ += 1;
-  count_launches(1);
+  const int64_t most = multi_step_ ? 256 : 64;
+  for (int64_t left = n; left > 0;) {
+    int64_t k = std::min(left, most);
+    void* args[] = {&d, &m, &k};
+    MDB_CUDA(cudaLaunchCooperativeKernel(multi_step_ ? steps_fn(dm, lanes_) : band_steps_fn(dm),
+                                         dim3(nblocks_), dim3(kThreads), args, steps_smem_,
+                                         stream_));
+    launches_ += 1;
+    count_launches(1);
+    left -= k;
+  }
   return MDB_OK;
 }
 
@@ -707,7 +738,7 @@ int Engine::get_graph(int kind, int dm, int fm, bool py, int chunk, cudaGraphExe
 int Engine::run_md(int dm, int fm, bool py, int64_t nsteps) {
   if (!built_) return set_error(MDB_ERR_STATE, "engine not built");
   MDB_CUDA(cudaSetDevice(device_));
-  if (multi_step_ && py == (dm != DM_PISTON)) return run_resident(dm, nsteps);
+  if ((multi_step_ || band_steps_) && py == (dm != DM_PISTON)) return run_resident(dm, nsteps);
   int64_t left = nsteps;
   if (use_graphs_) {
     static const int kChunks[] = {64, 8, 1};
@@ -770,7 +801,7 @@ int Engine::run_md_timed(int dm, int fm, bool py, int64_t nsteps, double* ms) {
 int Engine::run_fire(int64_t iters) {
   if (!built_) return set_error(MDB_ERR_STATE, "engine not built");
   MDB_CUDA(cudaSetDevice(device_));
-  if (multi_step_) return run_resident(DM_FIRE, iters);
+  if (multi_step_ || band_steps_) return run_resident(DM_FIRE, iters);
   int64_t left = iters;
   if (use_graphs_) {
     static const int kChunks[] = {100, 10, 1};

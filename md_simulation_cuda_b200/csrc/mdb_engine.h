@@ -136,8 +136,8 @@ class Engine {
   void drop_graphs();
   // The cached protocol graph (built at the first protocol run).
   int proto_graph(cudaGraphExec_t* exec);
-  // Whether steps run in the resident steps kernel (single system, all blocks
-  // resident), and n of them in one launch of it.
+  // Whether steps run in one of the resident steps kernels (single system, all
+  // blocks resident), and n of them that way.
   int choose_multi_step();
   int run_resident(int dm, int64_t n);
   void free_proto();
@@ -168,6 +168,7 @@ class Engine {
   bool lanes_ = false;  // some system has several lanes per slot (SysParams::lanes)
   int lanes_opt_ = MDB_LANES_ONE;  // mdb_options_t.lanes (AUTO counts as ONE here)
   int multi_cap_ = 0;  // blocks of the resident steps kernel the device holds at once
+  bool band_steps_ = false;  // the one over staged bands
   StepsMem steps_{};
   size_t steps_smem_ = 0;
   mdb_schedule_t schedule_{};

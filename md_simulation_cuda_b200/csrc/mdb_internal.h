@@ -26,9 +26,8 @@ constexpr double kSkinMD = 0.45;   // automatic list skin: MD systems
 constexpr double kSkinFire = 0.2;  // automatic list skin: a handle of FIRE systems only
 constexpr double kFireFp64Below = 1e-3;  // FIRE: FP64 pair terms below this max |a|
 constexpr int kNP = 6;         // reduction slots per block
-constexpr int kScanItems = 4;  // cells per thread in the scan kernels
-constexpr int kScanBlock = 512;
-constexpr int kScanTile = kScanItems * kScanBlock;
+constexpr int kScanItems = 8;   // cells per thread in the scan
+constexpr int kScanTile = kScanItems * kThreads;
 // ncount[] flag: the list needs neither the minimum image nor offset wrapping.
 constexpr int32_t kListInterior = 1 << 30;
 // Force phase: list rows of the next chunk prefetched into L1 per warp

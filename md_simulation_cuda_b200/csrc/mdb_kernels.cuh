@@ -1663,8 +1663,7 @@ struct RebuildSlots {
 
 // Cell of each slot, its arrival rank in the cell (arbitrary), and the particles
 // per cell and tile.
-__global__ void __launch_bounds__(kThreads) k_rb_bin(Dev D) {
-  if (!rebuild_requested(D)) return;
+__device__ __forceinline__ void rb_bin(const Dev& D) {
   constexpr int K = 4;
   const int lane = threadIdx.x & 31;
   for (int q = blockIdx.x; q < D.nchunks; q += K * (int)gridDim.x) {
@@ -1711,10 +1710,14 @@ __global__ void __launch_bounds__(kThreads) k_rb_bin(Dev D) {
   }
 }
 
+__global__ void __launch_bounds__(kThreads) k_rb_bin(Dev D) {
+  if (rebuild_requested(D)) rb_bin(D);
+}
+
 // First slot of each cell: the system's first slot, the particles of the tiles
-// before and of the cells before in the tile.
-__global__ void __launch_bounds__(kScanBlock) k_rb_scan(Dev D) {
-  if (!rebuild_requested(D)) return;
+// before and of the cells before in the tile. A block of kScanBlock threads.
+constexpr int kScanBlock = kScanTile / kScanItems;
+__device__ __forceinline__ void rb_scan(const Dev& D) {
   __shared__ int sh[kScanBlock / 32];
   __shared__ int sh_before[kScanBlock / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1768,8 +1771,11 @@ __global__ void __launch_bounds__(kScanBlock) k_rb_scan(Dev D) {
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_rb_scatter(Dev D) {
-  if (!rebuild_requested(D)) return;
+__global__ void __launch_bounds__(kScanBlock) k_rb_scan(Dev D) {
+  if (rebuild_requested(D)) rb_scan(D);
+}
+
+__device__ __forceinline__ void rb_scatter(const Dev& D) {
   constexpr int K = 4;
   for (int q = blockIdx.x; q < D.nchunks; q += K * (int)gridDim.x) {
     const RebuildSlots<K> R(D, q);
@@ -1789,15 +1795,17 @@ __global__ void __launch_bounds__(kThreads) k_rb_scatter(Dev D) {
   }
 }
 
+__global__ void __launch_bounds__(kThreads) k_rb_scatter(Dev D) {
+  if (rebuild_requested(D)) rb_scatter(D);
+}
+
 // Each particle to its place: after the particles of lower source slots in its
 // cell (the stable sort by cell), with the float-float copy, the cell and the
 // rebuild position. A thread takes an entry of perm, so a warp's reads may
 // scatter (particles that moved far) while its writes stay inside a few cells.
-__global__ void __launch_bounds__(kThreads, 4) k_rb_permute(Dev D) {
-  if (!rebuild_requested(D)) return;
+// (Inside an MD step the force phase that follows writes the accelerations.)
+__device__ __forceinline__ void rb_permute(const Dev& D, bool forced) {
   constexpr int K = 2;
-  // (inside an MD step the force phase that follows writes the accelerations)
-  const bool forced = *((volatile int*)&D.bg->forced) != 0;
   for (int q = blockIdx.x; q < D.nchunks; q += K * (int)gridDim.x) {
     const RebuildSlots<K> R(D, q);
     int src[K], cell[K], ca[K], ce[K], before[K];
@@ -1844,6 +1852,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_rb_permute(Dev D) {
       D.sb[at] = make_float2(sx, sy);
     }
   }
+}
+
+__global__ void __launch_bounds__(kThreads, 4) k_rb_permute(Dev D) {
+  if (rebuild_requested(D)) rb_permute(D, *((volatile int*)&D.bg->forced) != 0);
 }
 
 // Steps (MD) or iterations (FIRE) the system has run: the clock of its

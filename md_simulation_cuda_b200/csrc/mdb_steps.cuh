@@ -64,6 +64,29 @@ struct StepsShared {
   int need, stop, abort;
 };
 
+// The system's parameters and state into shared memory (a block barrier before
+// their first use is the caller's).
+__device__ __forceinline__ void load_state(const Dev& D, StepsShared& sh) {
+  for (int k = threadIdx.x; k < (int)(sizeof(SysParams) / 4); k += kThreads)
+    ((uint32_t*)&sh.P)[k] = ((const uint32_t*)D.sp)[k];
+  for (int k = threadIdx.x; k < (int)(sizeof(SysState) / 4); k += kThreads)
+    ((uint32_t*)&sh.S)[k] = ((const uint32_t*)D.st)[k];
+  if (threadIdx.x == 0) {
+    sh.need = 0;
+    sh.stop = 0;
+    sh.abort = 0;
+  }
+}
+// The state back to global memory (one block), but for what other blocks count
+// there themselves.
+__device__ __forceinline__ void store_state(const Dev& D, const SysState& S) {
+  for (int k = threadIdx.x; k < (int)(sizeof(SysState) / 4); k += kThreads) {
+    const size_t at = (size_t)k * 4;
+    if (at == offsetof(SysState, nonfinite) || at == offsetof(SysState, nl_overflow)) continue;
+    ((uint32_t*)D.st)[k] = ((const uint32_t*)&S)[k];
+  }
+}
+
 // What the threads of a block bring to an exchange, and thread 0 takes from
 // it: sums, maxima of 32-bit values (non-negative floats as bits, flags) and
 // one maximum of 64-bit ones (a non-negative double as bits).
@@ -387,15 +410,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
   __shared__ StepsShared sh;
   extern __shared__ int16_t sh_lists[];  // [list_rows][kThreads]
   const int tid = threadIdx.x;
-  for (int k = tid; k < (int)(sizeof(SysParams) / 4); k += kThreads)
-    ((uint32_t*)&sh.P)[k] = ((const uint32_t*)D.sp)[k];
-  for (int k = tid; k < (int)(sizeof(SysState) / 4); k += kThreads)
-    ((uint32_t*)&sh.S)[k] = ((const uint32_t*)D.st)[k];
-  if (tid == 0) {
-    sh.need = 0;
-    sh.stop = 0;
-    sh.abort = 0;
-  }
+  load_state(D, sh);
   uint32_t seq = *M.seq;
   const uint32_t seq0 = seq;
   __syncthreads();
@@ -758,11 +773,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
   // Every block has read D.st and M.seq (it took part in an exchange) unless
   // there was none, in which case nothing a block acts on has changed.
   if (blockIdx.x == 0) {
-    for (int k = tid; k < (int)(sizeof(SysState) / 4); k += kThreads) {
-      const size_t at = (size_t)k * 4;
-      if (at == offsetof(SysState, nonfinite) || at == offsetof(SysState, nl_overflow)) continue;
-      ((uint32_t*)D.st)[k] = ((const uint32_t*)&S)[k];
-    }
+    store_state(D, S);
     if (tid == 0 && seq != seq0) *M.seq = seq;
   }
 }

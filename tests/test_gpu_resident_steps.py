@@ -1,4 +1,5 @@
-"""The resident steps kernel (csrc/mdb_steps.cuh) against one kernel per phase.
+"""The resident steps kernels (csrc/mdb_steps.cuh, mdb_band_steps.cuh) against one
+kernel per phase.
 
 Sizes at the edges of its blocks (64 slots with four lanes a slot up to 16,384
 particles, 256 with one lane after that) and of what fits on the device, every
@@ -62,6 +63,18 @@ def test_beyond_the_device(built):
     assert mdb.MDSimulation(cfg, frame=f).schedule()["multi_step"] == 0
 
 
+@pytest.mark.parametrize("n,aspect,opt", [
+    (75777 + 256, 2.0, {}), (80001, 0.01, {}), (100003, 60.0, {}), (151808, 1.0, {}),
+    (230001, 3.0, {}), (90001, 1.0, dict(max_neighbors=15)), (90001, 1.0, dict(max_neighbors=-1)),
+    (90001, 1.0, dict(skin=1.4))])
+def test_staged_steps_equal_per_phase(built, n, aspect, opt):
+    """Systems of several hundred blocks: the steps kernel over staged bands."""
+    f, cfg = _frame(n, aspect)
+    _, a = _run(f, cfg, mdb.STEPS_PER_PHASE, 30, **opt)
+    _, b = _run(f, cfg, mdb.STEPS_AUTO, 30, **opt)
+    assert a == b
+
+
 @pytest.mark.parametrize("opt", [dict(max_neighbors=-1), dict(max_neighbors=14),
                                  dict(max_neighbors=400), dict(skin=0.12), dict(skin=1.4),
                                  dict(lanes=mdb.LANES_ONE),
@@ -74,7 +87,8 @@ def test_list_forms(built, opt):
 
 
 @pytest.mark.parametrize("n,precision,random", [(40, 0, False), (256, 2, True), (700, 0, True),
-                                                (2048, 1, False), (30001, 0, False)])
+                                                (2048, 1, False), (30001, 0, False),
+                                                (90001, 0, False), (160001, 2, False)])
 def test_fire_equals_per_phase(built, n, precision, random):
     if random:
         f, L = wl.random_frame(n, 0.8, 0.5, seed=n)
