@@ -146,6 +146,7 @@ Engine::~Engine() {
   drop_graphs();
   free_proto();
   for (void* p : allocs_) cudaFree(p);
+  if (d_prof_) cudaFree(d_prof_);
   if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -869,39 +870,51 @@ int Engine::get_frame(int s, mdb_particle_t* out) {
 
 int Engine::profiles(int s, int nb, bool py, double* ptens, int32_t* counts) {
   MDB_CUDA(cudaSetDevice(device_));
-  unsigned long long* d_acc = nullptr;
-  int* d_cnt = nullptr;
-  MDB_CUDA(cudaMalloc(&d_acc, sizeof(unsigned long long) * 3 * (size_t)nb));
-  cudaError_t e = cudaMalloc(&d_cnt, sizeof(int) * 2 * (size_t)nb);
-  if (e != cudaSuccess) {
-    cudaFree(d_acc);
-    return cuda_error(e, "cudaMalloc (profiles)");
+  // bins on the device: 3 nb sums, then 2 nb counts; kept, and grown on demand
+  const size_t bytes = (sizeof(unsigned long long) * 3 + sizeof(int) * 2) * (size_t)nb;
+  if (prof_bytes_ < bytes) {
+    if (d_prof_) cudaFree(d_prof_);  // (every call waits for its kernels below)
+    d_prof_ = nullptr;
+    bytes_ -= (int64_t)prof_bytes_;
+    prof_bytes_ = 0;
+    MDB_CUDA(cudaMalloc(&d_prof_, bytes));
+    prof_bytes_ = bytes;
+    bytes_ += (int64_t)bytes;
   }
-  e = cudaMemsetAsync(d_acc, 0, sizeof(unsigned long long) * 3 * (size_t)nb, stream_);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, sizeof(int) * 2 * (size_t)nb, stream_);
-  if (e == cudaSuccess) {
-    const int g = (int)std::max<int64_t>(1, std::min<int64_t>((hsp_[s].n + kThreads - 1) / kThreads, 4096));
-    if (py)
-      k_profiles<true><<<g, kThreads, 0, stream_>>>(dev_, s, nb, d_acc, d_cnt);
-    else
-      k_profiles<false><<<g, kThreads, 0, stream_>>>(dev_, s, nb, d_acc, d_cnt);
-    e = cudaGetLastError();
+  unsigned long long* d_acc = (unsigned long long*)d_prof_;
+  int* d_cnt = (int*)(d_acc + 3 * (size_t)nb);
+  MDB_CUDA(cudaMemsetAsync(d_prof_, 0, bytes, stream_));
+  const SysParams& P = hsp_[s];
+  const int g = (int)std::max<int64_t>(1, std::min<int64_t>((P.n + kThreads - 1) / kThreads, 4096));
+  if (counts) {
+    k_count_profile<<<g, kThreads, 0, stream_>>>(dev_, s, nb, d_cnt);
+    MDB_CUDA(cudaGetLastError());
     launches_ += 1;
     count_launches(1);
   }
-  std::vector<long long> acc((size_t)3 * nb);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(acc.data(), d_acc, sizeof(long long) * acc.size(), cudaMemcpyDeviceToHost,
-                        stream_);
-  if (e == cudaSuccess && counts)
-    e = cudaMemcpyAsync(counts, d_cnt, sizeof(int) * 2 * (size_t)nb, cudaMemcpyDeviceToHost,
-                        stream_);
-  if (e == cudaSuccess) e = wait_host();
-  cudaFree(d_acc);
-  cudaFree(d_cnt);
-  if (e != cudaSuccess) return cuda_error(e, "profiles");
-  if (ptens)
-    for (size_t k = 0; k < acc.size(); ++k) ptens[k] = (double)acc[k] / kProfileFix;
+  std::vector<long long> acc(ptens ? (size_t)3 * nb : 0);
+  if (ptens) {
+    // a window reaches as far as a pair's midpoint is from its particle (half
+    // the largest cutoff), within 48 KB of shared memory; finer bins than that
+    // covers add to the global bins one by one
+    const double reach = 0.5 * P.rc_max * (double)nb / P.Ly0;
+    const int win = 2 * (int)std::min(3.0, std::max(1.0, ceil(reach))) + 1;
+    const size_t smem = sizeof(unsigned long long) * 3 * (size_t)win * kThreads;
+    if (py)
+      k_pressure_profile<true><<<g, kThreads, smem, stream_>>>(dev_, s, nb, win, d_acc);
+    else
+      k_pressure_profile<false><<<g, kThreads, smem, stream_>>>(dev_, s, nb, win, d_acc);
+    MDB_CUDA(cudaGetLastError());
+    launches_ += 1;
+    count_launches(1);
+    MDB_CUDA(cudaMemcpyAsync(acc.data(), d_acc, sizeof(long long) * acc.size(),
+                             cudaMemcpyDeviceToHost, stream_));
+  }
+  if (counts)
+    MDB_CUDA(cudaMemcpyAsync(counts, d_cnt, sizeof(int) * 2 * (size_t)nb, cudaMemcpyDeviceToHost,
+                             stream_));
+  MDB_CUDA(wait_host());
+  for (size_t k = 0; k < acc.size(); ++k) ptens[k] = (double)acc[k] / kProfileFix;
   return MDB_OK;
 }
 

@@ -175,6 +175,8 @@ class Engine {
   int stream_priority_ = 0;  // levels above normal for stream_
   int64_t aos_cap_ = 0;
   void* d_aos_ = nullptr;
+  void* d_prof_ = nullptr;  // bins of profiles()
+  size_t prof_bytes_ = 0;
   void* d_obs_ = nullptr;  // one mdb_observables_t staging slot
   std::vector<void*> allocs_;
   std::map<std::tuple<int, int, int, int, int>, std::pair<cudaGraph_t, cudaGraphExec_t>> graphs_;
