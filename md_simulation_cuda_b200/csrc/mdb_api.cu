@@ -46,12 +46,17 @@ mdb_options_t opts_or_default(const mdb_options_t* opt) {
   return o;
 }
 
-int check_status(mdb_sim_t* sim) {
-  SysState S;
-  MDB_TRY(sim->eng->get_state(0, &S));
+// The error a system's state records.
+int state_status(const SysState& S) {
   if (S.err == MDB_ERR_BOX) return mdb::set_error(MDB_ERR_BOX, "invalid box (area <= 0 or non-finite) in a barostat step");
   if (S.err) return mdb::set_error(S.err, "device error flag set");
   return MDB_OK;
+}
+
+int check_status(mdb_sim_t* sim) {
+  SysState S;
+  MDB_TRY(sim->eng->get_state(0, &S));
+  return state_status(S);
 }
 
 int sim_make(const mdb_config_t* cfg, std::vector<mdb_particle_t>&& frame,
@@ -240,7 +245,7 @@ int mdb_sim_step_nph(mdb_sim_t* sim, double p_ext, int64_t nsteps) {
   if (!sim->nph_init || !sim->p_valid) {
     if (!sim->p_valid) MDB_TRY(sim->eng->force(mdb::FM_OBS, true));
     MDB_TRY(sim->eng->get_state(0, &S));
-    if (S.err) return check_status(sim);
+    if (S.err) return state_status(S);
     if (!sim->nph_init) {
       // init_nph_state_if_needed (src/md_env.cu:1757-1778)
       if (!(S.Lx > 0.0) || !(S.Ly > 0.0))
@@ -303,7 +308,7 @@ int mdb_sim_total_K(mdb_sim_t* sim, double* out) {
   MDB_TRY(sim->eng->get_state(0, &S));
   sim->k_valid = true;
   *out = S.K;
-  return check_status(sim);
+  return state_status(S);
 }
 
 int mdb_sim_total_U(mdb_sim_t* sim, double* out) {
@@ -312,7 +317,7 @@ int mdb_sim_total_U(mdb_sim_t* sim, double* out) {
   SysState S;
   MDB_TRY(sim->eng->get_state(0, &S));
   *out = sim->piston_active ? S.U + S.wallU : S.U;
-  return check_status(sim);
+  return state_status(S);
 }
 
 int mdb_sim_partial_U_lambda(mdb_sim_t* sim, double epsilon_lambda, double* out) {
@@ -322,7 +327,7 @@ int mdb_sim_partial_U_lambda(mdb_sim_t* sim, double epsilon_lambda, double* out)
   SysState S;
   MDB_TRY(sim->eng->get_state(0, &S));
   *out = -epsilon_lambda * S.Wani;
-  return check_status(sim);
+  return state_status(S);
 }
 
 int mdb_sim_n_profile(mdb_sim_t* sim, int32_t nb, int32_t* out) {
@@ -352,7 +357,7 @@ int mdb_sim_pressure_profile(mdb_sim_t* sim, int32_t nb, double* out) {
   // per bin area Lx * (Ly / nb) (src/md_env.cu:3899-3916)
   const double vol = S.Lx * (S.Ly / (double)nb);
   for (size_t k = 0; k < acc.size(); ++k) out[k] = (vol > 0.0) ? acc[k] / vol : acc[k];
-  return check_status(sim);
+  return state_status(S);
 }
 
 int mdb_sim_instant_pressure(mdb_sim_t* sim, double* out) {
@@ -371,7 +376,7 @@ int mdb_sim_instant_pressure(mdb_sim_t* sim, double* out) {
   }
   MDB_TRY(sim->eng->put_state(0, S));
   *out = S.last_P;
-  return check_status(sim);
+  return state_status(S);
 }
 
 int mdb_sim_observables(mdb_sim_t* sim, mdb_observables_t* out) {
@@ -394,7 +399,7 @@ int mdb_sim_observables(mdb_sim_t* sim, mdb_observables_t* out) {
   out->rebuilds = S.rebuilds;
   out->piston_mode_active = sim->piston_active ? 1 : 0;
   out->nonfinite = S.nonfinite;
-  return check_status(sim);
+  return state_status(S);
 }
 
 int mdb_sim_observables_async(mdb_sim_t* sim, mdb_observables_t* out) {

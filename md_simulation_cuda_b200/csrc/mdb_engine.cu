@@ -849,8 +849,8 @@ int Engine::get_states(std::vector<SysState>& out) {
 
 int Engine::put_state(int s, const SysState& st) {
   MDB_CUDA(cudaSetDevice(device_));
+  // (the call returns once the pageable source has been taken over)
   MDB_CUDA(cudaMemcpyAsync(dev_.st + s, &st, sizeof(SysState), cudaMemcpyHostToDevice, stream_));
-  MDB_CUDA(wait_host());
   return MDB_OK;
 }
 
