@@ -556,6 +556,11 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
           // global memory), or the whole system
           const int cell = S.allpairs ? 0 : ld_idx<NC>(D.cell_of + i);
           const int cx = cell % S.ncx, cy = cell / S.ncx;
+          // the minimum image for the warps that hold a slot within two cells of
+          // a periodic edge (its shift is zero for the others: see k_rb_nlist)
+          const bool image =
+              __any_sync(__activemask(), cx < 2 || cx > S.ncx - 3 ||
+                                             (S.periodic_y && (cy < 2 || cy > S.ncy - 3)));
 #pragma unroll 1
           for (int r = 0; r < 6; ++r) {
             int a, e;
@@ -566,40 +571,22 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
             } else if (!stencil_run<PY, NC>(D.cstart + P.c0, S.ncx, S.ncy, cx, cy, r, &a, &e)) {
               continue;
             }
-            const float4* src = staged ? band + band_place(sh.bands[buf], a) : D.pff + a;
             if constexpr (HP) {
+              const float4* src = staged ? band + band_place(sh.bands[buf], a) : D.pff + a;
 #pragma unroll 1
               for (int m = 0; m < e - a; ++m)
                 pair_one_hp<PY, kEnergy, kVirial, true>(src[m], cd, fx, fy, w, u, an);
+            } else if (staged) {
+              const float4* src = band + band_place(sh.bands[buf], a);
+              if (image)
+                pair_run<kEnergy, kVirial, true, kFloor>(src, e - a, c, fs, fc, ws, wc, u, an);
+              else
+                pair_run<kEnergy, kVirial, false, kFloor>(src, e - a, c, fs, fc, ws, wc, u, an);
             } else {
-            // a test that sets a bit, then the pair term for the set bits: the
-            // warp pays the term for its lane with the most partners, not for
-            // nearly every candidate
 #pragma unroll 1
-            for (int left = e - a; left > 0; left -= 32, src += 32) {
-              const int len = min(left, 32);
-              uint32_t in = 0;
-#pragma unroll 1
-              for (int m = 0; m < len; m += 4) {
-                uint32_t four = 0;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const float4 q = src[m + k < len ? m + k : 0];
-                  float2 d;
-                  const float r2 = pair_r2<true>(q, c, d);
-                  const bool same =
-                      (((__float_as_uint(q.z) ^ c.tsz) | __float_as_uint(q.w)) & 1u) == 0u;
-                  if (__float_as_uint(r2) - 1u < (same ? c.rc2s_m1 : c.rc2ab_m1)) four |= 1u << k;
-                }
-                in |= four << m;
-              }
-              if (len < 32) in &= (1u << len) - 1u;
-              while (in != 0u) {
-                pair_one<PY, kEnergy, kVirial, true, kFloor>(src[__ffs(in) - 1], c, fs, fc, ws, wc,
-                                                             u, an);
-                in &= in - 1u;
-              }
-            }
+              for (int m = a; m < e; ++m)
+                pair_one<PY, kEnergy, kVirial, true, kFloor>(ld_pos<NC>(D.pff + m), c, fs, fc, ws,
+                                                             wc, u, an);
             }
           }
         }

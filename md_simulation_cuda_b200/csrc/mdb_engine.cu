@@ -61,7 +61,8 @@ void* force_band_fn(int fm, bool py) {
 
 Engine::Kernel Engine::force_kernel(int fm, bool py) const {
   if (banded_)
-    return {force_band_fn(fm, py), nblocks_, kThreads, sizeof(float4) * 2 * kBandCap};
+    return {force_band_fn(fm, py), nblocks_, kThreads,
+            sizeof(float4) * (2 * kBandCap + kBandRoom)};
   return {force_fn(fm, py, lanes_), nblocks_, kThreads, 0};
 }
 

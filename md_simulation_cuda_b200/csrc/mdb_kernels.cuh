@@ -428,41 +428,90 @@ __device__ __forceinline__ float pair_r2(const float4 q, const PairCtx& c, float
   return fmaf(d.x, d.x, d.y * d.y);
 }
 
-// The LJ pair term of li_force_kernel (src/md_cuda_common.cu:193-254) for one
-// candidate j: strict cutoff 0 < r^2 < rc_ij^2 in FP32, FP32 pair force, Kahan
-// FP32 accumulation. ENERGY adds 1/2 (u_ij - V_c) in FP64 (:795-807); VIRIAL
-// adds 1/2 r.F (:676-686) as the compensated FP32 sum of tmp*r^2.
+// Whether candidate q's class equals the slot's (classes 0 and 1: the lo bits of
+// x and y are 0 / 0 and 1 / 0); a class-2 slot has its "same" parameters set to
+// AB.
+__device__ __forceinline__ bool pair_same(const float4 q, const PairCtx& c) {
+  return (((__float_as_uint(q.z) ^ c.tsz) | __float_as_uint(q.w)) & 1u) == 0u;
+}
+// The strict cutoff 0 < r2 < rc2 for the non-negative r2 (NaN fails): bits - 1
+// as unsigned.
+__device__ __forceinline__ bool pair_inside(float r2, bool same, const PairCtx& c) {
+  return __float_as_uint(r2) - 1u < (same ? c.rc2s_m1 : c.rc2ab_m1);
+}
+
+// The LJ pair term of li_force_kernel (src/md_cuda_common.cu:193-254) for a
+// pair inside the cutoff: FP32 pair force, Kahan FP32 accumulation. ENERGY adds
+// 1/2 (u_ij - V_c) in FP64 (:795-807); VIRIAL adds 1/2 r.F (:676-686) as the
+// compensated FP32 sum of tmp*r^2.
+template <bool ENERGY, bool VIRIAL, bool FLOOR>
+__device__ __forceinline__ void pair_term(const float2 d, float r2, bool same, const PairCtx& c,
+                                          float2& fs, float2& fc, float& ws, float& wc, double& u,
+                                          double& an) {
+  // FLOOR (FIRE and observations): pairs closer than ~0.003 sigma (random
+  // starts) take the pair term at r^2 = 1e-5 sigma^2, which keeps it finite
+  // in FP32; the reference's FP32 term overflows to inf/NaN there.
+  if (FLOOR) r2 = fmaxf(r2, same ? c.r2fs : c.r2fab);
+  const float sig2 = same ? c.sig2s : c.sig2ab;
+  const float e24 = same ? c.e24s : c.e24ab;
+  const float r2i = recip(r2);
+  const float sr2 = sig2 * r2i;
+  const float sr6 = sr2 * sr2 * sr2;
+  const float sr12 = sr6 * sr6;
+  const float tmp = e24 * fmaf(2.0f, sr12, -sr6) * r2i;
+  const float2 f = f2mul(make_float2(tmp, tmp), d);
+  kahan2(fs, fc, f);
+  if (VIRIAL) kahan(ws, wc, tmp * r2);
+  if (ENERGY) {
+    const float e4 = same ? c.e4s : c.e4ab;
+    const double vc = same ? c.Vcs : c.Vcab;
+    u = fma(0.5, (double)(e4 * (sr12 - sr6)) - vc, u);
+    // Fx dx - Fy dy of cal_partial_U_lambda_kernel (src/md_cuda_common.cu:
+    // 345-355): products of FP32 values, exact in FP64
+    an += (double)f.x * (double)d.x - (double)f.y * (double)d.y;
+  }
+}
+
+// One candidate: the cutoff, then the pair term.
 template <bool PY, bool ENERGY, bool VIRIAL, bool MIC = true, bool FLOOR = false>
 __device__ __forceinline__ void pair_one(const float4 q, const PairCtx& c, float2& fs, float2& fc,
                                          float& ws, float& wc, double& u, double& an) {
   float2 d;
-  float r2 = pair_r2<MIC>(q, c, d);
-  // j's class equals i's (classes 0 and 1: the lo bits of x and y are 0 / 0
-  // and 1 / 0); a class-2 slot i has its "same" parameters set to AB
-  const bool same = (((__float_as_uint(q.z) ^ c.tsz) | __float_as_uint(q.w)) & 1u) == 0u;
-  // 0 < r2 < rc2 for the non-negative r2 (NaN fails): bits - 1 as unsigned
-  if (__float_as_uint(r2) - 1u < (same ? c.rc2s_m1 : c.rc2ab_m1)) {
-    // FLOOR (FIRE and observations): pairs closer than ~0.003 sigma (random
-    // starts) take the pair term at r^2 = 1e-5 sigma^2, which keeps it finite
-    // in FP32; the reference's FP32 term overflows to inf/NaN there.
-    if (FLOOR) r2 = fmaxf(r2, same ? c.r2fs : c.r2fab);
-    const float sig2 = same ? c.sig2s : c.sig2ab;
-    const float e24 = same ? c.e24s : c.e24ab;
-    const float r2i = recip(r2);
-    const float sr2 = sig2 * r2i;
-    const float sr6 = sr2 * sr2 * sr2;
-    const float sr12 = sr6 * sr6;
-    const float tmp = e24 * fmaf(2.0f, sr12, -sr6) * r2i;
-    const float2 f = f2mul(make_float2(tmp, tmp), d);
-    kahan2(fs, fc, f);
-    if (VIRIAL) kahan(ws, wc, tmp * r2);
-    if (ENERGY) {
-      const float e4 = same ? c.e4s : c.e4ab;
-      const double vc = same ? c.Vcs : c.Vcab;
-      u = fma(0.5, (double)(e4 * (sr12 - sr6)) - vc, u);
-      // Fx dx - Fy dy of cal_partial_U_lambda_kernel (src/md_cuda_common.cu:
-      // 345-355): products of FP32 values, exact in FP64
-      an += (double)f.x * (double)d.x - (double)f.y * (double)d.y;
+  const float r2 = pair_r2<MIC>(q, c, d);
+  const bool same = pair_same(q, c);
+  if (pair_inside(r2, same, c))
+    pair_term<ENERGY, VIRIAL, FLOOR>(d, r2, same, c, fs, fc, ws, wc, u, an);
+}
+
+// A run of `len` consecutive candidates, in order: a test that sets a bit, then
+// the pair term for the set bits, so that a warp pays the term for its lane with
+// the most partners instead of for nearly every candidate. (Up to three
+// candidates past the run are read; their bits are cleared.)
+template <bool ENERGY, bool VIRIAL, bool MIC, bool FLOOR>
+__device__ __forceinline__ void pair_run(const float4* src, int len, const PairCtx& c, float2& fs,
+                                         float2& fc, float& ws, float& wc, double& u, double& an) {
+  for (; len > 0; len -= 32, src += 32) {
+    const int part = min(len, 32);
+    uint32_t in = 0;
+#pragma unroll 1
+    for (int m = 0; m < part; m += 4) {
+      uint32_t four = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float4 q = src[m + k];
+        float2 d;
+        const float r2 = pair_r2<MIC>(q, c, d);
+        if (pair_inside(r2, pair_same(q, c), c)) four |= 1u << k;
+      }
+      in |= four << m;
+    }
+    if (part < 32) in &= (1u << part) - 1u;
+    while (in != 0u) {
+      const float4 q = src[__ffs(in) - 1];
+      in &= in - 1u;
+      float2 d;
+      const float r2 = pair_r2<MIC>(q, c, d);
+      pair_term<ENERGY, VIRIAL, FLOOR>(d, r2, pair_same(q, c), c, fs, fc, ws, wc, u, an);
     }
   }
 }
@@ -2122,10 +2171,93 @@ __global__ void __launch_bounds__(kThreads) k_pressure_profile(Dev D, int s, int
         const double ddx = (double)dx, ddy = (double)dy;
         const double Fx = (double)(tmp * dx), Fy = (double)(tmp * dy);
         const int bp = profile_bin(p.y - 0.5 * ddy, Ly, nb, PY);
-        fix_add(ptens + bp, 0.5 * ddx * Fx);
-        fix_add(ptens + nb + bp, 0.5 * ddy * Fy);
-        fix_add(ptens + 2 * nb + bp, 0.5 * ddx * Fy);
+        const unsigned long long xx = to_fix(0.5 * ddx * Fx), yy = to_fix(0.5 * ddy * Fy),
+                                 xy = to_fix(0.5 * ddx * Fy);
+        int d = bp - bk;
+        if (2 * d > nb) d -= nb;  // across the periodic edge
+        if (2 * d < -nb) d += nb;
+        if (d >= -mid && d <= mid) {
+          mine[(mid + d) * kThreads] += xx;
+          mine[(win + mid + d) * kThreads] += yy;
+          mine[(2 * win + mid + d) * kThreads] += xy;
+        } else {
+          atomicAdd(ptens + bp, xx);
+          atomicAdd(ptens + nb + bp, yy);
+          atomicAdd(ptens + 2 * nb + bp, xy);
+        }
+      };
+      const int ncx = S.ncx, ncy = S.ncy;
+      const int cell = S.allpairs ? 0 : D.cell_of[i];
+      const int cx = cell % ncx, cy = cell / ncx;
+      for (int r = 0; r < 6; ++r) {
+        // run r: row r / 2, the second of a row across the periodic x edge
+        int a, e;
+        if (S.allpairs) {
+          if (r > 0) break;
+          a = (int)P.p0;
+          e = (int)(P.p0 + P.n);
+        } else {
+          int y = cy - 1 + (r >> 1);
+          if (PY) {
+            if (y < 0) y += ncy;
+            if (y >= ncy) y -= ncy;
+          } else if (y < 0 || y >= ncy) {
+            continue;
+          }
+          const int32_t* row = D.cstart + P.c0 + (int64_t)y * ncx;
+          const bool inner = cx > 0 && cx < ncx - 1;
+          if ((r & 1) != 0 && inner) continue;
+          if ((r & 1) != 0) {
+            a = row[cx == 0 ? ncx - 1 : 0];
+            e = row[cx == 0 ? ncx : 1];
+          } else {
+            a = row[inner ? cx - 1 : (cx == 0 ? 0 : ncx - 2)];
+            e = row[inner ? cx + 2 : (cx == 0 ? 2 : ncx)];
+          }
+        }
+        // a bit for each pair inside the cutoff, then the terms
+        for (int left = e - a; left > 0; left -= 32, a += 32) {
+          const int len = min(left, 32);
+          uint32_t in = 0;
+          for (int u = 0; u < len; u += 4) {
+            uint32_t four = 0;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+              const float4 q = D.pff[a + min(u + w, len - 1)];
+              float2 dd;
+              const float r2 = pair_r2<true>(q, c, dd);
+              const bool same = (((__float_as_uint(q.z) ^ c.tsz) | __float_as_uint(q.w)) & 1u) == 0u;
+              if (r2 > 0.0f && r2 < (same ? c.rc2s : c.rc2ab)) four |= 1u << w;
+            }
+            in |= four << u;
+          }
+          if (len < 32) in &= (1u << len) - 1u;
+          const int own = (int)i - a;
+          if (own >= 0 && own < 32) in &= ~(1u << own);
+          while (in != 0u) {
+            one(D.pff[a + __ffs(in) - 1]);
+            in &= in - 1u;
+          }
+        }
       }
+    }
+    // the warp's windows, one own bin after the other
+    unsigned todo = __ballot_sync(0xffffffffu, bk >= 0);
+    while (todo != 0u) {
+      const int bin = __shfl_sync(0xffffffffu, bk, __ffs(todo) - 1);
+      const bool part = bk == bin;
+      for (int e = 0; e < 3 * win; ++e) {
+        unsigned long long t = part ? mine[e * kThreads] : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0 && t != 0ull) {
+          int at = bin + e % win - mid;
+          at += at < 0 ? nb : 0;
+          at -= at >= nb ? nb : 0;
+          atomicAdd(ptens + (e / win) * nb + at, t);
+        }
+      }
+      todo &= ~__ballot_sync(0xffffffffu, part);
     }
   }
 }
