@@ -410,18 +410,32 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
   __shared__ StepsShared sh;
   extern __shared__ int16_t sh_lists[];  // [list_rows][kThreads]
   const int tid = threadIdx.x;
+  const int lane = tid % L;
+  const int li = blockIdx.x * spb + tid / L;
+  const bool act = li < (int)D.ntot;  // (the engine's one system)
+  const bool shared_list = M.list_rows > 0;
+  // What does not depend on the system's state is loaded first: a call of one
+  // step is mostly this chain of loads (20 calls of one step, 900 particles:
+  // 281 -> 250 us; a list entry at a time cost a trip to L2 each).
+  int nc = 0;
+  int16_t head[kListGroup];
+  if (act) {
+    nc = D.ncount[li];
+    if (shared_list) {
+#pragma unroll
+      for (int k = 0; k < kListGroup; ++k)
+        head[k] = k * L + lane < D.max_nbr ? D.nlist16[(int64_t)(k * L + lane) * D.ntot + li]
+                                           : (int16_t)0;
+    }
+  }
   load_state(D, sh);
   uint32_t seq = *M.seq;
   const uint32_t seq0 = seq;
   __syncthreads();
   const SysParams& P = sh.P;
   SysState& S = sh.S;
-  const int lane = tid % L;
-  const int li = blockIdx.x * spb + tid / L;
   const int64_t i = P.p0 + li;
-  const bool act = li < P.n;
   const bool own = act && lane == 0;
-  const bool shared_list = M.list_rows > 0;
   const int64_t rebuilds0 = S.rebuilds;
   const int64_t half = half_of(D, &S);  // (the sort in here is in place)
   int16_t* col = sh_lists + tid;
@@ -430,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
   double2 x = make_double2(0.0, 0.0), v = x, a = x;
   float2 sb = make_float2(0.f, 0.f);
   float4 qi = make_float4(0.f, 0.f, 0.f, 0.f);
-  int t = 0, nc = 0, rows = 0;
+  int t = 0, rows = 0;
   if (act) {
     x = D.pos[half + i];
     v = D.vel[half + i];
@@ -438,7 +452,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
     t = D.type[half + i];
     sb = D.sb[i];
     qi = D.pff[i];
-    nc = D.ncount[i];
   }
   // pads this thread's list column to whole groups
   auto pad_column = [&]() {
@@ -450,8 +463,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
   };
   if (act && shared_list) {
     const int kk = pad_column();
-    for (int k = 0; k < kk; ++k)
-      col[k * kThreads] = D.nlist16[(int64_t)(k * L + lane) * D.ntot + i];
+#pragma unroll
+    for (int k = 0; k < kListGroup; ++k)
+      if (k < kk) col[k * kThreads] = head[k];
+    for (int k0 = kListGroup; k0 < kk; k0 += kListGroup) {
+#pragma unroll
+      for (int k = 0; k < kListGroup; ++k)
+        if (k0 + k < kk) head[k] = D.nlist16[(int64_t)((k0 + k) * L + lane) * D.ntot + i];
+#pragma unroll
+      for (int k = 0; k < kListGroup; ++k)
+        if (k0 + k < kk) col[(k0 + k) * kThreads] = head[k];
+    }
   }
   const float4* cur = D.pff;  // positions of the last drift or rebuild
   Totals in, out;

@@ -103,3 +103,13 @@ def test_fire_equals_per_phase(built, n, precision, random):
                     r.nonfinite))
     assert out[0] == out[1]
     assert np.isfinite(out[0][3])
+
+
+@pytest.mark.parametrize("n,aspect", [(80001, 0.3), (151808, 2.0)])
+def test_lists_change_no_bit(built, n, aspect):
+    """Lists against stencil scans, through every integrator (forces of the same
+    pairs in the same order)."""
+    f, cfg = _frame(n, aspect)
+    _, a = _run(f, cfg, mdb.STEPS_AUTO, 45)
+    _, b = _run(f, cfg, mdb.STEPS_AUTO, 45, max_neighbors=-1)
+    assert a == b
