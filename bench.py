@@ -526,9 +526,8 @@ def run_ours(args):
     barrier()
     clk = clocks.stop()
     o1 = sim.observables()
-    # graph launches are counted as drift + force per step; the conditional
-    # rebuild body (11 kernels) runs only on the steps that rebuild
-    launches = mdb.kernel_launches() - l0 + 11 * (o1.rebuilds - o0.rebuilds)
+    # (a step of a single system is one launch; its rebuilds are inside)
+    launches = mdb.kernel_launches() - l0
     t_ms = sum(a.elapsed_time(b) for a, b in ev)
     t_max = max_over_ranks(t_ms / 1e3, dist, dev)
     value = N * ws * args.steps / t_max
@@ -588,9 +587,9 @@ def run_ours(args):
                   "asynchronous observables read into pinned memory, get_frame; wall clock"}
 
     # ---- one call of K steps (a driver that asks for many steps at once) -------
-    # For a system small enough for the multi-step kernel this runs all K
-    # steps in cooperative launches that return only for rebuilds; the L2 is
-    # not flushed inside the call (the state of such a system fits in it).
+    # For a system small enough for the resident steps kernel this runs all K
+    # steps in a few cooperative launches; the L2 is not flushed inside the
+    # call (the state of such a system fits in it).
     long_call = None
     if schedule.get("multi_step"):
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -605,7 +604,7 @@ def run_ours(args):
         t_call = max_over_ranks(a.elapsed_time(b) / 1e3, dist, dev)
         long_call = {"value": N * ws * args.steps / t_call, "unit": "particle-steps/s",
                      "steps_per_call": args.steps, "us_per_step": t_call / args.steps * 1e6,
-                     "how": "one step call of K steps (multi-step kernel), CUDA events, "
+                     "how": "one step call of K steps (resident steps kernel), CUDA events, "
                             "L2 flushed once before the call"}
 
     # ---- C4: the 512-system FIRE mix, batched vs one system at a time --------

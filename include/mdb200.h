@@ -132,18 +132,15 @@ typedef struct mdb_options {
                              ~/.cache/md_simulation_cuda_b200/schedule.txt).
                              None of these changes any result bit.
                              0 (default): the built-in schedule           */
-  int32_t step_kernel;    /* MD steps of a single-system handle:
+  int32_t step_kernel;    /* steps of a single-system handle:
                              MDB_STEPS_AUTO (0, default) or MDB_STEPS_MULTI:
-                             the multi-step kernel when every block of the
-                             system fits on the device at once (two per SM,
-                             so up to ~75k particles on a B200): one
-                             cooperative launch runs the drift and force
-                             phases of many steps with grid barriers between
-                             them and returns only for a cell-list rebuild
-                             (calls of fewer than 4 steps use the per-phase
-                             kernels, whose launch costs less);
+                             the resident steps kernels, for calls of any
+                             length: cooperative launches that run many
+                             steps (or FIRE iterations) each, rebuilds
+                             included; up to ~75k particles with the state
+                             in registers, above that over staged bands;
                              MDB_STEPS_PER_PHASE: one kernel per phase.
-                             Both give the same result bits.               */
+                             All give the same result bits.               */
   int32_t lanes;          /* lanes per particle in the force phase of MD
                              systems of at most 16,384 particles:
                              MDB_LANES_SPLIT: 4 lanes split each particle's
@@ -184,7 +181,8 @@ typedef struct mdb_schedule {
   int32_t from_cache;         /* 1: read from the schedule cache file        */
   double skin;                /* neighbour-list skin                         */
   double tune_ms;             /* time spent timing candidates                */
-  int32_t multi_step;         /* 1: MD steps run in the multi-step kernel    */
+  int32_t multi_step;         /* 1: steps run in the resident steps kernel
+                                 with the state in registers                 */
   int32_t multi_step_blocks;  /* blocks the device holds at once for it      */
 } mdb_schedule_t;
 

@@ -7,7 +7,7 @@
 //   slot back to the caller's particle index.
 //   SoA, FP64 state: pos/vel/acc double2 (16 B each), type int32, theta f64.
 //   pff  float4 per slot: position as an exact float-float pair (hi, lo) in a
-//        biased binade, hi parts' sign bits carry the type class. This is the
+//        biased binade, the lo parts' lowest bits carry the type class. This is the
 //        only array the pair loop gathers (16 B per candidate).
 //   sb   float2 per slot: position at the last rebuild (fractional for periodic
 //        axes, absolute for the piston's walled y axis).
