@@ -554,6 +554,8 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
         } else {
           // no list: the stencil's runs from the band (or, without one, from
           // global memory), or the whole system
+          // (A slot whose position is not a number has no pairs: every test fails.)
+          const bool some = qi.x == qi.x && qi.y == qi.y;
           const int cell = S.allpairs ? 0 : ld_idx<NC>(D.cell_of + i);
           const int cx = cell % S.ncx, cy = cell / S.ncx;
           // the minimum image for the warps that hold a slot within two cells of
@@ -562,7 +564,7 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
               __any_sync(__activemask(), cx < 2 || cx > S.ncx - 3 ||
                                              (S.periodic_y && (cy < 2 || cy > S.ncy - 3)));
 #pragma unroll 1
-          for (int r = 0; r < 6; ++r) {
+          for (int r = some ? 0 : 6; r < 6; ++r) {
             int a, e;
             if (S.allpairs) {
               if (r > 0) break;

@@ -1856,9 +1856,15 @@ __device__ __forceinline__ void rb_permute(const Dev& D, bool forced) {
       ce[k] = R.i[k] >= 0 ? cs[1] : 0;
       before[k] = 0;
     }
+    // (Non-finite positions all bin to cell 0. A cell of more than kSortedCell
+    // particles, which no finite system comes near, keeps the order of arrival:
+    // ordering it would take the square of its size.)
+    constexpr int kSortedCell = 1 << 16;
 #pragma unroll
     for (int k = 0; k < K; ++k)
-      for (int e = ca[k]; e < ce[k]; e += 4) {
+      if (ce[k] - ca[k] > kSortedCell) {
+        before[k] = (int)R.i[k] - ca[k];
+      } else for (int e = ca[k]; e < ce[k]; e += 4) {
         int other[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) other[u] = D.perm[min(e + u, ce[k] - 1)];

@@ -30,7 +30,7 @@
 // rebuild (us per step, one call of many steps, rebuilds included): NVE 4,096
 // particles 17.2 -> 5.0, Nose-Hoover slab 60,013 31 -> 14.8; against one launch
 // per phase (piston, FIRE and one-step calls had no other): piston 20,011
-// 30.6 -> 11.2, 20 one-step NVE calls of 900 particles 495 -> 297 us. What is
+// 30.6 -> 11.2, 20 one-step NVE calls of 900 particles 495 -> 250 us. What is
 // left of a Nose-Hoover step at 4,096 (8.2 us, ~15,000 cycles): exchanges 9,000,
 // pair sums 2,300, drift 1,300, rebuilds 1,600, scalars 1,000.
 #pragma once

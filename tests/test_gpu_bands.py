@@ -51,3 +51,14 @@ def test_large_systems_against_the_oracle(built, n, aspect, periodic):
                          cells=True)
     assert np.linalg.norm(acc - F) <= 1e-5 * np.linalg.norm(F)
     assert abs(U - Uo) <= 1e-6 * abs(Uo)
+
+
+@pytest.mark.parametrize("n", [100003, 400001])
+def test_nonfinite_system_ends(built, n):
+    """A system that has lost its numbers (all positions in one cell) still steps
+    in bounded time and says so."""
+    f, Lx, Ly = wl.lattice_frame(n, 0.8, 1.0, 0.5, 0.8, seed=n, jitter=0.1)
+    f["vel"] = np.nan
+    sim = mdb.MDSimulation(wl.config_dict(n, Lx, Ly, dt=0.002, T=0.8), frame=f)
+    sim.step_single_NVE(nsteps=3)
+    assert sim.observables().nonfinite == 1
