@@ -635,9 +635,9 @@ def run_ours(args):
             "config": {"workload": desc, "N": N, "parallelism": f"replicas x{ws}",
                        "l2": "flushed between timed steps (256 MiB write outside the events)"},
             "roofline": {"bound": "hbm", "kernel": {
-                             "nh": "k_force<FM_NH> (pair force + NH kick + K)",
-                             "nph": "k_force<FM_NPH> (pair force + virial + kick + barostat)",
-                             "nve": "k_force<FM_NVE> (pair force + kick)"}[mode],
+                             "nh": "force phase, Nose-Hoover (pair force + NH kick + K)",
+                             "nph": "force phase, NPH (pair force + virial + kick + barostat)",
+                             "nve": "force phase, NVE (pair force + kick)"}[mode],
                          "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                          "frac": achieved / hbm_peak, "peak_source": peak_kind,
                          "traffic": traffic,
