@@ -349,7 +349,6 @@ __global__ void __launch_bounds__(kThreads, 4) k_rb_band(Dev D) {
   __syncthreads();
   uint32_t parity = 0;
   if (!rb_band(D, sh_band, band, full, parity, forced)) {
-    atomicExch(&D.bg->bar_err, 1);
     for (int s = 0; s < D.nsys; ++s) D.st[s].err = 6;  // MDB_ERR_CUDA: a copy never arrived
   }
   rebuild_finish(D, forced);
@@ -661,10 +660,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_band(Dev D) {
   double tot[kNP];
   double tmx[3];
   if (!reduce_system<kNS, kNM>(D, P, S, fin.red, fin.mx, tot, tmx)) {
-    if (threadIdx.x == 0 && sh.lost) {
-      atomicExch(&D.bg->bar_err, 1);
-      S->err = 6;  // MDB_ERR_CUDA: a band never arrived
-    }
+    if (threadIdx.x == 0 && sh.lost) S->err = 6;  // MDB_ERR_CUDA: a band never arrived
     return;
   }
   if (threadIdx.x != 0) return;
@@ -672,10 +668,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_band(Dev D) {
   if (!skip) conv = force_tail<FM, PY>(S, tin, Lx, Ly, 0.5 * P.dt, tot, tmx);
   // (a system that was converged at launch is skipped)
   if (FM == FM_FIRE) S->f_drift = (!skip && !conv) ? 1 : 0;
-  if (sh.lost) {
-    atomicExch(&D.bg->bar_err, 1);
-    S->err = 6;
-  }
+  if (sh.lost) S->err = 6;
   S->counter = 0u;
 }
 

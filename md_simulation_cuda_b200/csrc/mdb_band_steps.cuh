@@ -230,10 +230,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_run_band(Dev D, StepsMem M, int
   }
   if (bad) atomicOr(&D.st->nonfinite, 1);
   if (sh.steps.abort) {
-    if (tid == 0) {
-      atomicExch(&D.bg->bar_err, 1);
-      D.st->err = 6;  // MDB_ERR_CUDA: an exchange or a copy gave up
-    }
+    if (tid == 0) atomicExch(&D.st->err, 6);  // MDB_ERR_CUDA: an exchange or a copy gave up
     return;
   }
   __syncthreads();

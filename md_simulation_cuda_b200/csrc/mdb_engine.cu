@@ -566,6 +566,16 @@ int Engine::choose_multi_step() {
   steps_.max = (unsigned long long*)(base + pos + part);
   steps_.seq = (uint32_t*)(base + pos + part + mx);
   steps_.tile = (int32_t*)(steps_.seq + 2);
+  // MDB_EXCHANGE_POLLS=<polls>[@<block>] makes every block, or one, give up its
+  // exchanges after that many polls (to test that the error is reported).
+  steps_.polls = kExchangePolls;
+  steps_.polls_block = -1;
+  const char* polls = getenv("MDB_EXCHANGE_POLLS");
+  if (polls && polls[0]) {
+    steps_.polls = (uint32_t)std::min<unsigned long>(strtoul(polls, nullptr, 10), kExchangePolls);
+    const char* at = strchr(polls, '@');
+    if (at) steps_.polls_block = atoi(at + 1);
+  }
   return MDB_OK;
 }
 

@@ -127,7 +127,6 @@ struct BatchGlobal {
   uint32_t sys_counter;
   int32_t nsys;
   int32_t all_done;
-  int32_t bar_err;     // resident steps kernel: an exchange ran out of polls
   uint32_t rb_count;   // blocks of the list kernel that have arrived
   int32_t forced;      // the pending rebuild was forced (not asked for by a drift)
 };
@@ -221,6 +220,8 @@ struct StepsMem {
   unsigned long long* max;  // [4][4] maxima of the exchanges
   uint32_t* seq;    // [0] exchanges run so far, [1] arrivals (nblocks per exchange)
   int32_t list_rows;  // rows of the shared list (0: lists are read from global memory)
+  uint32_t polls;     // polls of an exchange before a block gives up
+  int32_t polls_block;  // the block they hold for (-1: every block), for tests
 };
 
 }  // namespace mdb

@@ -46,7 +46,7 @@ namespace mdb {
 // groups, with all of a group's gathers in flight at once.
 constexpr int kListGroup = 8;
 // Polls of an exchange before it gives up (each is a round trip to L2).
-constexpr unsigned kExchangePolls = 1u << 22;
+constexpr uint32_t kExchangePolls = 1u << 22;
 
 // What a block keeps in shared memory beside its lists.
 struct StepsShared {
@@ -77,14 +77,19 @@ __device__ __forceinline__ void load_state(const Dev& D, StepsShared& sh) {
     sh.abort = 0;
   }
 }
-// The state back to global memory (one block), but for what other blocks count
-// there themselves.
+// The state back to global memory (one block), but for what other blocks write
+// there themselves: counts, flags and errors. An error is final for the handle
+// and never lowered: a block that gave up an exchange has set it, perhaps one
+// that this block saw through.
 __device__ __forceinline__ void store_state(const Dev& D, const SysState& S) {
   for (int k = threadIdx.x; k < (int)(sizeof(SysState) / 4); k += kThreads) {
     const size_t at = (size_t)k * 4;
-    if (at == offsetof(SysState, nonfinite) || at == offsetof(SysState, nl_overflow)) continue;
+    if (at == offsetof(SysState, nonfinite) || at == offsetof(SysState, nl_overflow) ||
+        at == offsetof(SysState, err))
+      continue;
     ((uint32_t*)D.st)[k] = ((const uint32_t*)&S)[k];
   }
+  if (threadIdx.x == 0 && S.err != 0) atomicCAS(&D.st->err, 0, S.err);
 }
 
 // What the threads of a block bring to an exchange, and thread 0 takes from
@@ -161,11 +166,13 @@ __device__ __forceinline__ void exchange(const StepsMem& M, StepsShared& sh, uin
       // before by the block barrier)
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(M.seq + 1) : "memory");
       const uint32_t target = seq * (uint32_t)nb;
+      const uint32_t most =
+          M.polls_block < 0 || M.polls_block == (int)blockIdx.x ? M.polls : kExchangePolls;
       uint32_t got;
       unsigned polls = 0;
       do {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(M.seq + 1) : "memory");
-      } while ((int32_t)(got - target) < 0 && ++polls < kExchangePolls);
+      } while ((int32_t)(got - target) < 0 && ++polls < most);
       if ((int32_t)(got - target) < 0) sh.abort = 1;
     }
   }
@@ -773,6 +780,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
     ++done;
   }
   if (bad) atomicOr(&D.st->nonfinite, 1);
+  if (sh.abort) {
+    // MDB_ERR_CUDA: an exchange gave up. (The slots stay as they are: others may
+    // have finished a rebuild that this block has not.)
+    if (tid == 0) atomicExch(&D.st->err, 6);
+    return;
+  }
   if (own) {
     D.pos[half + i] = x;
     D.vel[half + i] = v;
@@ -783,13 +796,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_run_steps(Dev D, StepsMem M, in
     const int nn = nc >= 0 ? (nc & (kListInterior - 1)) : 0;
     for (int k = 0; k * L + lane < nn; ++k)
       D.nlist16[(int64_t)(k * L + lane) * D.ntot + i] = col[k * kThreads];
-  }
-  if (sh.abort) {
-    if (tid == 0) {
-      atomicExch(&D.bg->bar_err, 1);
-      D.st->err = 6;  // MDB_ERR_CUDA: an exchange gave up
-    }
-    return;
   }
   __syncthreads();
   // Every block has read D.st and M.seq (it took part in an exchange) unless
