@@ -36,8 +36,12 @@ namespace mdb {
 //  * one row: the cells x0 - 1 .. x1 + 1 of three rows, and for an end cell of
 //    the row the cell across the edge;
 //  * two rows (y1 = y0 + 1): of four rows the cells 0 .. x1 + 1 and
-//    x0 - 1 .. ncx - 1.
-// Rows beyond a walled y axis are empty.
+//    x0 - 1 .. ncx - 1. (Of a periodic side of three rows the fourth is the first
+//    again; a side of fewer has no cell lists.)
+// Rows beyond a walled y axis are empty. A box three or four cells high takes the
+// row pieces too: its rows are long, and as whole rows they left its chunks
+// without lists (16 systems of 9,000 particles in strips of four rows: 55 us a
+// step, 32 with lists).
 struct BandShape {
   int x0, y0, x1, y1, ncx, ncy;
   bool py, full;
@@ -101,6 +105,7 @@ __device__ __forceinline__ bool band_piece(const BandShape& s, int r, int* c0, i
       some = !joined;
     }
   }
+  if (s.py && s.ncy == 3 && r >= 6) some = false;
   if (y < 0 || y >= s.ncy) {
     if (!s.py) some = false;
     y += (y < 0) ? s.ncy : -s.ncy;
@@ -134,8 +139,6 @@ __device__ __forceinline__ void make_band(const Dev& D, const SysParams& P, cons
     if (s.py && s.y0 == 0) rows += cst[s.ncy * s.ncx] - cst[(s.ncy - 1) * s.ncx];
     if (s.py && s.y1 == s.ncy - 1) rows += cst[s.ncx] - cst[0];
     s.full = s.y1 > s.y0 + 1 || rows <= kBandCap;
-    // (three rows or fewer on a side: pieces could meet across the edge)
-    if (s.ncy < 5) s.full = true;
   }
   const int np = band_pieces(s);
   int start = 0, len = 0;

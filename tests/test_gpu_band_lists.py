@@ -1,0 +1,59 @@
+"""Neighbour lists of staged bands (csrc/mdb_band.cuh) in boxes few cells high.
+
+A box three or four cells high has rows longer than a staged band. Its chunks
+take stretches of rows like any other's: every slot keeps its list (the batch
+counts the ones that lost it), and the results are those of the per-phase kernels
+and of stencil scans, bit for bit.
+"""
+import numpy as np
+import pytest
+
+import md_simulation_cuda_b200 as mdb
+from md_simulation_cuda_b200 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+
+def _strip(n, Ly, rho=0.8, **cfg):
+    """A lattice in a box of height Ly (cells are 2.95 high, for FIRE 2.7)."""
+    f, Lx, Ly = wl.lattice_frame(n, rho, n / rho / Ly ** 2, 0.5, 0.8, seed=n, jitter=0.1)
+    return f, wl.config_dict(n, Lx, Ly, dt=0.002, T=0.8, barostat_mass=50.0, k_piston=100.0,
+                             n_cap=n, **cfg)
+
+
+@pytest.mark.parametrize("n,Ly", [(9000, 9.2), (9001, 12.5), (20011, 14.7)])
+@pytest.mark.parametrize("fire", [False, True])
+def test_low_boxes_keep_their_lists(built, n, Ly, fire):
+    f, cfg = _strip(n, Ly)
+    b = mdb.Batch()
+    for _ in range(2):
+        if fire:
+            b.add_fire(cfg, f, 1e-9, 1000, wl.fire_params())
+        else:
+            b.add_md(cfg, f, mdb.JOB_NVT, 40)
+    b.run(0 if fire else -1)
+    for k in range(2):
+        assert b.system_stats(k)[1] == 0  # (rebuilds, slots without a list)
+
+
+def _run(f, cfg, steps, **opt):
+    sim = mdb.MDSimulation(cfg, frame=f, **opt)
+    out = []
+    for step in (lambda: sim.step_single_nose_hoover(nsteps=steps),
+                 lambda: sim.step_single_NPH(1.2, nsteps=steps),
+                 lambda: sim.step_single_NPH_piston(0.8, nsteps=steps),
+                 lambda: sim.step_single_NVE(nsteps=5)):
+        step()
+        sim.sample_collect()
+        o = sim.observables()
+        out.append((sim.get_host_particles().tobytes(), o.Lx, o.Ly, o.xi, o.rebuilds,
+                    sim.cal_total_U()))
+    return out
+
+
+@pytest.mark.parametrize("n,Ly", [(80001, 9.2), (80003, 12.5), (100003, 16.0)])
+def test_low_boxes_in_the_steps_kernel(built, n, Ly):
+    f, cfg = _strip(n, Ly)
+    a = _run(f, cfg, 30)
+    assert a == _run(f, cfg, 30, step_kernel=mdb.STEPS_PER_PHASE)
+    assert a == _run(f, cfg, 30, max_neighbors=-1)
