@@ -301,8 +301,11 @@ __device__ __forceinline__ bool rb_band(const Dev& D, float4* sh_band, Band& ban
       ((int32_t*)(D.bands + q))[threadIdx.x] = ((const int32_t*)&band)[threadIdx.x];
     if (band.total == 0 || !lists) {
       if (act) D.ncount[k] = -1;
-      if (threadIdx.x == 0 && lists)  // the chunk's particles scan their stencils
-        atomicAdd(&S->nl_overflow, (int)min((int64_t)kThreads, P.p0 + P.n - cs));
+      if (threadIdx.x == 0) {
+        const int slots = (int)min((int64_t)kThreads, P.p0 + P.n - cs);
+        if (lists) atomicAdd(&S->nl_overflow, slots);  // they scan their stencils
+        if (forced && band.total == 0) atomicAdd(&D.bg->unbanded, slots);
+      }
       __syncthreads();  // (the band is rewritten for the next chunk)
       continue;
     }

@@ -199,6 +199,81 @@ int Engine::add_system(SystemSpec&& spec) {
   return MDB_OK;
 }
 
+int Engine::alloc(void** p, size_t bytes) {
+  MDB_CUDA(cudaMalloc(p, bytes < 16 ? 16 : bytes));
+  allocs_.push_back(*p);
+  bytes_ += (int64_t)(bytes < 16 ? 16 : bytes);
+  return MDB_OK;
+}
+
+int Engine::alloc_slot_lists() {
+  if (max_nbr_ <= 0) return MDB_OK;
+  if (dev_.nl16)
+    return alloc((void**)&dev_.nlist16, sizeof(*dev_.nlist16) * (size_t)max_nbr_ * ntot_);
+  return alloc((void**)&dev_.nlist, sizeof(*dev_.nlist) * (size_t)max_nbr_ * ntot_);
+}
+
+// The list build is instruction-bound with per-slot costs that vary (list
+// lengths, minimum-image slots): one wave of resident blocks, grid-stride, so
+// that no SM is left with a partial second wave.
+void Engine::set_list_grid() {
+  int nsm = 148, per_sm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device_);
+  const Kernel lk = list_kernel();
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lk.fn, kThreads, lk.smem) !=
+          cudaSuccess ||
+      per_sm <= 0) {
+    (void)cudaGetLastError();
+    nlist_grid_ = rb_grid_;
+  } else {
+    nlist_grid_ = std::max(1, std::min(dev_.nchunks, nsm * per_sm));
+  }
+}
+
+// A band holds 1,408 positions: enough for a chunk of a system whose cells hold up
+// to some 25 particles (a cutoff of 5 at density 0.8), not for the chunks that
+// span two rows of a longer cutoff, and there is none for all-pairs systems. A
+// chunk without one scans its stencil from global memory, which is slow enough
+// that a few hold a force phase up; then the lists of slot offsets and their
+// kernels are the faster ones. (Estimated for a system of its mean density: a chunk
+// that spans two rows takes from four of them its 256 slots and about three cells
+// more. The frame's own count only says where it is far from uniform: a lattice's
+// rows of cells hold two or three of its own rows, and fit or don't until it melts.) 16 systems of 9,000 a step, bands / slot lists, us: cutoff 5
+// 52 / 62, 7 162 / 93, 9 249 / 132, 15 748 / 413; all-pairs strips of 3,000
+// 549 / 321. 262,144 particles: cutoff 5 65 / 83, 5.5 (1% of the
+// chunks) 200 / 107, 7 (7%) 347 / 149.
+int Engine::use_slot_lists() {
+  BatchGlobal g;
+  MDB_CUDA(cudaMemcpyAsync(&g, dev_.bg, sizeof(g), cudaMemcpyDeviceToHost, stream_));
+  MDB_CUDA(wait_host());
+  double mean = 0.0;
+  for (const SysParams& P : hsp_) {
+    const double cols = std::max(1.0, floor(P.Lx0 / P.r_cell));
+    const double rows = std::max(1.0, floor(P.Ly0 / P.r_cell));
+    const double cell = P.n / (cols * rows), row = P.n / rows;
+    if (4.0 * row > kBandCap && 4.0 * (kThreads + 3.0 * cell) > 0.95 * kBandCap)
+      mean += P.n * std::min(1.0, kThreads / row);
+  }
+  if (g.unbanded * (double)kBandUnfitNow <= (double)ntot_ &&
+      mean * kBandUnfitMean <= (double)ntot_)
+    return MDB_OK;
+  const size_t bytes[2] = {sizeof(Band) * (size_t)dev_.nchunks,
+                           sizeof(uint2) * (size_t)((max_nbr_ + 3) / 4) * ntot_};
+  void* const gone[2] = {dev_.bands, dev_.lists};
+  dev_.bands = nullptr;
+  dev_.lists = nullptr;
+  for (int k = 0; k < 2; ++k) {
+    if (!gone[k]) continue;
+    allocs_.erase(std::find(allocs_.begin(), allocs_.end(), gone[k]));
+    bytes_ -= (int64_t)std::max<size_t>(16, bytes[k]);
+    MDB_CUDA(cudaFree(gone[k]));
+  }
+  banded_ = band_steps_ = false;
+  if (int rc = alloc_slot_lists()) return rc;
+  set_list_grid();
+  return rebuild_now(-1);
+}
+
 int Engine::build() {
   if (built_) return set_error(MDB_ERR_STATE, "engine already built");
   if (specs_.empty()) return set_error(MDB_ERR_STATE, "no systems");
@@ -344,12 +419,6 @@ int Engine::build() {
   if (ntot_ >= (int64_t)INT32_MAX || ncells_ >= (int64_t)INT32_MAX)
     return set_error(MDB_ERR_CAPACITY, "batch exceeds 2^31 particles or cells");
 
-  auto alloc = [&](void** p, size_t bytes) -> int {
-    MDB_CUDA(cudaMalloc(p, bytes < 16 ? 16 : bytes));
-    allocs_.push_back(*p);
-    bytes_ += (int64_t)(bytes < 16 ? 16 : bytes);
-    return MDB_OK;
-  };
 #define MDB_ALLOC(ptr, count)                                                 \
   do {                                                                        \
     int rc_ = alloc((void**)&(ptr), sizeof(*(ptr)) * (size_t)(count));       \
@@ -394,7 +463,7 @@ int Engine::build() {
   rc = choose_multi_step();
   if (rc) return rc;
   // Systems that do not run in the resident steps kernel take the staged bands
-  // (one lane per slot).
+  // (one lane per slot), where these fit: see use_slot_lists.
   banded_ = !multi_step_ && !lanes_;
   int32_t *soc = nullptr, *sot = nullptr;
   D.nchunks = ch0;
@@ -407,11 +476,9 @@ int Engine::build() {
   if (banded_) {
     MDB_ALLOC(D.bands, ch0);
     if (max_nbr_ > 0) MDB_ALLOC(D.lists, (int64_t)((max_nbr_ + 3) / 4) * ntot_);
-  } else if (max_nbr_ > 0) {
-    if (D.nl16)
-      MDB_ALLOC(D.nlist16, (int64_t)max_nbr_ * ntot_);
-    else
-      MDB_ALLOC(D.nlist, (int64_t)max_nbr_ * ntot_);
+  } else {
+    rc = alloc_slot_lists();
+    if (rc) return rc;
   }
   MDB_ALLOC(D.ccount, ncells_);
   MDB_ALLOC(D.cstart, ncells_ + 1);
@@ -429,22 +496,7 @@ int Engine::build() {
   rb_grid_ = std::max(1, std::min(ch0, nsm * 8));
   scan_grid_ = std::max(1, std::min(t0, nsm * 4));
   D.pf_rows = kListPrefetchRows;
-  // The list build is instruction-bound with per-slot costs that vary (list
-  // lengths, minimum-image slots): one wave of resident blocks, grid-stride,
-  // so that no SM is left with a partial second wave.
-  {
-    int per_sm = 0;
-    const Kernel lk = list_kernel();
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lk.fn, kThreads, lk.smem) !=
-            cudaSuccess ||
-        per_sm <= 0) {
-      (void)cudaGetLastError();
-      nlist_grid_ = rb_grid_;
-    } else {
-      nlist_grid_ = std::min(ch0, nsm * per_sm);
-      nlist_grid_ = std::max(nlist_grid_, 1);
-    }
-  }
+  set_list_grid();
 
   // block table, per-slot system ids, parameters, state
   std::vector<int32_t> hsob(nblocks_), hsoc(ch0), hsot(t0);
@@ -487,6 +539,10 @@ int Engine::build() {
   }
   rc = rebuild_now(-1);
   if (rc) return rc;
+  if (banded_) {
+    rc = use_slot_lists();
+    if (rc) return rc;
+  }
   int items_max = 1;
   for (int s = 0; s < ns; ++s) items_max = std::max(items_max, (int)hsp_[s].items);
   schedule_.list_prefetch_rows = dev_.pf_rows;

@@ -105,6 +105,14 @@ class Engine {
 
  private:
   int ensure_device();
+  int alloc(void** p, size_t bytes);
+  // Memory of the lists of slot offsets (no lists with max_neighbors < 0).
+  int alloc_slot_lists();
+  // One wave of resident blocks for the list build.
+  void set_list_grid();
+  // Gives the staged bands up after the first rebuild when they do not fit the
+  // systems, and rebuilds with lists of slot offsets.
+  int use_slot_lists();
   // A kernel, its launch shape and dynamic shared memory.
   struct Kernel {
     void* fn;

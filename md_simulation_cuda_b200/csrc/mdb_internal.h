@@ -129,6 +129,8 @@ struct BatchGlobal {
   int32_t all_done;
   uint32_t rb_count;   // blocks of the list kernel that have arrived
   int32_t forced;      // the pending rebuild was forced (not asked for by a drift)
+  int32_t unbanded;    // banded engines: slots in chunks without a band, counted by
+                       // the last forced rebuild
 };
 
 // The NPH driver protocol (run_test_NPH.cpp:137-290) run on the device: its
@@ -165,6 +167,10 @@ constexpr int kBandRanges = 8;
 constexpr int kBandCap = 1408;   // positions of a staged band: two bands and four
                                  // blocks an SM leave L1 some 50 KB
 constexpr int kBandRoom = 4;     // positions after it that may be read (never used)
+// An engine keeps lists of slot offsets instead (Engine::use_slot_lists) when more
+// than one slot in kBandUnfitNow is in a chunk without a band at the first rebuild,
+// or more than one in kBandUnfitMean would be at the systems' mean densities.
+constexpr int kBandUnfitNow = 16, kBandUnfitMean = 256;
 struct Band {
   int32_t start[kBandRanges], len[kBandRanges], off[kBandRanges];
   int32_t total;  // 0: no band

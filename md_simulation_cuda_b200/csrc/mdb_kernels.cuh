@@ -2358,6 +2358,7 @@ __global__ void k_force_rebuild(Dev D, int periodic_y) {
   if (threadIdx.x == 0) {
     D.bg->any_rebuild = 1;
     D.bg->forced = 1;
+    D.bg->unbanded = 0;
   }
 }
 

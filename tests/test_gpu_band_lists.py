@@ -57,3 +57,31 @@ def test_low_boxes_in_the_steps_kernel(built, n, Ly):
     a = _run(f, cfg, 30)
     assert a == _run(f, cfg, 30, step_kernel=mdb.STEPS_PER_PHASE)
     assert a == _run(f, cfg, 30, max_neighbors=-1)
+
+
+@pytest.mark.parametrize("cutoff,nbr", [(7.0, 190), (9.0, 320), (3.0, None)])
+def test_long_cutoffs_keep_their_lists(built, cutoff, nbr):
+    """Cells too full for a band: lists of slot offsets instead of stencil scans."""
+    n = 9000
+    f, Lx, Ly = wl.lattice_frame(n, 0.8, 1.0, 0.5, 0.8, seed=3, jitter=0.1)
+    cfg = wl.config_dict(n, Lx, Ly, dt=0.002, T=0.8, cutoff=cutoff)
+    b = mdb.Batch(max_neighbors=nbr)
+    for _ in range(2):
+        b.add_md(cfg, f, mdb.JOB_NVT, 40)
+    b.run()
+    assert b.system_stats(1)[1] == 0
+    sim = mdb.MDSimulation(cfg, frame=f, max_neighbors=nbr, lanes=mdb.LANES_ONE)
+    sim.step_single_nose_hoover(nsteps=40)
+    sim.sample_collect()
+    for k in range(2):
+        assert np.array_equal(sim.get_host_particles()["pos"], b.frame(k)["pos"])
+
+
+@pytest.mark.parametrize("n,Ly,cutoff", [(80001, 8.0, 2.5), (90001, 300.0, 8.0)])
+def test_large_systems_without_bands(built, n, Ly, cutoff):
+    """All pairs, and a long cutoff: the forms agree bit for bit."""
+    f, cfg = _strip(n, Ly, cutoff=cutoff)
+    steps = 3 if Ly < 8.85 else 20
+    a = _run(f, cfg, steps, max_neighbors=240)
+    assert a == _run(f, cfg, steps, max_neighbors=240, step_kernel=mdb.STEPS_PER_PHASE)
+    assert a == _run(f, cfg, steps, max_neighbors=-1)
