@@ -38,6 +38,10 @@ namespace mdb {
 //  * two rows (y1 = y0 + 1): of four rows the cells 0 .. x1 + 1 and
 //    x0 - 1 .. ncx - 1. (Of a periodic side of three rows the fourth is the first
 //    again; a side of fewer has no cell lists.)
+//  * more rows: its rows whole, as one run, and of the rows before and after them
+//    the cells x0 - 1 .. ncx - 1 and 0, and 0 .. x1 + 1 and ncx - 1. (A lattice's
+//    rows of cells are as unequal as 256 and 384 particles: as whole rows, the
+//    chunks of an eighth of 16,384 did not fit.)
 // Rows beyond a walled y axis are empty. A box three or four cells high takes the
 // row pieces too: its rows are long, and as whole rows they left its chunks
 // without lists (16 systems of 9,000 particles in strips of four rows: 55 us a
@@ -48,6 +52,7 @@ struct BandShape {
 };
 __device__ __forceinline__ int band_pieces(const BandShape& s) {
   if (s.full) return 3;
+  if (s.y1 > s.y0 + 1) return 5;
   return s.y1 == s.y0 ? 6 : 8;
 }
 __device__ __forceinline__ bool band_piece(const BandShape& s, int r, int* c0, int* c1) {
@@ -92,6 +97,22 @@ __device__ __forceinline__ bool band_piece(const BandShape& s, int r, int* c0, i
       a = b = (s.x0 == 0) ? s.ncx - 1 : 0;
       some = (s.x0 == 0 || s.x1 == s.ncx - 1) && !(a >= lo && a <= hi);
     }
+  } else if (s.y1 > s.y0 + 1) {
+    if (r == 2) {
+      *c0 = s.y0 * s.ncx;
+      *c1 = (s.y1 + 1) * s.ncx;
+      return true;
+    }
+    y = r < 2 ? s.y0 - 1 : s.y1 + 1;
+    if (r < 2) {
+      a = r == 0 ? max(s.x0 - 1, 0) : 0;
+      b = r == 0 ? s.ncx - 1 : 0;
+      some = r == 0 || s.x0 > 1;
+    } else {
+      a = r == 3 ? 0 : s.ncx - 1;
+      b = r == 3 ? min(s.x1 + 1, s.ncx - 1) : s.ncx - 1;
+      some = r == 3 || s.x1 < s.ncx - 2;
+    }
   } else {
     y = s.y0 - 1 + r / 2;
     const int left = min(s.x1 + 1, s.ncx - 1), right = max(s.x0 - 1, 0);
@@ -105,7 +126,7 @@ __device__ __forceinline__ bool band_piece(const BandShape& s, int r, int* c0, i
       some = !joined;
     }
   }
-  if (s.py && s.ncy == 3 && r >= 6) some = false;
+  if (s.py && s.ncy == 3 && s.y1 == s.y0 + 1 && r >= 6) some = false;
   if (y < 0 || y >= s.ncy) {
     if (!s.py) some = false;
     y += (y < 0) ? s.ncy : -s.ncy;
@@ -132,13 +153,14 @@ __device__ __forceinline__ void make_band(const Dev& D, const SysParams& P, cons
   s.x1 = l % s.ncx;
   s.y1 = l / s.ncx;
   const int32_t* cst = D.cstart + P.c0;
-  // whole rows when they fit (one run), or when the chunk spans more than two
+  // whole rows when they fit (one run), or when the rows before and after the
+  // chunk's meet
   {
     const int lo = max(s.y0 - 1, 0), hi = min(s.y1 + 1, s.ncy - 1);
     int rows = cst[(hi + 1) * s.ncx] - cst[lo * s.ncx];
     if (s.py && s.y0 == 0) rows += cst[s.ncy * s.ncx] - cst[(s.ncy - 1) * s.ncx];
     if (s.py && s.y1 == s.ncy - 1) rows += cst[s.ncx] - cst[0];
-    s.full = s.y1 > s.y0 + 1 || rows <= kBandCap;
+    s.full = rows <= kBandCap || (s.py && s.y1 > s.y0 + 1 && s.y1 - s.y0 + 3 > s.ncy);
   }
   const int np = band_pieces(s);
   int start = 0, len = 0;

@@ -1,7 +1,9 @@
-"""Neighbour lists of staged bands (csrc/mdb_band.cuh) in boxes few cells high.
+"""Neighbour lists of staged bands (csrc/mdb_band.cuh) where whole rows of cells
+do not fit one, and of the systems that bands do not fit at all.
 
-A box three or four cells high has rows longer than a staged band. Its chunks
-take stretches of rows like any other's: every slot keeps its list (the batch
+A box three or four cells high has rows longer than a staged band, and a
+lattice's rows of cells are so unequal that three of them and their neighbours
+are. Their chunks take stretches of rows: every slot keeps its list (the batch
 counts the ones that lost it), and the results are those of the per-phase kernels
 and of stencil scans, bit for bit.
 """
@@ -34,6 +36,17 @@ def test_low_boxes_keep_their_lists(built, n, Ly, fire):
     b.run(0 if fire else -1)
     for k in range(2):
         assert b.system_stats(k)[1] == 0  # (rebuilds, slots without a list)
+
+
+@pytest.mark.parametrize("n,aspect", [(16384, 1.0), (16385, 1.0), (40000, 1.0), (25600, 0.4)])
+def test_lattices_keep_their_lists(built, n, aspect):
+    f, Lx, Ly = wl.lattice_frame(n, 0.8, aspect, 0.5, 0.8, seed=n, jitter=0.1)
+    b = mdb.Batch()
+    for _ in range(2):
+        b.add_md(wl.config_dict(n, Lx, Ly, dt=0.002, T=0.8), f, mdb.JOB_NVT, 40)
+    b.run(0)
+    for k in range(2):
+        assert b.system_stats(k) == (1, 0)  # one rebuild, no slot without a list
 
 
 def _run(f, cfg, steps, **opt):
