@@ -271,7 +271,7 @@ int Engine::use_slot_lists() {
   banded_ = band_steps_ = false;
   if (int rc = alloc_slot_lists()) return rc;
   set_list_grid();
-  return rebuild_now(-1);
+  return rebuild_now(-1, true);
 }
 
 int Engine::build() {
@@ -676,10 +676,10 @@ int Engine::launch_rebuild_eager() {
   return MDB_OK;
 }
 
-int Engine::rebuild_now(int periodic_y) {
+int Engine::rebuild_now(int periodic_y, bool again) {
   if (!built_) return set_error(MDB_ERR_STATE, "engine not built");
   MDB_CUDA(cudaSetDevice(device_));
-  k_force_rebuild<<<1, kThreads, 0, stream_>>>(dev_, periodic_y);
+  k_force_rebuild<<<1, kThreads, 0, stream_>>>(dev_, periodic_y, again ? 1 : 0);
   MDB_CUDA(cudaGetLastError());
   launches_ += 1;
   count_launches(1);

@@ -54,8 +54,9 @@ class Engine {
   int force(int fm, bool py);
   int reduce_K();
   // Flags every system for a rebuild (periodic_y >= 0 also switches the y
-  // convention) and runs the rebuild pipeline now.
-  int rebuild_now(int periodic_y);
+  // convention) and runs the rebuild pipeline now; again: in place of the one just
+  // run (it does not count as another).
+  int rebuild_now(int periodic_y, bool again = false);
   int set_pext(double p);
 
   int get_state(int s, SysState* out);

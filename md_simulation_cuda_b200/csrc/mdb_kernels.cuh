@@ -2348,10 +2348,12 @@ __global__ void k_observables(Dev D, int s, double t, int piston_active,
   *out = o;
 }
 
-// Rebuild flag for every system (creation, frame import, mode switches).
-__global__ void k_force_rebuild(Dev D, int periodic_y) {
+// Rebuild flag for every system (creation, frame import, mode switches). again: in
+// place of the rebuild just done, which then does not count.
+__global__ void k_force_rebuild(Dev D, int periodic_y, int again) {
   for (int s = threadIdx.x; s < D.nsys; s += blockDim.x) {
     D.st[s].need_rebuild = 1;
+    if (again) D.st[s].rebuilds -= 1;
     if (periodic_y >= 0) D.st[s].periodic_y = periodic_y;
     set_cell_grid(D.sp[s], D.st + s);
   }

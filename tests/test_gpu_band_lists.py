@@ -81,6 +81,8 @@ def test_long_cutoffs_keep_their_lists(built, cutoff, nbr):
     b = mdb.Batch(max_neighbors=nbr)
     for _ in range(2):
         b.add_md(cfg, f, mdb.JOB_NVT, 40)
+    b.run(0)
+    assert b.system_stats(1)[0] == 1  # one rebuild, whichever lists it ended with
     b.run()
     assert b.system_stats(1)[1] == 0
     sim = mdb.MDSimulation(cfg, frame=f, max_neighbors=nbr, lanes=mdb.LANES_ONE)
