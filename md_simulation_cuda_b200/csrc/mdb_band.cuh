@@ -603,8 +603,10 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
             if constexpr (HP) {
               const float4* src = staged ? band + band_place(sh.bands[buf], a) : D.pff + a;
 #pragma unroll 1
-              for (int m = 0; m < e - a; ++m)
+              for (int m = 0; m < e - a; ++m) {
                 pair_one_hp<PY, kEnergy, kVirial, true>(src[m], cd, fx, fy, w, u, an);
+                if (!NC && (m + 1) % kScanPiece == 0) mark_progress(D);
+              }
             } else if (staged) {
               const float4* src = band + band_place(sh.bands[buf], a);
               if (image)
@@ -613,9 +615,11 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
                 pair_run<kEnergy, kVirial, false, kFloor>(src, e - a, c, fs, fc, ws, wc, u, an);
             } else {
 #pragma unroll 1
-              for (int m = a; m < e; ++m)
+              for (int m = a; m < e; ++m) {
                 pair_one<PY, kEnergy, kVirial, true, kFloor>(ld_pos<NC>(D.pff + m), c, fs, fc, ws,
                                                              wc, u, an);
+                if (!NC && (m + 1) % kScanPiece == 0) mark_progress(D);
+              }
             }
           }
         }

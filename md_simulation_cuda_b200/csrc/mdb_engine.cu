@@ -610,7 +610,7 @@ int Engine::choose_multi_step() {
   const size_t pos = multi_step_ ? sizeof(float4) * (size_t)ntot_ : 0;
   const size_t part = sizeof(double) * 2 * kNP * (size_t)nblocks_;
   const size_t mx = sizeof(unsigned long long) * 16;
-  const size_t cnt = sizeof(int32_t) * (size_t)(nblocks_ + 2);
+  const size_t cnt = sizeof(int32_t) * (size_t)(nblocks_ + 3);
   const size_t bytes = pos + part + mx + cnt;
   char* base = nullptr;
   MDB_CUDA(cudaMalloc((void**)&base, bytes));
@@ -621,7 +621,8 @@ int Engine::choose_multi_step() {
   steps_.part = (double*)(base + pos);
   steps_.max = (unsigned long long*)(base + pos + part);
   steps_.seq = (uint32_t*)(base + pos + part + mx);
-  steps_.tile = (int32_t*)(steps_.seq + 2);
+  steps_.tile = (int32_t*)(steps_.seq + 3);
+  dev_.progress = steps_.seq + 2;
   // MDB_EXCHANGE_POLLS=<polls>[@<block>] makes every block, or one, give up its
   // exchanges after that many polls (to test that the error is reported).
   steps_.polls = kExchangePolls;

@@ -216,6 +216,7 @@ struct Dev {
   cudaGraphConditionalHandle cond;
   int32_t use_cond;
   int32_t pf_rows;    // force phase: list rows of the next chunk prefetched per warp
+  uint32_t* progress;  // steps kernel over staged bands: counts pieces of long scans
 };
 
 // Device memory of the resident steps kernel.
@@ -224,9 +225,10 @@ struct StepsMem {
   int32_t* tile;    // particles per block's range of cells; all zero outside a rebuild
   double* part;     // [2][kNP][nblocks] block sums of the exchanges
   unsigned long long* max;  // [4][4] maxima of the exchanges
-  uint32_t* seq;    // [0] exchanges run so far, [1] arrivals (nblocks per exchange)
+  uint32_t* seq;    // [0] exchanges run so far, [1] arrivals (nblocks per exchange),
+                    // [2] pieces of long scans (Dev::progress)
   int32_t list_rows;  // rows of the shared list (0: lists are read from global memory)
-  uint32_t polls;     // polls of an exchange before a block gives up
+  uint32_t polls;     // polls of an exchange without progress before a block gives up
   int32_t polls_block;  // the block they hold for (-1: every block), for tests
 };
 

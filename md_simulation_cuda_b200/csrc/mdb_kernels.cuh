@@ -598,6 +598,14 @@ __device__ __forceinline__ void pair_list(const float4* __restrict__ pff,
   }
 }
 
+// Scans without lists are marked piece by piece where blocks wait for one another:
+// a wait that runs out of polls looks whether the blocks at work get on. (A pass
+// over all pairs of two million particles takes seconds.)
+constexpr int kScanPiece = 1024;
+__device__ __forceinline__ void mark_progress(const Dev& D) {
+  if (D.progress && (int)(threadIdx.x & 31) == __ffs(__activemask()) - 1) atomicAdd(D.progress, 1u);
+}
+
 // Candidates j in [j0, j1) (cell stencil rows or the whole system).
 template <bool PY, bool ENERGY, bool VIRIAL, bool FLOOR, bool NC, int LANES = 1>
 __device__ __forceinline__ void pair_range(const float4* __restrict__ pff, int j0, int j1,

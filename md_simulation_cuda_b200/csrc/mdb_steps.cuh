@@ -45,7 +45,9 @@ namespace mdb {
 // offset, which the pair term skips (r^2 = 0): the pair loop then takes whole
 // groups, with all of a group's gathers in flight at once.
 constexpr int kListGroup = 8;
-// Polls of an exchange before it gives up (each is a round trip to L2).
+// Polls of an exchange (each is a round trip to L2, so some 1.5 s) before it looks
+// whether the blocks it waits for have got on with a long scan (mark_progress); it
+// gives up when nothing has moved since it last looked.
 constexpr uint32_t kExchangePolls = 1u << 22;
 
 // What a block keeps in shared memory beside its lists.
@@ -115,8 +117,8 @@ __device__ __forceinline__ double warps_sum(const double (&w)[kThreads / 32]) {
 // own flag instead (all to all) cost 8,700 cycles at 148 blocks against 2,600.
 // The partials alternate between two buffers and the maxima between four (the
 // one used two exchanges ago is cleared here), so a block may be one exchange
-// ahead of another. A wait that runs out of polls sets sh.abort, after which
-// the kernel ends with the system's error flag set; it does not wait again.
+// ahead of another. A wait that gives up sets sh.abort, after which the kernel ends
+// with the system's error flag set; it does not wait again.
 template <int NS, int N32, int N64>
 __device__ __forceinline__ void exchange(const StepsMem& M, StepsShared& sh, uint32_t& seq,
                                          const Totals& in, Totals& out) {
@@ -168,12 +170,21 @@ __device__ __forceinline__ void exchange(const StepsMem& M, StepsShared& sh, uin
       const uint32_t target = seq * (uint32_t)nb;
       const uint32_t most =
           M.polls_block < 0 || M.polls_block == (int)blockIdx.x ? M.polls : kExchangePolls;
-      uint32_t got;
-      unsigned polls = 0;
-      do {
+      uint32_t got, polls = 0, seen = 0;
+      bool looked = false;
+      for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(got) : "l"(M.seq + 1) : "memory");
-      } while ((int32_t)(got - target) < 0 && ++polls < most);
-      if ((int32_t)(got - target) < 0) sh.abort = 1;
+        if ((int32_t)(got - target) >= 0) break;
+        if (++polls < most) continue;
+        const uint32_t now = *(volatile uint32_t*)(M.seq + 2);
+        if (looked && now == seen) {
+          sh.abort = 1;
+          break;
+        }
+        looked = true;
+        seen = now;
+        polls = 0;
+      }
     }
   }
   // (a block barrier, not only a warp's: it also brings warp 0 together after

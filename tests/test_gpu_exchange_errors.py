@@ -1,10 +1,10 @@
-"""Exchanges of the resident steps kernels that give up.
+"""Exchanges of the resident steps kernels that give up, and ones that must not.
 
 MDB_EXCHANGE_POLLS=1@1 lets block 1 look once whether the others have arrived:
 sooner or later it gives up an exchange that the others see through. That was the
 launch's last exchange for a one-step call, whose other blocks then finish as
 usual. The call has to end with an error all the same, and the error is final for
-the handle.
+the handle. Blocks that are only slow are waited for.
 """
 import pytest
 
@@ -34,3 +34,22 @@ def test_one_block_gives_up_the_last_exchange(built, monkeypatch, n):
             sim.synchronize()
     with pytest.raises(mdb.MDBError):
         sim.observables()
+
+
+def test_slow_blocks_are_waited_for(built, monkeypatch):
+    """A strip that its barostat squeezes below three cells turns into an all-pairs
+    system in the middle of a run, with force phases (some 15 ms) many times longer
+    than two waits of 1,024 polls."""
+    n, Ly = 80001, 8.87
+    f, Lx, Ly = wl.lattice_frame(n, 0.8, n / 0.8 / Ly ** 2, 0.5, 0.8, seed=n, jitter=0.1)
+    cfg = wl.config_dict(n, Lx, Ly, dt=0.002, T=0.8, barostat_mass=5e-5, n_cap=n)
+    out = []
+    for kernel in (mdb.STEPS_PER_PHASE, mdb.STEPS_AUTO):
+        monkeypatch.setenv("MDB_EXCHANGE_POLLS", "1024")
+        sim = mdb.MDSimulation(cfg, frame=f, step_kernel=kernel)
+        sim.step_single_NPH(50.0, nsteps=40)
+        sim.sample_collect()
+        o = sim.observables()
+        assert o.Ly < 8.85 and o.rebuilds > 1
+        out.append((sim.get_host_particles().tobytes(), o.Lx, o.Ly, o.steps, o.rebuilds))
+    assert out[0] == out[1]
