@@ -108,7 +108,7 @@ struct SysState {
   int32_t f_conv_step;
   int32_t f_drift;  // the force phase of this iteration ran and did not converge
   int32_t f_fp64;   // FP64 pair terms for this system (FIRE and its observations)
-  int32_t f_pad;
+  int32_t lost;     // a position was not finite at the last rebuild
   // step (MD) or iteration (FIRE) counter at the last rebuild that the drift
   // asked for; a forced rebuild resets it to kNoRebuildYet
   int64_t rb_last;

@@ -1305,6 +1305,7 @@ __device__ __forceinline__ void set_cell_grid(const SysParams& P, SysState* S) {
   S->Lx_b = Lx;
   S->Ly_b = Ly;
   S->nl_overflow = 0;
+  S->lost = 0;
 }
 
 // Scalars of one drift that its tail writes back to the system.
@@ -1723,8 +1724,10 @@ __device__ __forceinline__ void rb_bin(const Dev& D) {
       const SysState* S = D.st + R.s[k];
       const SysParams& P = D.sp[R.s[k]];
       cell[k] = -1;
-      if (R.i[k] >= 0)
+      if (R.i[k] >= 0) {
         cell[k] = bin_axis(p[k].y * S->inv_wy, S->ncy) * S->ncx + bin_axis(p[k].x * S->inv_wx, S->ncx);
+        if (!isfinite(p[k].x) || !isfinite(p[k].y)) D.st[R.s[k]].lost = 1;
+      }
       // one add for the slots of a warp in one cell
       mates[k] = __match_any_sync(0xffffffffu, cell[k]);
       first[k] = __ffs(mates[k]) - 1;
@@ -1843,6 +1846,21 @@ __global__ void __launch_bounds__(kThreads) k_rb_scatter(Dev D) {
   if (rebuild_requested(D)) rb_scatter(D);
 }
 
+// Particles of lower source slots than src among the entries [ca, ce) of perm. For
+// the cells of a system whose cutoff spans most of its box, which cost less here
+// than in the force phase that follows.
+constexpr int kLargeCell = 1 << 16;
+__device__ __noinline__ int large_cell_rank(const Dev& D, int ca, int ce, int src) {
+  int before = 0;
+  for (int piece = ca; piece < ce; piece += kLargeCell) {
+    const int end = min(ce, piece + kLargeCell);
+#pragma unroll 4
+    for (int e = piece; e < end; ++e) before += D.perm[e] < src ? 1 : 0;
+    mark_progress(D);
+  }
+  return before;
+}
+
 // Each particle to its place: after the particles of lower source slots in its
 // cell (the stable sort by cell), with the float-float copy, the cell and the
 // rebuild position. A thread takes an entry of perm, so a warp's reads may
@@ -1864,14 +1882,14 @@ __device__ __forceinline__ void rb_permute(const Dev& D, bool forced) {
       ce[k] = R.i[k] >= 0 ? cs[1] : 0;
       before[k] = 0;
     }
-    // (Non-finite positions all bin to cell 0. A cell of more than kSortedCell
-    // particles, which no finite system comes near, keeps the order of arrival:
-    // ordering it would take the square of its size.)
-    constexpr int kSortedCell = 1 << 16;
+    // (Positions that are not finite bin to the cells of a few corners. There a
+    // system that has lost its numbers keeps the order of arrival: ordering such a
+    // cell takes the square of its size, and nothing else of its steps does.)
 #pragma unroll
     for (int k = 0; k < K; ++k)
-      if (ce[k] - ca[k] > kSortedCell) {
-        before[k] = (int)R.i[k] - ca[k];
+      if (ce[k] - ca[k] > kLargeCell) {
+        before[k] = D.st[R.s[k]].lost ? (int)R.i[k] - ca[k]
+                                      : large_cell_rank(D, ca[k], ce[k], src[k]);
       } else for (int e = ca[k]; e < ce[k]; e += 4) {
         int other[4];
 #pragma unroll
