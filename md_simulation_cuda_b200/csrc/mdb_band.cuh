@@ -581,8 +581,9 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
         } else {
           // no list: the stencil's runs from the band (or, without one, from
           // global memory), or the whole system
-          // (A slot whose position is not a number has no pairs: every test fails.)
-          const bool some = qi.x == qi.x && qi.y == qi.y;
+          // (A slot whose position is not finite has no pairs: every test fails. The
+          // walled y axis is not wrapped, so it can be infinite.)
+          const bool some = isfinite(qi.x) && isfinite(qi.y);
           const int cell = S.allpairs ? 0 : ld_idx<NC>(D.cell_of + i);
           const int cx = cell % S.ncx, cy = cell / S.ncx;
           // the minimum image for the warps that hold a slot within two cells of
