@@ -114,7 +114,11 @@ typedef struct mdb_options {
   int32_t stream_priority; /* 0 (default): the handle's stream has normal
                               priority; k > 0: k levels above it (clamped to
                               the device's range), so its kernels' blocks
-                              are scheduled before those of lower streams   */
+                              are scheduled before those of lower streams.
+                              A kernel that runs many steps (step_kernel)
+                              holds its places until it ends, about a
+                              millisecond: a handle that must let others in
+                              sooner takes MDB_STEPS_PER_PHASE              */
   int32_t fire_precision; /* FIRE pair arithmetic: MDB_FIRE_AUTO (default)
                              runs the reference's FP32 pair terms until a
                              system's max |a| falls below 1e-3, then FP64
@@ -137,8 +141,13 @@ typedef struct mdb_options {
                              the resident steps kernels, for calls of any
                              length: cooperative launches that run many
                              steps (or FIRE iterations) each, rebuilds
-                             included; up to ~75k particles with the state
-                             in registers, above that over staged bands;
+                             included, for about a millisecond; up to ~75k
+                             particles with the state in registers, above
+                             that over staged bands (the whole device, so
+                             several such handles take turns: four threads
+                             with 262,144 particles each 34 us a step and
+                             system, 23 with one kernel per phase, which
+                             overlap; one alone 34 against 44);
                              MDB_STEPS_PER_PHASE: one kernel per phase.
                              All give the same result bits.               */
   int32_t lanes;          /* lanes per particle in the force phase of MD

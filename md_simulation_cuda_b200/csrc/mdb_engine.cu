@@ -636,14 +636,21 @@ int Engine::choose_multi_step() {
   return MDB_OK;
 }
 
-// n steps (FIRE: iterations) in cooperative launches. A launch holds the device
-// until it ends, so it is kept short enough for the kernels of other streams to
-// run in between.
+// n steps (FIRE: iterations) in cooperative launches. A launch holds its blocks'
+// places until it ends, over staged bands the whole device, whatever the priority of
+// the streams that wait. So its steps are those of about a millisecond, by a rule on
+// the size (measured us a step: 5.0 at 900 particles, 14.8 at 60,013; 33 at 262,144,
+// 97 at 1,048,576; launches of 0.3 ms cost a step 2% there, of 1 ms less than 0.5%).
+// 200 steps of 4,096 particles at a higher priority, 1.4 ms alone, took 7.6 ms beside
+// launches of 64 steps of 1,048,576 particles, 3.4 beside these, 1.7 beside one kernel
+// per phase (MDB_STEPS_PER_PHASE).
 int Engine::run_resident(int dm, int64_t n) {
   Dev d = dev_;
   d.use_cond = 0;
   StepsMem m = steps_;
-  const int64_t most = multi_step_ ? 256 : 64;
+  const double us = multi_step_ ? 5.0 + ntot_ / 6000.0 : 8.0 + ntot_ / 11500.0;
+  const int64_t most =
+      std::max<int64_t>(1, std::min<int64_t>(multi_step_ ? 256 : 64, (int64_t)(1000.0 / us)));
   for (int64_t left = n; left > 0;) {
     int64_t k = std::min(left, most);
     void* args[] = {&d, &m, &k};
@@ -917,8 +924,12 @@ int Engine::get_states(std::vector<SysState>& out) {
 
 int Engine::put_state(int s, const SysState& st) {
   MDB_CUDA(cudaSetDevice(device_));
-  // (the call returns once the pageable source has been taken over)
-  MDB_CUDA(cudaMemcpyAsync(dev_.st + s, &st, sizeof(SysState), cudaMemcpyHostToDevice, stream_));
+  // (as a kernel argument, which the launch copies: the caller may let go of `st`
+  // at once, and nothing waits)
+  k_put_state<<<1, 1, 0, stream_>>>(dev_, s, st);
+  MDB_CUDA(cudaGetLastError());
+  launches_ += 1;
+  count_launches(1);
   return MDB_OK;
 }
 

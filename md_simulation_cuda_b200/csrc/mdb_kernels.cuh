@@ -2390,6 +2390,10 @@ __global__ void k_force_rebuild(Dev D, int periodic_y, int again) {
   }
 }
 
+__global__ void k_put_state(Dev D, int s, SysState S) {
+  D.st[s] = S;
+}
+
 __global__ void k_set_pext(Dev D, double p) {
   for (int s = threadIdx.x; s < D.nsys; s += blockDim.x) D.st[s].p_ext = p;
 }
