@@ -125,6 +125,12 @@ double next_pow2(double x) {
 
 }  // namespace
 
+int64_t resident_limit(int device) {
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  return (int64_t)nsm * 2 * kThreads;  // two blocks an SM, one slot a thread
+}
+
 Engine::Engine(const mdb_options_t& opt) {
   device_ = opt.device;
   skin_ = opt.skin > 0.0 ? opt.skin : 0.0;  // 0: chosen at build from the systems' kinds

@@ -199,6 +199,9 @@ class Engine {
   long long last_rebuilds_ = 0;
 };
 
+// Particles up to which a single system runs in the resident steps kernel.
+int64_t resident_limit(int device);
+
 int reference_initial_frame(const mdb_config_t& cfg, std::vector<mdb_particle_t>& out);
 
 // For the trajectory writer: queue the export of a simulation's frame into
