@@ -1195,9 +1195,13 @@ int Engine::tune() {
   const int nsm = prop.multiProcessorCount;
   int kinds = 0;
   for (const SystemSpec& sp : specs_) kinds |= 1 << sp.kind;
+  // (the kernels that the schedule was timed on, and a number that goes up with them:
+  // a line of other kernels does not fit)
+  const char* form = multi_step_ ? "resident" : band_steps_ ? "bandsteps" : banded_ ? "bands"
+                     : lanes_ ? "lanes" : "lists";
   char keyb[512];
-  snprintf(keyb, sizeof(keyb), "%s|sm%d|sys%d|n%d|cells%d|nbr%d|nl16_%d|skin%.3f|kinds%d",
-           prop.name, nsm, bucket((int64_t)specs_.size()), bucket(ntot_), bucket(ncells_),
+  snprintf(keyb, sizeof(keyb), "2|%s|%s|sm%d|sys%d|n%d|cells%d|nbr%d|nl16_%d|skin%.3f|kinds%d",
+           form, prop.name, nsm, bucket((int64_t)specs_.size()), bucket(ntot_), bucket(ncells_),
            max_nbr_, dev_.nl16, skin_, kinds);
   const std::string key(keyb);
   int pf = dev_.pf_rows, nlg = nlist_grid_, rbg = rb_grid_;
