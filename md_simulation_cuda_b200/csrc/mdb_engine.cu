@@ -1210,6 +1210,9 @@ int Engine::tune() {
     nlist_grid_ = std::max(1, nlg);
     rb_grid_ = std::max(1, rbg);
     schedule_.from_cache = 1;
+  } else if (multi_step_) {
+    // (the resident steps kernel reads none of these: the built-in schedule stands)
+    cache_store(key, dev_.pf_rows, nlist_grid_, rb_grid_);
   } else {
     // force phase: list prefetch depth, timed on the workload's force kernel
     // with the velocities (kicked by it) and the scalar state put back after
@@ -1247,12 +1250,15 @@ int Engine::tune() {
     MDB_CUDA(cudaMemcpyAsync(dev_.st, snap.data(), sizeof(SysState) * snap.size(),
                              cudaMemcpyHostToDevice, stream_));
     MDB_CUDA(wait_host());
-    // rebuild: list-build grid, then the grid of the other rebuild kernels
+    // rebuild: list-build grid, then the grid of the other rebuild kernels (the
+    // steps kernel over staged bands rebuilds on its own blocks)
     const int one_wave = nlist_grid_;
     const int cap = std::max(1, dev_.nchunks);
     best = 1e30;
     int best_nlg = one_wave;
+    const bool grids = !band_steps_;
     for (int cand : {one_wave, std::min(cap, 2 * one_wave), std::max(1, one_wave / 2)}) {
+      if (!grids) break;
       nlist_grid_ = cand;
       double ms = 0.0;
       const int rc = time_rebuild(2, &ms);
@@ -1266,6 +1272,7 @@ int Engine::tune() {
     best = 1e30;
     int best_rbg = rb_grid_;
     for (int cand : {rb_grid_, std::min(cap, nsm * 16), std::min(cap, nsm * 4)}) {
+      if (!grids) break;
       rb_grid_ = std::max(1, cand);
       double ms = 0.0;
       const int rc = time_rebuild(2, &ms);

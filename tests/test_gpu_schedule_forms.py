@@ -21,3 +21,18 @@ def test_schedules_of_other_kernels_do_not_match(built, tmp_path, monkeypatch):
               _sim(80000, autotune=True, step_kernel=mdb.STEPS_PER_PHASE).schedule()["from_cache"],
               _sim(70000, autotune=True).schedule()["from_cache"]]
     assert cached == [0, 0, 0, 1]
+
+
+@pytest.mark.parametrize("n,extra", [(900, 0), (20000, 0), (100000, 16)])
+def test_only_what_steps_read_is_timed(built, tmp_path, monkeypatch, n, extra):
+    """Launches at creation beyond those of an untuned handle: none for the resident
+    steps kernel, four candidates of the prefetch depth (one launch and three) over
+    staged bands."""
+    monkeypatch.setenv("MDB_SCHEDULE_CACHE", str(tmp_path / "schedule.txt"))
+    count = []
+    for tune in (False, True):
+        before = mdb.kernel_launches()
+        sim = _sim(n, autotune=tune)
+        count.append(mdb.kernel_launches() - before)
+        assert sim.schedule()["tuned"] == int(tune)
+    assert count[1] - count[0] == extra
