@@ -1220,17 +1220,14 @@ int Engine::tune() {
     const int fm = all_fire ? FM_FIRE : FM_NH;
     std::vector<SysState> snap;
     if (int rc = get_states(snap)) return rc;
-    // (both halves of each array: SysState::buf names the one in use)
-    const size_t bytes = sizeof(double2) * 2 * (size_t)ntot_;
-    double2* keep = nullptr;
-    MDB_CUDA(cudaMalloc((void**)&keep, 2 * bytes));
-    struct Free {
-      void* p;
-      ~Free() { cudaFree(p); }
-    } free_keep{keep};
-    MDB_CUDA(cudaMemcpyAsync(keep, dev_.vel, bytes, cudaMemcpyDeviceToDevice, stream_));
-    MDB_CUDA(cudaMemcpyAsync(keep + 2 * ntot_, dev_.acc, bytes, cudaMemcpyDeviceToDevice,
-                             stream_));
+    // (kept in the half of each array that is not in use; the rebuilds so far were of
+    // all systems, so it is the same half for every one)
+    const size_t bytes = sizeof(double2) * (size_t)ntot_;
+    const int64_t used = snap[0].buf ? ntot_ : 0, idle = ntot_ - used;
+    for (const SysState& S : snap)
+      if (S.buf != snap[0].buf) return set_error(MDB_ERR_STATE, "systems in unlike halves");
+    for (double2* p : {dev_.vel, dev_.acc})
+      MDB_CUDA(cudaMemcpyAsync(p + idle, p + used, bytes, cudaMemcpyDeviceToDevice, stream_));
     double best = 1e30;
     int best_pf = dev_.pf_rows;
     for (int cand : {28, 16, 8, 0}) {
@@ -1244,9 +1241,8 @@ int Engine::tune() {
       }
     }
     dev_.pf_rows = best_pf;
-    MDB_CUDA(cudaMemcpyAsync(dev_.vel, keep, bytes, cudaMemcpyDeviceToDevice, stream_));
-    MDB_CUDA(cudaMemcpyAsync(dev_.acc, keep + 2 * ntot_, bytes, cudaMemcpyDeviceToDevice,
-                             stream_));
+    for (double2* p : {dev_.vel, dev_.acc})
+      MDB_CUDA(cudaMemcpyAsync(p + used, p + idle, bytes, cudaMemcpyDeviceToDevice, stream_));
     MDB_CUDA(cudaMemcpyAsync(dev_.st, snap.data(), sizeof(SysState) * snap.size(),
                              cudaMemcpyHostToDevice, stream_));
     MDB_CUDA(wait_host());
