@@ -532,7 +532,9 @@ def run_ours(args):
     t_max = max_over_ranks(t_ms / 1e3, dist, dev)
     value = N * ws * args.steps / t_max
 
-    # ---- the dominant kernel: per-phase CUDA events on the launching stream --
+    # ---- what a step consists of: the per-phase kernels, launched one by one --
+    # (the timed steps above are one launch each of a kernel that runs the phases
+    # itself; its roofline is the timed step's)
     nph = 20
     ms = sim.phase_times(nph, nose_hoover=(mode == "nh"), nph=(mode == "nph"))
     t_force = ms[2] / nph / 1e3
@@ -540,12 +542,13 @@ def run_ours(args):
     hbm_peak, peak_kind = _peaks()
     force_bytes = 65.0 * N   # read pos(ff) 16 + type 1 + vel 16; write acc 16 + vel 16
     step_bytes = 97.0 * N    # per particle-step, whole step
-    prof = os.path.join(ROOT, "profiles", "force_kernel_traffic.json")
-    traffic = None
-    if os.path.exists(prof):
-        pj = json.load(open(prof))
-        traffic = pj.get("dram_bytes_per_particle", None)
-        traffic = traffic * N if traffic else None
+
+    def dram_bytes(name):  # of a launch at this N, from the profile of the nvt_slab one
+        prof = os.path.join(ROOT, "profiles", name)
+        if args.workload != "nvt_slab" or not os.path.exists(prof):
+            return None
+        return json.load(open(prof))["dram_bytes_per_particle"] * N
+
     from oracle import pyoracle as po
 
     p_ord = None
@@ -625,7 +628,10 @@ def run_ours(args):
             reference_gpu["ours_e2e_over_reference"] = e2e["value"] / reference_gpu["value"]
 
     if rank == 0:
-        achieved = force_bytes / t_force / 1e9
+        t_step = t_max / args.steps
+        achieved = step_bytes / t_step / 1e9
+        flops = 24.0 * p_ord * N if p_ord else None
+        kernel = "k_run_steps" if schedule.get("multi_step") else "k_run_band"
         out = {
             "metric": "particle-steps/s", "value": value, "unit": "particle-steps/s",
             "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
@@ -634,22 +640,27 @@ def run_ours(args):
             "dtype": "fp32-pair/fp64-state", "data": "synthetic (seeded jittered lattice)",
             "config": {"workload": desc, "N": N, "parallelism": f"replicas x{ws}",
                        "l2": "flushed between timed steps (256 MiB write outside the events)"},
-            "roofline": {"bound": "hbm", "kernel": {
-                             "nh": "force phase, Nose-Hoover (pair force + NH kick + K)",
-                             "nph": "force phase, NPH (pair force + virial + kick + barostat)",
-                             "nve": "force phase, NVE (pair force + kick)"}[mode],
+            # the kernel of the timed region (one launch a step: drift, a rebuild when it
+            # is due, force), and its phases as kernels of their own
+            "roofline": {"bound": "hbm", "kernel": kernel + {
+                             "nh": ", one Nose-Hoover step", "nph": ", one NPH step",
+                             "nve": ", one NVE step"}[mode],
                          "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                          "frac": achieved / hbm_peak, "peak_source": peak_kind,
-                         "traffic": traffic,
-                         "algorithmic_bytes_per_particle": 65,
-                         "force_ms": t_force * 1e3, "drift_ms": t_drift * 1e3,
-                         "step_GBps_97B": step_bytes * value / ws / N / 1e9 if N else None,
-                         "fp32": {"achieved_tflops": (24.0 * p_ord * N / t_force / 1e12)
-                                  if p_ord else None,
+                         "traffic": dram_bytes("step_kernel_traffic.json"),
+                         "algorithmic_bytes_per_particle": 97,
+                         "fp32": {"achieved_tflops": flops / t_step / 1e12 if flops else None,
                                   "peak_tflops": FP32_NOMINAL_TFLOPS, "peak_source": "nominal",
-                                  "frac": (24.0 * p_ord * N / t_force / 1e12 / FP32_NOMINAL_TFLOPS)
-                                  if p_ord else None,
+                                  "frac": (flops / t_step / 1e12 / FP32_NOMINAL_TFLOPS)
+                                  if flops else None,
                                   "pairs_per_particle": p_ord},
+                         "phases": {"how": "the per-phase kernels, launched one by one "
+                                           "(phase_times); the timed steps do not launch them",
+                                    "force_ms": t_force * 1e3, "drift_ms": t_drift * 1e3,
+                                    "force_GBps_65B": force_bytes / t_force / 1e9,
+                                    "force_traffic": dram_bytes("force_kernel_traffic.json"),
+                                    "force_fp32_tflops": flops / t_force / 1e12
+                                    if flops else None},
                          # whole step: per-GPU particle-steps/s over the step's bound,
                          # min(HBM peak / 97 B, FP32 peak / (24 flops x P_ord))
                          "step": step_roofline(value / ws, hbm_peak, p_ord),
