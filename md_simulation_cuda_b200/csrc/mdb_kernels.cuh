@@ -399,7 +399,6 @@ __device__ __forceinline__ void copy_bulk(T* dst, const T* src, int n, uint64_t*
 struct PairCtx {
   float2 ih, il;        // slot i's float-float position (hi, lo), x and y lanes
   float2 nLh, nLl, invL;  // -L_hi, -L_lo, 1/L_hi per axis (invL.y = 0: walled y)
-  uint32_t ts;  // class whose pairs with i use the "same" parameters
   uint32_t tsz;  // pair loop: bit 0 = slot i is class 1 (B)
   uint32_t rc2s_m1, rc2ab_m1;  // pair loop: bits of rc^2, minus 1
   float rc2s, rc2ab, sig2s, sig2ab, e24s, e24ab, e4s, e4ab;
@@ -656,7 +655,6 @@ __device__ __forceinline__ void set_pair_box(PairCtx& c, const float4 qi, double
 // Pair parameters of class tci for the force loops.
 template <bool FLOOR>
 __device__ __forceinline__ void set_pair_class(PairCtx& c, const SysParams& P, int tci) {
-  c.ts = (tci == 2) ? 99u : (uint32_t)tci;
   c.tsz = (tci == 1) ? 1u : 0u;
   const int sc = (tci == 2) ? 2 : tci;
   c.rc2s = P.frc2[sc];
