@@ -100,3 +100,20 @@ def test_large_systems_without_bands(built, n, Ly, cutoff):
     a = _run(f, cfg, steps, max_neighbors=240)
     assert a == _run(f, cfg, steps, max_neighbors=240, step_kernel=mdb.STEPS_PER_PHASE)
     assert a == _run(f, cfg, steps, max_neighbors=-1)
+
+
+def test_fire_with_a_long_cutoff(built):
+    """FIRE on lists of slot offsets: a batch against quenches by themselves."""
+    res = []
+    for n in (3000, 3333):
+        f, Lx, Ly = wl.lattice_frame(n, 0.8, 1.0, 0.5, 0.8, seed=n, jitter=0.2)
+        res.append((f, wl.config_dict(n, Lx, Ly, dt=0.001, T=0.0, cutoff=7.0, n_cap=n)))
+    b = mdb.Batch(max_neighbors=190)
+    for f, cfg in res:
+        b.add_fire(cfg, f, 1e-5, 200, wl.fire_params())
+    b.run()
+    for k, (f, cfg) in enumerate(res):
+        a = mdb.EnergyMinimizer(cfg).minimize_frame(f, 1e-5, 200, wl.fire_params())
+        r = b.fire_result(k)
+        assert a.steps == r.steps and a.max_force == r.max_force
+        assert np.array_equal(a.frame["pos"], r.frame["pos"])
