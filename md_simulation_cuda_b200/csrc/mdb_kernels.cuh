@@ -2162,6 +2162,7 @@ __global__ void __launch_bounds__(kThreads) k_count_profile(Dev D, int s, int nb
 // add per pair and component 131,072 particles put 5 million adds on 600
 // addresses (200 bins: 410 -> 120 us a call, the copy to the host included). The sums are integers, so any
 // order gives the same result.
+constexpr int kMergedBins = 6;
 template <bool PY>
 __global__ void __launch_bounds__(kThreads) k_pressure_profile(Dev D, int s, int nb, int win,
                                                                unsigned long long* ptens) {
@@ -2276,8 +2277,24 @@ __global__ void __launch_bounds__(kThreads) k_pressure_profile(Dev D, int s, int
         }
       }
     }
-    // the warp's windows, one own bin after the other
+    // the warp's windows, one own bin after the other; with fine bins nearly every
+    // slot has its own, and each thread adds its window by itself (20,000 bins, a call:
+    // 1,048,576 particles 985 -> 605 us, 4,096 345 -> 250; merged from the start it was
+    // slower there than an add per pair, 709 and 270)
     unsigned todo = __ballot_sync(0xffffffffu, bk >= 0);
+    const unsigned mates = __match_any_sync(0xffffffffu, bk);
+    const int bins = __popc(__ballot_sync(0xffffffffu, bk >= 0 && lane == __ffs(mates) - 1));
+    if (bins > kMergedBins) {
+      for (int e = 0; bk >= 0 && e < 3 * win; ++e) {
+        const unsigned long long t = mine[e * kThreads];
+        if (t == 0ull) continue;
+        int at = bk + e % win - mid;
+        at += at < 0 ? nb : 0;
+        at -= at >= nb ? nb : 0;
+        atomicAdd(ptens + (e / win) * nb + at, t);
+      }
+      todo = 0u;
+    }
     while (todo != 0u) {
       const int bin = __shfl_sync(0xffffffffu, bk, __ffs(todo) - 1);
       const bool part = bk == bin;
