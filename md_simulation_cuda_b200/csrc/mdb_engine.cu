@@ -629,8 +629,8 @@ int Engine::choose_multi_step() {
   steps_.seq = (uint32_t*)(base + pos + part + mx);
   steps_.tile = (int32_t*)(steps_.seq + 3);
   dev_.progress = steps_.seq + 2;
-  // MDB_EXCHANGE_POLLS=<polls>[@<block>] makes every block, or one, give up its
-  // exchanges after that many polls (to test that the error is reported).
+  // MDB_EXCHANGE_POLLS=<polls>[@<block>] makes every block, or one, look after that
+  // many polls whether others get on, for tests.
   steps_.polls = kExchangePolls;
   steps_.polls_block = -1;
   const char* polls = getenv("MDB_EXCHANGE_POLLS");
