@@ -130,7 +130,8 @@ typedef struct mdb_options {
   int32_t autotune;       /* 1: at build, time the engine's schedule
                              candidates on the device (list prefetch depth
                              of the force phase, list-build grid, rebuild
-                             grid) and keep the fastest, cached per device
+                             grid; what the handle's steps do not read is
+                             not timed) and keep the fastest, cached per device
                              and workload shape in the file named by
                              MDB_SCHEDULE_CACHE (default
                              ~/.cache/md_simulation_cuda_b200/schedule.txt).
