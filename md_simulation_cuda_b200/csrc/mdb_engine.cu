@@ -248,21 +248,25 @@ void Engine::set_list_grid() {
 // 52 / 62, 7 162 / 93, 9 249 / 132, 15 748 / 413; all-pairs strips of 3,000
 // 549 / 321. 262,144 particles: cutoff 5 65 / 83, 5.5 (1% of the
 // chunks) 200 / 107, 7 (7%) 347 / 149.
-int Engine::use_slot_lists() {
-  BatchGlobal g;
-  MDB_CUDA(cudaMemcpyAsync(&g, dev_.bg, sizeof(g), cudaMemcpyDeviceToHost, stream_));
-  MDB_CUDA(wait_host());
-  double mean = 0.0;
+bool Engine::bands_fit() const {
+  double mean = 0.0, all_pairs = 0.0;
   for (const SysParams& P : hsp_) {
     const double cols = std::max(1.0, floor(P.Lx0 / P.r_cell));
     const double rows = std::max(1.0, floor(P.Ly0 / P.r_cell));
     const double cell = P.n / (cols * rows), row = P.n / rows;
-    if (4.0 * row > kBandCap && 4.0 * (kThreads + 3.0 * cell) > 0.95 * kBandCap)
+    if (cols < 3.0 || rows < 3.0)
+      all_pairs += P.n;
+    else if (4.0 * row > kBandCap && 4.0 * (kThreads + 3.0 * cell) > 0.95 * kBandCap)
       mean += P.n * std::min(1.0, kThreads / row);
   }
-  if (g.unbanded * (double)kBandUnfitNow <= (double)ntot_ &&
-      mean * kBandUnfitMean <= (double)ntot_)
-    return MDB_OK;
+  return all_pairs * kBandUnfitNow <= (double)ntot_ && mean * kBandUnfitMean <= (double)ntot_;
+}
+
+int Engine::use_slot_lists() {
+  BatchGlobal g;
+  MDB_CUDA(cudaMemcpyAsync(&g, dev_.bg, sizeof(g), cudaMemcpyDeviceToHost, stream_));
+  MDB_CUDA(wait_host());
+  if (g.unbanded * (double)kBandUnfitNow <= (double)ntot_) return MDB_OK;
   const size_t bytes[2] = {sizeof(Band) * (size_t)dev_.nchunks,
                            sizeof(uint2) * (size_t)((max_nbr_ + 3) / 4) * ntot_};
   void* const gone[2] = {dev_.bands, dev_.lists};
@@ -469,8 +473,9 @@ int Engine::build() {
   rc = choose_multi_step();
   if (rc) return rc;
   // Systems that do not run in the resident steps kernel take the staged bands
-  // (one lane per slot), where these fit: see use_slot_lists.
-  banded_ = !multi_step_ && !lanes_;
+  // (one lane per slot), where these fit.
+  banded_ = !multi_step_ && !lanes_ && bands_fit();
+  band_steps_ = band_steps_ && banded_;
   int32_t *soc = nullptr, *sot = nullptr;
   D.nchunks = ch0;
   D.ntiles = t0;

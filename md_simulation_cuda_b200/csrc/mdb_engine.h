@@ -111,8 +111,10 @@ class Engine {
   int alloc_slot_lists();
   // One wave of resident blocks for the list build.
   void set_list_grid();
+  // Whether staged bands hold the chunks of systems of these sizes and densities.
+  bool bands_fit() const;
   // Gives the staged bands up after the first rebuild when they do not fit the
-  // systems, and rebuilds with lists of slot offsets.
+  // frames as they are, and rebuilds with lists of slot offsets.
   int use_slot_lists();
   // A kernel, its launch shape and dynamic shared memory.
   struct Kernel {

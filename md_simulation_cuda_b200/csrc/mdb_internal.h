@@ -167,9 +167,10 @@ constexpr int kBandRanges = 8;
 constexpr int kBandCap = 1408;   // positions of a staged band: two bands and four
                                  // blocks an SM leave L1 some 50 KB
 constexpr int kBandRoom = 4;     // positions after it that may be read (never used)
-// An engine keeps lists of slot offsets instead (Engine::use_slot_lists) when more
-// than one slot in kBandUnfitNow is in a chunk without a band at the first rebuild,
-// or more than one in kBandUnfitMean would be at the systems' mean densities.
+// An engine keeps lists of slot offsets instead (Engine::bands_fit, use_slot_lists)
+// when more than one slot in kBandUnfitNow belongs to an all-pairs system or is in a
+// chunk without a band at the first rebuild, or more than one in kBandUnfitMean would
+// be at the systems' mean densities.
 constexpr int kBandUnfitNow = 16, kBandUnfitMean = 256;
 struct Band {
   int32_t start[kBandRanges], len[kBandRanges], off[kBandRanges];

@@ -117,3 +117,22 @@ def test_fire_with_a_long_cutoff(built):
         r = b.fire_result(k)
         assert a.steps == r.steps and a.max_force == r.max_force
         assert np.array_equal(a.frame["pos"], r.frame["pos"])
+
+
+def test_clustered_frames_keep_their_lists(built):
+    """A droplet of a high density in a large empty box: the mean density says that its
+    chunks fit, the frame's own count that they don't."""
+    n = 9000
+    f, Lx, Ly = wl.lattice_frame(n, 0.8, 1.0, 0.5, 0.1, seed=4, jitter=0.02)
+    f["pos"] += 3.0 * Lx
+    cfg = wl.config_dict(n, 7.0 * Lx, 7.0 * Ly, dt=0.0005, T=0.1, cutoff=7.0)
+    b = mdb.Batch(max_neighbors=190)
+    for _ in range(2):
+        b.add_md(cfg, f, mdb.JOB_NVE, 20)
+    b.run(0)
+    assert b.system_stats(0) == (1, 0)
+    b.run()
+    sim = mdb.MDSimulation(cfg, frame=f, max_neighbors=190, lanes=mdb.LANES_ONE)
+    sim.step_single_NVE(nsteps=20)
+    sim.sample_collect()
+    assert np.array_equal(sim.get_host_particles()["pos"], b.frame(1)["pos"])
