@@ -603,10 +603,12 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
             }
             if constexpr (HP) {
               const float4* src = staged ? band + band_place(sh.bands[buf], a) : D.pff + a;
+              for (int m = 0; m < e - a;) {
+                const int end = NC ? e - a : min(e - a, m + kScanPiece);
 #pragma unroll 1
-              for (int m = 0; m < e - a; ++m) {
-                pair_one_hp<PY, kEnergy, kVirial, true>(src[m], cd, fx, fy, w, u, an);
-                if (!NC && (m + 1) % kScanPiece == 0) mark_progress(D);
+                for (; m < end; ++m)
+                  pair_one_hp<PY, kEnergy, kVirial, true>(src[m], cd, fx, fy, w, u, an);
+                if (!NC && end < e - a) mark_progress(D);
               }
             } else if (staged) {
               const float4* src = band + band_place(sh.bands[buf], a);
@@ -615,11 +617,13 @@ __device__ __forceinline__ void band_items(const Dev& D, const SysParams& P, con
               else
                 pair_run<kEnergy, kVirial, false, kFloor>(src, e - a, c, fs, fc, ws, wc, u, an);
             } else {
+              for (int m = a; m < e;) {
+                const int end = NC ? e : min(e, m + kScanPiece);
 #pragma unroll 1
-              for (int m = a; m < e; ++m) {
-                pair_one<PY, kEnergy, kVirial, true, kFloor>(ld_pos<NC>(D.pff + m), c, fs, fc, ws,
-                                                             wc, u, an);
-                if (!NC && (m + 1) % kScanPiece == 0) mark_progress(D);
+                for (; m < end; ++m)
+                  pair_one<PY, kEnergy, kVirial, true, kFloor>(ld_pos<NC>(D.pff + m), c, fs, fc,
+                                                               ws, wc, u, an);
+                if (!NC && end < e) mark_progress(D);
               }
             }
           }
