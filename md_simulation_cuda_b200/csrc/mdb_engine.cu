@@ -634,15 +634,16 @@ int Engine::choose_multi_step() {
   steps_.seq = (uint32_t*)(base + pos + part + mx);
   steps_.tile = (int32_t*)(steps_.seq + 3);
   dev_.progress = steps_.seq + 2;
-  // MDB_EXCHANGE_POLLS=<polls>[@<block>] makes every block, or one, look after that
-  // many polls whether others get on, for tests.
+  // MDB_EXCHANGE_POLLS=<polls>[@<block>] makes blocks look after that many polls
+  // whether others get on, and one of them wait for an arrival that never comes in a
+  // launch's last exchange (for tests).
   steps_.polls = kExchangePolls;
-  steps_.polls_block = -1;
+  steps_.late_block = -1;
   const char* polls = getenv("MDB_EXCHANGE_POLLS");
   if (polls && polls[0]) {
     steps_.polls = (uint32_t)std::min<unsigned long>(strtoul(polls, nullptr, 10), kExchangePolls);
     const char* at = strchr(polls, '@');
-    if (at) steps_.polls_block = atoi(at + 1);
+    if (at) steps_.late_block = atoi(at + 1);
   }
   return MDB_OK;
 }

@@ -230,7 +230,7 @@ struct StepsMem {
                     // [2] pieces of long scans (Dev::progress)
   int32_t list_rows;  // rows of the shared list (0: lists are read from global memory)
   uint32_t polls;     // polls of an exchange without progress before a block gives up
-  int32_t polls_block;  // the block they hold for (-1: every block), for tests
+  int32_t late_block;   // a block that waits for one arrival too many (-1: none), for tests
 };
 
 }  // namespace mdb
