@@ -634,9 +634,9 @@ int Engine::choose_multi_step() {
   steps_.seq = (uint32_t*)(base + pos + part + mx);
   steps_.tile = (int32_t*)(steps_.seq + 3);
   dev_.progress = steps_.seq + 2;
-  // MDB_EXCHANGE_POLLS=<polls>[@<block>] makes blocks look after that many polls
-  // whether others get on, and one of them wait for an arrival that never comes in a
-  // launch's last exchange (for tests).
+  // For tests, MDB_EXCHANGE_POLLS=<polls> makes blocks look after that many polls
+  // whether others get on; with @<block> only that block, which also waits for an
+  // arrival that never comes in a launch's last exchange.
   steps_.polls = kExchangePolls;
   steps_.late_block = -1;
   const char* polls = getenv("MDB_EXCHANGE_POLLS");

@@ -230,7 +230,8 @@ struct StepsMem {
                     // [2] pieces of long scans (Dev::progress)
   int32_t list_rows;  // rows of the shared list (0: lists are read from global memory)
   uint32_t polls;     // polls of an exchange without progress before a block gives up
-  int32_t late_block;   // a block that waits for one arrival too many (-1: none), for tests
+  int32_t late_block;   // for tests: the one block that `polls` holds for, which waits for
+                        // one arrival too many (-1: none, and `polls` holds for all)
 };
 
 }  // namespace mdb

@@ -167,8 +167,10 @@ __device__ __forceinline__ void exchange(const StepsMem& M, StepsShared& sh, uin
       // counts the block in; the release covers the block's writes (ordered
       // before by the block barrier)
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(M.seq + 1) : "memory");
-      const uint32_t target = seq * (uint32_t)nb + (M.late_block == (int)blockIdx.x ? 1u : 0u);
-      const uint32_t most = M.polls;
+      uint32_t target = seq * (uint32_t)nb;
+      const uint32_t most =
+          M.late_block < 0 || M.late_block == (int)blockIdx.x ? M.polls : kExchangePolls;
+      if (M.late_block == (int)blockIdx.x) ++target;
       uint32_t got, polls = 0, seen = 0;
       bool looked = false;
       for (;;) {
